@@ -19,10 +19,13 @@
  *   - One handle = one block of elements on one GPU, one CUDA stream.  Calls on
  *     one handle must not overlap (like the reference's ModelData, which is not
  *     thread-safe); different handles are independent.
- *   - Arithmetic: NSM_PRECISION_FP64 computes in IEEE FP64 throughout.
- *     NSM_PRECISION_FP32_MIXED computes the element work (gradient, F, stress,
- *     B^T sigma) in FP32 and keeps the nodal state, mass, time step and
- *     energies in FP64.
+ *   - Arithmetic: NSM_PRECISION_FP64 takes and gives FP64 numbers; nodal
+ *     state, mass, time step and energies are computed in IEEE FP64, the
+ *     element work (gradient, F, stress, B^T sigma) in 64-bit fixed point whose
+ *     error is below an FP64 evaluation's, or in FP64 where an element leaves
+ *     its domain (strains of about 0.1; csrc/hex_fixed.cuh).
+ *     NSM_PRECISION_FP32_MIXED computes the element work in FP32 and keeps the
+ *     nodal state, mass, time step and energies in FP64.
  */
 #ifndef NIMBLE_GB300_H
 #define NIMBLE_GB300_H

@@ -1,0 +1,431 @@
+// The FP64 form's element kernel in 64-bit fixed point (hex_fixed.cuh): gather
+// -> deformation gradient -> neo-Hookean or elastic Cauchy stress -> B^T
+// sigma, from FP64 displacements to FP64 element forces and records.
+//
+// Bound: the integer pipes and issue.  On the FP64 pipe the same work is 170
+// FP64 instructions per point at 16 clocks each per SM: 5.08 ms for 128^3
+// elements, pipe 89% busy.  Here it is about 1,500 integer instructions per
+// point, 380 of them wide products (one per clock and SM), the others at two
+// to four per clock: 1.24 ms, 1.84 ms with F and sigma stored (issue 52%,
+// multiplier 64%); one launch on 4,096 elements 12 us against 60 us.
+//
+// Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
+// j-th of 8 consecutive elements), two points each, in a loop that is not
+// unrolled: the code of one point stays in the instruction cache (four points
+// unrolled, two lanes per element, ran at 25% issue with instruction fetch the
+// largest stall), and a small mesh waits for two points in a row, not eight.
+// The lanes exchange 18 numbers before and 18 after.  Everything an element's
+// result depends on is its own, so any launch shape gives the same bits.
+//
+// The warps are persistent and independent of one another: each walks groups
+// of 8 elements with the next group's geometry (one 5 KB bulk copy),
+// displacements (cp.async) and connectivity in flight.
+//
+// An element outside the fixed-point domain is evaluated by the FP64 code
+// (element_work), records included.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "element_work.cuh"
+#include "hex_fixed.cuh"
+#include "tc05.cuh"
+
+namespace nsm {
+
+using fx::i64;
+using fx::Limbs;
+using fx::u64;
+
+// Geometry of 8 elements in fixed point, one block of kGeoRows rows of 32
+// lanes (row (side along xi, value), lane [side along (zeta, eta)][element]):
+// per point G0 (9 values, row-major, as limbs) and the reference volume; the
+// last row holds each element's exponents.  A warp's working set is this one
+// block, which a bulk copy brings to shared memory while the previous one is
+// computed on.
+constexpr int kGeoPoint = 10, kGeoRows = 2 * kGeoPoint + 1, kGeoBlock = kGeoRows * 32;  // words
+constexpr int kGeoBytes = kGeoBlock * 8;
+
+// From the FP64 planes: G0 scaled by 2^sG so that its largest entry over the
+// points is in [2^60, 2^61), the volume det J_X over 2^Ed (the largest in
+// [1/2, 1)) at 2^62, and the exponents su = 124 - sG and Ed - sG + 2.
+__global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ geo, i64* __restrict__ out)
+{
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  double gmax = 0.0, dmax = 0.0;
+  for (int p = 0; p < 8; p++) {
+    for (int q = 0; q < 9; q++) gmax = fmax(gmax, fabs(geo[(p * kGeoPerPoint + q) * ld_e + e]));
+    dmax = fmax(dmax, geo[(p * kGeoPerPoint + 9) * ld_e + e]);
+  }
+  int eg = 0, ed = 0;
+  frexp(gmax, &eg);
+  frexp(dmax, &ed);
+  // (values far from 1 leave the element to the FP64 code)
+  const bool fits = gmax > 1e-90 && gmax < 1e90 && dmax > 1e-60 && dmax < 1e60;
+  const int  sG   = 61 - eg, su = fits ? 124 - sG : 1 << 20, ef = fits ? ed - sG + 2 : 0;
+  i64* const base = out + (size_t)(e >> 3) * kGeoBlock + (e & 7);
+  for (int p = 0; p < 8; p++) {
+    const int  y = sy_of(p), z = sz_of(p), lane = (2 * z + y) * 8;
+    i64* const dst = base + sx_of(p) * kGeoPoint * 32 + lane;
+    for (int q = 0; q < 9; q++) {
+      const double g    = geo[(p * kGeoPerPoint + q) * ld_e + e];
+      const bool   flip = (q / 3 == 1 && y == 0) || (q / 3 == 2 && z == 0);  // mirrored rows
+      const Limbs  l    = fx::split(fits ? __double2ll_rn(scalbn(flip ? -g : g, sG)) : 0);
+      dst[q * 32]       = (i64)(((u64)(unsigned)l.hi << 32) | (unsigned)l.lo);
+    }
+    dst[9 * 32] = fits ? __double2ll_rn(scalbn(geo[(p * kGeoPerPoint + 9) * ld_e + e], 62 - ed)) : 0;
+    if (sx_of(p) == 0) base[2 * kGeoPoint * 32 + lane] = (i64)(((u64)(unsigned)su << 32) | (unsigned)ef);
+  }
+}
+
+size_t fixed_geometry_words(long ld_e) { return (size_t)((ld_e + 7) / 8) * kGeoBlock; }
+
+cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, long long* out, cudaStream_t stream)
+{
+  if (E == 0) return cudaSuccess;
+  k_fixed_geometry<<<grid_for(E, 128), 128, 0, stream>>>(E, ld_e, geo, out);
+  return cudaGetLastError();
+}
+
+FixedMaterial fixed_material(const GroupMaterial& m)
+{
+  FixedMaterial f{0, 0, 0, 1 << 20, m.model};
+  const double  most = std::fmax(m.bulk, m.shear);
+  if (!std::isfinite(most) || !(most > 1e-90) || !(most < 1e90)) return f;  // left to the FP64 code
+  f.exponent = std::ilogb(most) + 4;
+  f.half_k   = std::llrint(std::ldexp(m.bulk, 61 - f.exponent));
+  f.shear    = std::llrint(std::ldexp(m.shear, 62 - f.exponent));
+  f.lambda   = std::llrint(std::ldexp(m.bulk - 2.0 * m.shear / 3.0, 62 - f.exponent));
+  return f;
+}
+
+template <int kXor>
+__device__ __forceinline__ i64 other(i64 x)
+{
+  return __shfl_xor_sync(0xffffffffu, x, kXor);
+}
+constexpr int kAcrossEta = 8, kAcrossZeta = 16;  // lane masks
+
+// The element as a whole on the FP64 pipe, by one lane.
+__device__ __noinline__ void fallback_fp64(const ElementArgs& a, int e)
+{
+  element_work<double, true, GlobalNodes<double>, 0, false>(a, e, GlobalNodes<double>(a, e));
+}
+
+// The records of one point per lane: 8 consecutive records in each of four
+// planes, through the warp's tile (warp_store's slots: rows of 8 chunks), 512
+// contiguous bytes per instruction.  Elements outside [e_begin, E) are not
+// this launch's.
+__device__ __forceinline__ void store_records(const ElementArgs& a, long eb, int sx, const double* r, uint4* tile, int lane)
+{
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; c++) tile[tile_slot<8>(lane, c)] = pack16(r, c);
+  __syncwarp();
+  uint4* const ip = reinterpret_cast<uint4*>(a.ip);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int  yz = k >> 1, j = (k & 1) * 32 + lane;  // chunk j of the plane's 8 records
+    const int  p  = corner_of(sx, yz & 1, yz >> 1);
+    const long e  = eb + (j >> 3);
+    if (e >= a.e_begin && e < a.E) ip[((size_t)p * a.ld_e + eb) * 8 + j] = tile[tile_slot<8>(yz * 8 + (j >> 3), j & 7)];
+  }
+}
+
+// A warp's shared memory: two geometry blocks, two sets of the lanes' nodal
+// displacements, the barriers of the blocks' copies; then, where records are
+// stored, their tile.
+constexpr int kStageU     = 2 * kGeoBytes;
+constexpr int kStageBar   = kStageU + 2 * 6 * 32 * 8;
+constexpr int kStageTile  = kStageBar + 128;
+constexpr int kStageBytes = kStageTile, kStageBytesStore = kStageTile + 32 * 128;
+static_assert(kStageTile % 128 == 0 && kGeoBytes % 16 == 0, "alignment");
+
+__device__ __forceinline__ void load_g0(const i64* gp, Limbs g0[3][3])
+{
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    const i64 w      = gp[q * 32];
+    g0[q / 3][q % 3] = Limbs{(int)(w >> 32), (int)w};
+  }
+}
+
+// kStore: F and sigma are formed and stored when the launch asks for it.
+// kElastic: some material of the model is elastic.
+template <bool kStore, bool kHasElastic>
+__global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementArgs a)
+{
+  extern __shared__ __align__(128) uint8_t stage_all[];
+  const int      lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 7, y = (lane >> 3) & 1, z = lane >> 4;
+  const long     ld_e = a.ld_e, ld_n = a.ld_n;
+  uint8_t* const stage = stage_all + warp * (kStore ? kStageBytesStore : kStageBytes);
+  double* const  us    = reinterpret_cast<double*>(stage + kStageU) + lane;  // [2][6][32]
+  i64* const     us_i  = reinterpret_cast<i64*>(us);
+  uint64_t*      bar   = reinterpret_cast<uint64_t*>(stage + kStageBar);
+  const bool     store =
+      kStore && (a.store_ip == kStoreAlways || (a.sched != nullptr && a.sched[(long)(*a.step_base + a.k) * a.num_groups].is_output));
+  const int* const conn = a.conn + (long)(corner_of(0, y, 0) + 4 * z) * ld_e;
+  const long       next_corner = (corner_of(1, y, 0) - corner_of(0, y, 0)) * ld_e;
+
+  // groups of 8 elements; those at the ends of [e_begin, E) may be partial
+  const long g_end = (a.E + 7) >> 3, g_step = (long)gridDim.x * (blockDim.x >> 5);
+  long       g     = (a.e_begin >> 3) + (long)blockIdx.x * (blockDim.x >> 5) + warp;
+  const long first = g;
+  if (g >= g_end) return;
+  auto load_ids = [&](long gr, int id[2]) {
+    const long e = min(gr * 8 + j, (long)a.E - 1);  // (spare lanes repeat the last element)
+    id[0]        = __ldg(&conn[e]);
+    id[1]        = __ldg(&conn[e + next_corner]);
+  };
+  auto stage_u = [&](int buf, const int id[2]) {
+#pragma unroll
+    for (int bx = 0; bx < 2; bx++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) cp_async8(us + (buf * 6 + i * 2 + bx) * 32, a.u + i * ld_n + id[bx]);
+  };
+  auto stage_geo = [&](int buf, long gr) {
+    if (lane == 0) tc::bulk_load(stage + buf * kGeoBytes, a.geo_fixed + gr * kGeoBlock, kGeoBytes, &bar[buf]);
+  };
+  if (lane == 0) {
+    tc::mbar_init(&bar[0], 1);
+    tc::mbar_init(&bar[1], 1);
+    tc::fence_mbar_init();
+  }
+  __syncwarp();
+  int id[2];
+  load_ids(g, id);
+  stage_geo(0, g);
+  stage_u(0, id);
+  cp_async_commit();
+  if (g + g_step < g_end) load_ids(g + g_step, id);
+
+  unsigned any_bad = 0;
+  uint32_t phase = 0;  // bit b: parity of block b's next copy
+  for (int buf = 0; g < g_end; g += g_step, buf ^= 1) {
+    cp_async_wait_all();
+    if (!tc::mbar_wait(&bar[buf], (phase >> buf) & 1u)) {  // (bounded; nothing else of this warp is in flight)
+      atomicOr(a.status, NSM_STATUS_TIMEOUT);
+      return;
+    }
+    phase ^= 1u << buf;
+    if (g + g_step < g_end) {
+      stage_geo(buf ^ 1, g + g_step);
+      stage_u(buf ^ 1, id);
+      cp_async_commit();
+      if (g + 2 * g_step < g_end) load_ids(g + 2 * g_step, id);
+    }
+    const long       eb    = g * 8;
+    const int        e     = (int)min(eb + j, (long)a.E - 1);
+    const bool       valid = eb + j >= a.e_begin && eb + j < a.E;
+    i64* const       gs    = reinterpret_cast<i64*>(stage + buf * kGeoBytes) + lane;
+
+    // ---- displacements of the lane's two corners, at 2^sc ----
+    u64 u[3][2];
+    int exm = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int bx = 0; bx < 2; bx++) {
+        u[i][bx] = (u64)__double_as_longlong(us[(buf * 6 + i * 2 + bx) * 32]);
+        exm      = max(exm, (int)((unsigned)(u[i][bx] >> 32) & 0x7fffffffu));
+      }
+    exm = max(exm, __shfl_xor_sync(0xffffffffu, exm, kAcrossEta));
+    exm = max(exm, __shfl_xor_sync(0xffffffffu, exm, kAcrossZeta)) >> 20;
+    const i64           ge      = gs[2 * kGeoPoint * 32];
+    const FixedMaterial mat     = a.fixed_mats[a.elem_group ? __ldg(&a.elem_group[e]) : 0];
+    const bool          elastic = kHasElastic && mat.model == kElastic;
+    const int           su      = (int)(ge >> 32);
+    int                 sc      = 1079 - exm;
+    if (!elastic) sc = min(sc, su);
+    int      sh = su - sc, ee = 0;
+    unsigned bad = (unsigned)(mat.exponent + 400) > 800u;
+
+    // ---- modes and gradients ----
+    fx::Gradient G[3];
+    {
+      i64 v[3][7];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const i64 c0 = fx::to_fixed((unsigned)(u[i][0] >> 32), (unsigned)u[i][0], 1086 - sc);
+        const i64 c1 = fx::to_fixed((unsigned)(u[i][1] >> 32), (unsigned)u[i][1], 1086 - sc);
+        const i64 s = c1 + c0, d = c1 - c0;
+        const i64 so = other<kAcrossEta>(s), dn = other<kAcrossEta>(d);
+        i64       q[2][2] = {{s + so, d + dn}, {s - so, d - dn}}, o[2][2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k >> 1][k & 1] = other<kAcrossZeta>(q[k >> 1][k & 1]);
+        fx::lane_modes(q, o, v[i]);
+      }
+      if (kHasElastic && __any_sync(0xffffffffu, elastic)) {
+        u64 m = 0;
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int k = 0; k < 7; k++) m |= (u64)(v[i][k] ^ (v[i][k] >> 63));
+        m |= (u64)other<kAcrossEta>((i64)m);
+        m |= (u64)other<kAcrossZeta>((i64)m);
+        if (elastic) {
+          if (m == 0) sh = 0;
+          else fx::elastic_scale(64 - __clzll((i64)m), sc, su, sh, ee);
+          if (ee < -3) bad = 1, sh = 0, ee = 0;
+          const int up = max(sh, 0), down = min(max(-sh, 0), 63);
+#pragma unroll
+          for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int k = 0; k < 7; k++) v[i][k] = (i64)((u64)v[i][k] << up) >> down;
+        }
+      }
+      if (!elastic && sh != 0) {
+        if (sh > 26) bad = 1, sh = 26;
+#pragma unroll
+        for (int i = 0; i < 3; i++) bad |= fx::lane_shift(v[i], sh);
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        fx::lane_gradient(v[i], G[i]);
+        // (the second point's increments wait where the displacements were)
+        us_i[(buf * 6 + i) * 32]     = G[i].y1;
+        us_i[(buf * 6 + 3 + i) * 32] = G[i].z1;
+      }
+    }
+
+    // ---- the lane's two points ----
+    // What a point does not need while it is computed waits in shared memory
+    // (registers spilled to local memory would miss the small L1 that the
+    // staging leaves): G0 is read twice, and the first point's forces are kept
+    // in its own geometry rows.
+    i64              Q[3][3];
+    const fx::Moduli mod{mat.half_k, mat.shear, mat.lambda, mat.exponent, mat.model};
+    i64*             gp = gs;
+#pragma unroll 1
+    for (int sx = 0; sx < 2; sx++, gp += kGeoPoint * 32) {
+      i64 P[3][3];
+      {
+        Limbs g0[3][3];
+        load_g0(gp, g0);
+        i64 Du[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) Du[i][0] = G[i].x, Du[i][1] = G[i].y, Du[i][2] = G[i].z;
+        const i64 det = gp[9 * 32];
+        fx::Point pt;
+        if (kHasElastic && elastic) {
+          i64       He[3][3];
+          const int up = max(-ee, 0), down = max(ee, 0);
+          fx::displacement_gradient(Du, g0, He);
+#pragma unroll
+          for (int q = 0; q < 9; q++) {
+            pt.H[q / 3][q % 3] = (i64)((u64)He[q / 3][q % 3] << up) >> down;
+            bad |= fx::outside<27>(pt.H[q / 3][q % 3]);  // (|H|^2 below would not show it)
+          }
+          bad |= fx::kinematics(pt);
+          bad |= fx::elastic_force<kStore>(mod, det, He, pt, P);
+        } else {
+          fx::displacement_gradient(Du, g0, pt.H);
+          bad |= fx::kinematics(pt);
+          fx::neohookean_force<kStore>(mod, det, pt, P);
+        }
+        if (store) {
+          double       r[kIpRecord];
+          const double ss = __longlong_as_double((i64)(1023 - 62 + mat.exponent - ee) << 52);
+#pragma unroll
+          for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+              r[full_slot(i, k)] = (double)(pt.H[i][k] + (i == k ? fx::kOne : 0)) * (1.0 / 1152921504606846976.0);
+#pragma unroll
+          for (int q = 0; q < 6; q++) r[9 + q] = (double)pt.sig[q] * ss;
+          r[15] = 0.0;
+          store_records(a, eb, sx, r, reinterpret_cast<uint4*>(stage + kStageTile), lane);
+        }
+      }
+      asm volatile("" ::: "memory");  // G0 is read again rather than kept
+      Limbs g0[3][3];
+      load_g0(gp, g0);
+      fx::point_force(g0, P, Q);
+      if (sx == 0) {
+#pragma unroll
+        for (int q = 0; q < 9; q++) gp[q * 32] = Q[q / 3][q % 3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          G[i].y += us_i[(buf * 6 + i) * 32];
+          G[i].z += us_i[(buf * 6 + 3 + i) * 32];
+        }
+      }
+    }
+
+    // ---- nodal forces of the lane's corners ----
+    const int    ef    = (int)ge + mat.exponent - ee - (elastic ? fx::kElasticForce : 0);
+    const double scale = __longlong_as_double((i64)(1023 + ef) << 52);
+    double       f[2][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const i64      qx = gs[i * 32], qy = gs[(3 + i) * 32], qz = gs[(6 + i) * 32];
+      const fx::Sums S{Q[0][i] + qx, Q[1][i] + qy, Q[1][i] - qy, Q[2][i] + qz, Q[2][i] - qz};
+      fx::Parts      keep, send;
+      if (elastic) bad |= fx::too_large(S);
+      fx::lane_adjoint(S, keep, send);
+      const i64 e0 = keep.e0 + other<kAcrossZeta>(send.e0), e1 = keep.e1 + other<kAcrossZeta>(send.e1);
+      const i64 o0 = keep.o0 + other<kAcrossZeta>(send.o0), o1 = keep.o1 + other<kAcrossZeta>(send.o1);
+      const i64 ev = (e0 + e1) + other<kAcrossEta>(e0 - e1), od = (o0 + o1) + other<kAcrossEta>(o0 - o1);
+      f[0][i] = (double)(od - ev) * scale;
+      f[1][i] = (double)(-od - ev) * scale;
+    }
+    bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossEta);
+    bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossZeta);
+    if (bad == 0 && valid) {
+      double* const fe = reinterpret_cast<double*>(a.fe) + e;
+#pragma unroll
+      for (int bx = 0; bx < 2; bx++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) fe[(size_t)(3 * (corner_of(bx, y, 0) + 4 * z) + i) * ld_e] = f[bx][i];
+    }
+    // which elements are left to the FP64 code
+    any_bad |= bad;
+    if (y == 0 && z == 0 && valid) a.elem_left[e] = bad != 0;
+    tc::fence_proxy_async();  // this lane's writes to the block come before the next copy into it
+    __syncwarp();             // this group's staged data are read, its records written
+  }
+  // (after the loop: a call inside it would spill the loop's state)
+  if (__any_sync(0xffffffffu, any_bad != 0) && y == 0 && z == 0)
+    for (g = first; g < g_end; g += g_step) {
+      const long e = g * 8 + j;
+      if (e >= a.e_begin && e < a.E && a.elem_left[e]) fallback_fp64(a, (int)e);
+    }
+}
+
+// Blocks of 128 threads, four warps, four blocks per SM (three where records
+// are stored): 16 warps of 128 registers and 14 KB of staging.
+template <bool kStore, bool kHasElastic>
+static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
+{
+  constexpr int     bytes = kStore ? kStageBytesStore : kStageBytes;
+  // set once per device; repeated by a thread that races the first, to the same values
+  static std::atomic<unsigned long long> configured{0};
+  int               dev = 0;
+  cudaError_t       err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(configured.load(std::memory_order_acquire) & bit)) {
+    err = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * bytes);
+    if (err == cudaSuccess)
+      err = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (err != cudaSuccess) return err;
+    configured.fetch_or(bit, std::memory_order_release);
+  }
+  const int  warps  = l.block == 64 ? 2 : 4;
+  const long groups = ((a.E + 7L) >> 3) - (a.e_begin >> 3);
+  const int  per_sm = l.persistent ? l.blocks_per_sm : (kStore ? 3 : 4) * (4 / warps);
+  const long grid   = std::min<long>((groups + warps - 1) / warps, (long)per_sm * num_sms());
+  k_element_fixed<kStore, kHasElastic><<<(int)grid, 32 * warps, warps * bytes, stream>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_element_fp64(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
+{
+  if (a.E <= a.e_begin) return cudaSuccess;
+  if (a.store_ip == kStoreNever)
+    return a.has_elastic ? launch_fixed<false, true>(a, l, stream) : launch_fixed<false, false>(a, l, stream);
+  return a.has_elastic ? launch_fixed<true, true>(a, l, stream) : launch_fixed<true, false>(a, l, stream);
+}
+
+}  // namespace nsm

@@ -6,8 +6,11 @@
 // (src/nimble_element.h:430-502), the neo-Hookean stress
 // (src/nimble_material.cc:252-310) and the element nodal forces
 // f_a = -sum_ip (dN_a/dx . sigma) det(dx/dxi) w (src/nimble_element.h:540-625).
-// How it is computed is chosen to spend as few FP64 operations as possible
-// (FP64 is this chip's narrow pipe, ~1.2 TFLOP/s):
+// How it is computed is chosen to spend as few floating-point operations as
+// possible.  T = float is the FP32 form's element; T = double evaluates what
+// the FP64 form's fixed-point kernel (hex_fixed.cuh) leaves to it, and the two
+// passes of models with block-material callbacks (FP64 is this chip's narrow
+// pipe, ~1.2 TFLOP/s):
 //   * Modal (tensor-product) form of the trilinear hex: du/dxi at the 8
 //     points takes only 4 distinct values (it does not depend on xi), formed
 //     from the Hadamard transform of the corner values; same for eta and

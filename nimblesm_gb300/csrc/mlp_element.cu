@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
   const uint32_t tb    = tslot;
   const uint32_t taddr = tb + ((uint32_t)(warp * 32) << 16);
   uint8_t* const stage = sm + el::A + warp * el::kStageWarp;
-  const bool     store = a.store_ip || (a.sched != nullptr && a.sched[(long)(*a.step_base + a.k) * a.num_groups].is_output);
+  const bool     store = a.store_ip == kStoreAlways ||
+                         (a.store_ip == kStoreOutput && a.sched != nullptr && a.sched[(long)(*a.step_base + a.k) * a.num_groups].is_output);
   const float    K = (float)a.bulk, Gm = (float)a.shear;
   float          w[3][2][2];
   point_weights(p, w);

@@ -31,6 +31,15 @@ struct GroupMaterial {
 // those of the modal gradient (8 du/dxi); powers of two, so exact.
 constexpr int kGeoPerPoint = 20;
 
+// A material in fixed point (element_fixed.cu): K / 2, G and K - 2 G / 3 over
+// 2^exponent, at 2^62.
+struct FixedMaterial {
+  long long half_k, shear, lambda;
+  int       exponent;  // large: outside the range, its elements take the FP64 code
+  int       model;
+};
+FixedMaterial fixed_material(const GroupMaterial& m);
+
 struct SetupArgs {
   int           N, E;
   int           num_groups;      // samples; elements of sample g are [elem_off[g], elem_off[g+1])
@@ -69,6 +78,11 @@ cudaError_t launch_derived_element(int E, long ld_e, const int* conn, const doub
 // stores; a warp writes 2 or 4 KB contiguous.
 constexpr int kIpRecord = 16;
 
+// When an element launch writes the records: on the schedule's output steps,
+// always, or never (a step inside a launch sequence, whose records the next
+// step overwrites before anything can read them).
+constexpr int kStoreOutput = 0, kStoreAlways = 1, kStoreNever = -1;
+
 // Element kernel arguments (one launch = all elements of a block).
 struct ElementArgs {
   int           E;         // elements [e_begin, E) are computed by this launch
@@ -79,6 +93,10 @@ struct ElementArgs {
   const float*  uf;        // [3][ld_n] FP32 copy of u (FP32 form)
   const float*  Xf;        // [3][ld_n] FP32 copy of X (FP32 form)
   const double* geo;       // [8 * kGeoPerPoint][ld_e] (FP64 form only)
+  const long long* geo_fixed;      // fixed-point geometry (FP64 form only; element_fixed.cu)
+  const struct FixedMaterial* fixed_mats;  // materials in fixed point
+  int              has_elastic;    // one of them is elastic
+  unsigned char*   elem_left;      // [ld_e] scratch: elements outside the fixed-point domain
   double        bulk, shear;     // material when elem_group is null
   int           model;           // material model when elem_group is null
   const int*    elem_group;      // [E] material of each element, or null
@@ -87,7 +105,7 @@ struct ElementArgs {
   int           persistent;      // 0: one thread per element; 1: grid-stride over elements
   void*         ip;        // [8][ld_e][16] per-point records (T)
   void*         fe;        // [ld_e][24] element nodal forces, corner-major (T)
-  int               store_ip;   // 1: write F and sigma; 0: only on output steps of the schedule
+  int               store_ip;   // kStore*
   const StepSched*  sched;      // schedule (nullable: outside the time loop)
   const int*        step_base;  // device step counter
   int               k;          // schedule offset of this step
@@ -108,6 +126,9 @@ cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cu
 // recorded sigma (one thread per element).
 cudaError_t launch_element_pass(const ElementArgs& a, int is_float, int pass, cudaStream_t stream);
 int         num_sms();
+// The FP64 form's fixed-point geometry (words: 64-bit), from the geo planes.
+size_t      fixed_geometry_words(long ld_e);
+cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, long long* out, cudaStream_t stream);
 // F = I (sigma = 0) in every point record: the element data before the first step.
 cudaError_t launch_ip_identity(int E, long ld_e, void* ip, int ip_is_float, cudaStream_t stream);
 

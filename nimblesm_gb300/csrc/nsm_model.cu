@@ -73,6 +73,9 @@ struct nsm_model {
   double* d_mass = nullptr;
   double* d_inv_mass = nullptr;
   double* d_geo = nullptr;  // [8 * kGeoPerPoint][ld_e]
+  long long*          d_geo_fixed = nullptr;   // FP64 form: fixed-point geometry, materials
+  nsm::FixedMaterial* d_fixed_mats = nullptr;
+  unsigned char*      d_elem_left = nullptr;
   void*   d_ip = nullptr;   // [8][ld_e][16] per-point F and sigma records
   void*   d_fe = nullptr;   // [24][ld_e] element nodal forces, corner-major planes (3 c + i)
   float*  d_Xf = nullptr;   // FP32 copies of X and u (FP32 form)
@@ -168,7 +171,8 @@ void free_all(nsm_model* m)
                   m->d_bcs,  m->d_ibc_slot, m->d_ibcs,     m->d_sched, m->d_group_out, m->d_elem_group,
                   m->d_node_group, m->d_elem_off, m->d_mats, m->d_fallbacks, m->d_node_off, m->d_closure,
                   m->d_stage_out, m->d_expr_code, m->d_expr_start, m->d_bc_slot_node, m->d_bc_expr_val,
-                  m->d_closure_geo, m->d_ip_n, m->d_state, m->d_state_n};
+                  m->d_closure_geo, m->d_ip_n, m->d_state, m->d_state_n,
+                  m->d_geo_fixed, m->d_fixed_mats, m->d_elem_left};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (cudaStream_t s : m->hp_stream)
@@ -289,7 +293,9 @@ double* field_ptr(nsm_model* m, int field)
   }
 }
 
-nsm::ElementArgs element_args(nsm_model* m, int k)
+// k: schedule offset of the step, or -1 outside the loop; `last`: nothing is
+// launched after this step that overwrites its records.
+nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
 {
   nsm::ElementArgs a;
   a.E         = m->E;
@@ -301,6 +307,11 @@ nsm::ElementArgs element_args(nsm_model* m, int k)
   a.uf        = m->d_uf;
   a.Xf        = m->d_Xf;
   a.geo       = m->d_geo;
+  a.geo_fixed  = m->d_geo_fixed;
+  a.fixed_mats = m->d_fixed_mats;
+  a.elem_left  = m->d_elem_left;
+  a.has_elastic = 0;
+  for (const auto& mat : m->h_mats) a.has_elastic |= mat.model == nsm::kElastic;
   a.bulk      = m->K;
   a.shear     = m->G;
   a.model     = m->model;
@@ -310,7 +321,8 @@ nsm::ElementArgs element_args(nsm_model* m, int k)
   a.mats       = m->d_mats;
   a.num_groups = m->S;
   a.persistent = 0;
-  a.store_ip  = (k < 0 || m->store_ip) ? 1 : 0;
+  a.store_ip  = k < 0 ? nsm::kStoreAlways
+                      : (!m->store_ip ? nsm::kStoreOutput : (last ? nsm::kStoreAlways : nsm::kStoreNever));
   a.sched     = k < 0 ? nullptr : m->d_sched;
   a.step_base = m->d_step_base;
   a.k         = k;
@@ -390,7 +402,7 @@ cudaError_t element_split(nsm_model* m, int k)
     t_np1          = m->h_time[s + 1];
   }
   const int        is_float = m->precision == NSM_PRECISION_FP64 ? 0 : 1;
-  nsm::ElementArgs a        = element_args(m, k);
+  nsm::ElementArgs a        = element_args(m, k, true);
   cudaError_t      e        = nsm::launch_element_pass(a, is_float, 1, m->stream);
   for (size_t b = 0; b < m->block_cb.size() && e == cudaSuccess; b++) {
     const auto& cb = m->block_cb[b];
@@ -421,10 +433,10 @@ cudaError_t element_split(nsm_model* m, int k)
   return e;
 }
 
-cudaError_t launch_element(nsm_model* m, int k)
+cudaError_t launch_element(nsm_model* m, int k, bool last)
 {
   if (has_callbacks(m)) return element_split(m, k);
-  nsm::ElementArgs a = element_args(m, k);
+  nsm::ElementArgs a = element_args(m, k, last);
   if (m->closure) {
     nsm::mlp::MlpElementArgs ma;
     nsm::mlp::element_args(m->closure, &ma, nullptr, nullptr);
@@ -469,14 +481,14 @@ cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
     if (timed) {
       auto ev = next_events(m->ev_elem, m->ev_elem_used);
       cudaEventRecord(ev.first, m->stream);
-      if ((e = launch_element(m, k)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, true)) != cudaSuccess) return e;
       cudaEventRecord(ev.second, m->stream);
       auto en = next_events(m->ev_node, m->ev_node_used);
       cudaEventRecord(en.first, m->stream);
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
       cudaEventRecord(en.second, m->stream);
     } else {
-      if ((e = launch_element(m, k)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, true)) != cudaSuccess) return e;
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
     }
   }
@@ -580,10 +592,8 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     delete m;
     return fail(NSM_ERR_INVALID_ARGUMENT, "unknown precision");
   }
-  // default launch shapes, the fastest measured at 128^3: FP64 one thread per
-  // element; FP32 the persistent grid with the nodal values staged ahead
-  // the measured fastest shapes at 128^3: FP64 registers bounded for 3 CTAs of
-  // 128 per SM (5.34 ms against 5.38 unbounded), FP32 the staged persistent grid
+  // default launch shapes, the fastest measured at 128^3: FP64 as many blocks
+  // of 128 as fit (element_fixed.cu), FP32 the staged persistent grid
   m->elaunch = m->precision == NSM_PRECISION_FP64 ? nsm::ElementLaunch{128, 0, 3, 0} : nsm::ElementLaunch{128, 1, 3, 1};
   m->density   = materials[0].density;
   m->K         = materials[0].bulk_modulus;
@@ -745,6 +755,18 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     s.inv_mass   = m->d_inv_mass;
     s.status     = m->d_status;
     cudaError_t e = nsm::launch_setup(s, m->stream);  // also for no elements: mass 0, the largest step
+    std::vector<nsm::FixedMaterial> fixed_mats;
+    if (e == cudaSuccess && m->precision == NSM_PRECISION_FP64) {
+      for (const auto& b : gm) fixed_mats.push_back(nsm::fixed_material(b));
+      e = cudaMalloc(&m->d_geo_fixed, sizeof(long long) * nsm::fixed_geometry_words(m->ld_e));
+      if (e == cudaSuccess) e = cudaMalloc(&m->d_elem_left, m->ld_e);
+      if (e == cudaSuccess) e = cudaMalloc(&m->d_fixed_mats, sizeof(nsm::FixedMaterial) * num_mats);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(m->d_fixed_mats, fixed_mats.data(), sizeof(nsm::FixedMaterial) * num_mats,
+                            cudaMemcpyHostToDevice, m->stream);
+      if (e == cudaSuccess)
+        e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_geo_fixed, m->stream);
+    }
     m->dt_group.assign(S, 1.7976931348623157e308);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(m->dt_group.data(), m->d_group_out, sizeof(double) * S, cudaMemcpyDeviceToHost, m->stream);
@@ -1028,7 +1050,7 @@ int nsm_compute_internal_force(nsm_model* m, double time_previous, double time_c
   m->ci_t_prev  = time_previous;  // the step's times for block-material callbacks
   m->ci_t_cur   = time_current;
   m->cb_failed  = false;
-  cudaError_t e = launch_element(m, -1);
+  cudaError_t e = launch_element(m, -1, true);
   if (m->cb_failed) return fail(NSM_ERR_STATE, "a block-material callback failed");
   NSM_CUDA(e);
   NSM_CUDA(nsm::launch_node_update(node_args(m, -1, -1, 1), m->stream));
@@ -1120,7 +1142,7 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
     cudaStream_t s = s_el[j & 1];
     err            = cudaStreamWaitEvent(s, ev[1 + 3 * j], 0);
     if (err == cudaSuccess) {
-      nsm::ElementArgs a = element_args(m, -1);
+      nsm::ElementArgs a = element_args(m, -1, true);
       a.e_begin          = m->hp_e[j];
       a.E                = m->hp_e[j + 1];
       err = m->precision == NSM_PRECISION_FP64 ? nsm::launch_element_fp64(a, m->elaunch, s)
@@ -1181,7 +1203,7 @@ int nsm_compute_internal_force_host(nsm_model* m, const double* displacement, do
   const size_t bytes = sizeof(double) * 3 * m->N;
   NSM_CUDA(cudaMemcpyAsync(m->d_stage, displacement, bytes, cudaMemcpyHostToDevice, m->stream));
   NSM_CUDA(nsm::launch_node_aos_to_soa(m->N, m->ld_n, m->d_stage, m->d_u, m->d_uf, m->stream));
-  NSM_CUDA(launch_element(m, -1));
+  NSM_CUDA(launch_element(m, -1, true));
   NSM_CUDA(nsm::launch_node_update(node_args(m, -1, -1, 1), m->stream));
   NSM_CUDA(nsm::launch_node_soa_to_aos(m->N, m->ld_n, m->d_f, m->d_stage, m->stream));
   NSM_CUDA(cudaMemcpyAsync(internal_force, m->d_stage, bytes, cudaMemcpyDeviceToHost, m->stream));
@@ -1473,7 +1495,7 @@ int nsm_time_kernels(nsm_model* m, int repeats, double* element_ms, double* node
   NSM_CUDA(cudaEventCreate(&b));
   NSM_CUDA(cudaEventCreate(&c));
   cudaEventRecord(a, m->stream);
-  for (int r = 0; r < repeats; r++) NSM_CUDA(launch_element(m, -1));
+  for (int r = 0; r < repeats; r++) NSM_CUDA(launch_element(m, -1, true));
   cudaEventRecord(b, m->stream);
   for (int r = 0; r < repeats; r++) NSM_CUDA(nsm::launch_node_update(node_args(m, -1, -1, 1), m->stream));
   cudaEventRecord(c, m->stream);
@@ -1489,11 +1511,11 @@ int nsm_time_kernels(nsm_model* m, int repeats, double* element_ms, double* node
   return read_status(m);
 }
 
-// Element-kernel launch shapes the autotuner tries: elements per block; one
-// pass (one thread per element; blocks_per_sm > 0 then bounds the registers
-// so that many 128-thread blocks fit an SM, FP64 form) or a persistent grid of
-// blocks per SM walking the elements of all samples; and, in the FP32 form,
-// the persistent grid with the nodal values staged one element ahead.
+// Element-kernel launch shapes the autotuner tries: threads per block; as many
+// blocks as the work (FP32 form) or the SMs (FP64 form, always persistent)
+// take, or a persistent grid of blocks per SM walking the elements of all
+// samples; and, in the FP32 form, the persistent grid with the nodal values
+// staged one element ahead.
 // Shapes a form does not have fall back to its plain launch.
 static const nsm::ElementLaunch kLaunchCandidates[] = {
     {128, 0, 0, 0}, {64, 0, 0, 0},  {128, 1, 1, 0}, {128, 1, 2, 0}, {128, 1, 4, 0}, {64, 1, 2, 0},
@@ -1513,9 +1535,9 @@ int nsm_launch_candidate_times(nsm_model* m, int repeats, double* ms, int capaci
   cudaError_t err = cudaSuccess;
   for (int c = 0; c < kNumLaunchCandidates && c < capacity && err == cudaSuccess; c++) {
     m->elaunch = kLaunchCandidates[c];
-    err        = launch_element(m, -1);  // warm
+    err        = launch_element(m, -1, true);  // warm
     if (err == cudaSuccess) err = cudaEventRecord(a, m->stream);
-    for (int r = 0; r < repeats && err == cudaSuccess; r++) err = launch_element(m, -1);
+    for (int r = 0; r < repeats && err == cudaSuccess; r++) err = launch_element(m, -1, true);
     if (err == cudaSuccess) err = cudaEventRecord(b, m->stream);
     if (err == cudaSuccess) err = cudaEventSynchronize(b);
     float t = 0;
@@ -1575,7 +1597,7 @@ int nsm_set_mlp_closure(nsm_model* m, nsm_mlp* closure)
   }
   if (closure && !m->d_closure_geo) {  // the reference geometry of every point, once
     NSM_CUDA(cudaMalloc(&m->d_closure_geo, sizeof(float) * 96 * (size_t)m->ld_e));
-    NSM_CUDA(nsm::mlp::launch_closure_geometry(element_args(m, -1), m->d_closure_geo, m->stream));
+    NSM_CUDA(nsm::mlp::launch_closure_geometry(element_args(m, -1, true), m->d_closure_geo, m->stream));
   }
   m->closure = closure;
   for (auto& g : m->graphs) cudaGraphExecDestroy(g.second);

@@ -121,6 +121,18 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mbar)), "r"(count) : "memory");
 }
+// Make initialised barriers visible to the asynchronous copies that arrive on them.
+__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+// Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
+// global to this CTA's shared memory, by one thread: the barrier's phase
+// completes when all of them have arrived.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* mbar)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(mbar))
+               : "memory");
+}
 // One test of the phase parity.  A thread whose phase is not complete is
 // suspended in hardware until it completes or up to kSuspendNs (the
 // instruction's time hint) have passed, instead of spinning through issue
