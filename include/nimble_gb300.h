@@ -98,8 +98,10 @@ typedef struct nsm_material {
 
 typedef struct nsm_options {
   int precision;     /* NSM_PRECISION_* */
-  int store_ip_data; /* 1: write F and sigma per integration point every step (the
-                        ModelData element-data contract); 0: only on output steps */
+  int store_ip_data; /* 1: F and sigma per integration point are those of the latest step
+                        whenever they can be read (the ModelData element-data contract; a
+                        step whose records the next one overwrites within the same
+                        nsm_advance does not write them); 0: only of output steps */
   int device;        /* CUDA device ordinal */
   int graph_steps;   /* steps per captured CUDA graph in nsm_advance (0 = default 50) */
 } nsm_options;

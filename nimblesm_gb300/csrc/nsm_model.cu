@@ -481,14 +481,14 @@ cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
     if (timed) {
       auto ev = next_events(m->ev_elem, m->ev_elem_used);
       cudaEventRecord(ev.first, m->stream);
-      if ((e = launch_element(m, k, true)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, k + 1 == K)) != cudaSuccess) return e;
       cudaEventRecord(ev.second, m->stream);
       auto en = next_events(m->ev_node, m->ev_node_used);
       cudaEventRecord(en.first, m->stream);
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
       cudaEventRecord(en.second, m->stream);
     } else {
-      if ((e = launch_element(m, k, true)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, k + 1 == K)) != cudaSuccess) return e;
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
     }
   }
