@@ -225,7 +225,7 @@ int nsm_mlp_train(nsm_mlp* m, int epochs, int batch_tiles, double lr, double* fi
       const double lr_t  = lr * (0.01 + 0.99 * 0.5 * (1.0 + std::cos(3.141592653589793 * frac)));
       float* d_loss = ep == epochs - 1 ? d_epoch_loss + st * batch_tiles : m->d_loss;
       MLP_CUDA(launch_train(tiles, m->d_X, m->d_Y, m->n, first, a, b, m->d_img, m->d_P, m->sc, (float)(1.0 / pts),
-                            m->d_grad, d_loss, m->d_status, m->stream));
+                            m->d_grad, d_loss, m->d_status, st > 0, m->stream));
       MLP_CUDA(launch_adam(tiles, m->d_grad, m->d_P, m->d_m1, m->d_m2, (float)lr_t, (float)beta1, (float)beta2,
                            (float)eps, (float)(1.0 - std::pow(beta1, (double)k)), (float)(1.0 - std::pow(beta2, (double)k)),
                            m->d_img, m->stream));
@@ -295,7 +295,7 @@ int nsm_mlp_gradient(nsm_mlp* m, long n, const float* H, const float* Y, float* 
   if (e == cudaSuccess) e = cudaMemcpyAsync(dY, Y, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, m->stream);
   if (e == cudaSuccess)
     e = launch_train(tiles, dH, dY, n, 0, 1, 0, m->d_img, m->d_P, m->sc, (float)(1.0 / n), m->d_grad, m->d_loss,
-                     m->d_status, m->stream);
+                     m->d_status, false, m->stream);
   if (e == cudaSuccess) e = launch_sum_gradient(tiles, m->d_grad, dg, m->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(grad, dg, sizeof(float) * kParams, cudaMemcpyDeviceToHost, m->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(lp.data(), m->d_loss, sizeof(float) * tiles, cudaMemcpyDeviceToHost, m->stream);

@@ -120,22 +120,37 @@ __global__ void k_images(const float* __restrict__ P, uint8_t* __restrict__ img)
 // Training step: one tile of 128 points per CTA (thread r <-> point r, whose
 // accumulator row is tensor-memory lane r).  Writes this CTA's gradient of
 // the mean-squared residual loss and its loss sum.
+//
+// Bound: the serial chain of six dependent MMA rounds and the two launches of
+// a step; the tensor pipe is busy a few percent of the time.  The rounds are
+// therefore kept short:
+//   * Every activation and gradient is written once, as rows [point][feature].
+//     The forward and data-gradient products read the rows K-major (K =
+//     features), the weight gradients read the same bytes MN-major (K =
+//     points): an 8 x 8 core matrix of one layout is a core matrix of the
+//     other.  (Separate transposed copies were 2-byte stores four lanes to a
+//     bank, and a 130 KB region to clear first.)
+//   * Weight gradients are formed transposed, D[input][neuron], so that the 32
+//     lanes of a warp store 32 consecutive parameters.
+//   * A weight gradient is issued behind the data gradient that the chain
+//     waits for, and stored while a later round runs.
+//   * The pairs are gathered before the wait for the previous step's Adam
+//     launch (programmatic dependent launch).
 namespace tr {
-constexpr int X    = 0;                        // [128][32]
-constexpr int A1   = X + 128 * kInX * 2;       // [128][64]
-constexpr int A2   = A1 + 128 * kHid * 2;      // [128][64]
-constexpr int DZ3  = A2 + 128 * kHid * 2;      // [128][16]
-constexpr int DZ2  = DZ3 + 128 * kOutX * 2;    // [128][64]
-constexpr int AOP  = DZ2 + 128 * kHid * 2;     // [128][128 points]: dZ2^T rows 0-63, dZ1^T 64-127
-constexpr int BOP  = AOP + 128 * 128 * 2;      // [112][128]: A1^T 0-63, X^T 64-95, ones 96
-constexpr int AOP3 = BOP + 112 * 128 * 2;      // [128][128]: dZ3^T rows 0-5, zeros elsewhere
-constexpr int BOP3 = AOP3 + 128 * 128 * 2;     // [80][128]: A2^T 0-63, ones 64
-constexpr int W    = BOP3 + 80 * 128 * 2;      // operand images
+// rows [128][kF]: A1 at columns 0-63, the extended input X at 64-95, A2 at
+// 96-159; and [128][kD]: dZ2 at 0-63, dZ1 at 64-127, dZ3 at 128-143
+constexpr int kF = 160, cA1 = 0, cX = 64, cA2 = 96;
+constexpr int kD = 144, cD2 = 0, cD1 = 64, cD3 = 128;
+constexpr int F    = 0;
+constexpr int D    = F + 128 * kF * 2;
+constexpr int W    = D + 128 * kD * 2;         // operand images
 constexpr int B    = W + kImgBytes;            // b2[64], b3[6]
-constexpr int END  = B + 512;
-constexpr int SMEM = END + 16384;              // slack past the last operand
-// tensor-memory columns
-constexpr uint32_t cZ1 = 0, cZ2 = 64, cZ3 = 128, cDA2 = 144, cDA1 = 208, cGW = 272, cGW3 = 384, kCols = 512;
+constexpr int SMEM = B + 512;
+// tensor-memory columns; the weight gradients take over columns whose values
+// have been read (W2's those of Z2, W1's those of Z1, W3's those of Z3)
+constexpr uint32_t cZ1 = 0, cZ2 = 64, cDA = 128, cZ3 = 192, kCols = 256;
+constexpr uint32_t cGW1 = cZ1, cGW2 = cZ2, cGW3 = cZ3;
+constexpr int      kOnes = cX + 9;             // column of F that is 1 (the bias column of X)
 }  // namespace tr
 
 struct Sync {
@@ -185,6 +200,18 @@ __device__ __forceinline__ void gemm(uint32_t d, const uint8_t* a, int a_rows_k,
   }
 }
 
+// D[128][N] = A^T B over the 128 points of two row tiles [128][a_width],
+// [128][b_width]: both operands MN-major, a and b at the first of their 128
+// and N columns.  A's columns may run past its rows' end (into the next rows,
+// or what follows the tile): they give rows of D that nobody reads.
+__device__ __forceinline__ void gemm_points(uint32_t d, const uint8_t* a, int a_width, const uint8_t* b, int b_width, int N)
+{
+  const uint32_t idesc = idesc_bf16_f32(128, N) | kIdescMnMajor;
+  for (int ks = 0; ks < 128 / 16; ks++)
+    mma_bf16(d, smem_desc(smem_addr(a) + ks * 2 * 16 * a_width, 16 * a_width, 128),
+             smem_desc(smem_addr(b) + ks * 2 * 16 * b_width, 16 * b_width, 128), idesc, ks > 0);
+}
+
 // Two warpgroups per tile: thread t owns row r = t % 128 (tensor-memory lane r)
 // and, in the 64-column epilogues, the columns [32 h, 32 h + 32) of half
 // h = t / 128, so each thread's share of the activation and gradient work is
@@ -194,60 +221,39 @@ constexpr int kTrainThreads = 256;
 
 __global__ void __launch_bounds__(kTrainThreads) k_train(const float* __restrict__ X, const float* __restrict__ Y,
                                                          long n, long first, long stride_a, long offset_b,
-                                                         const uint8_t* __restrict__ img, const float* __restrict__ P,
+                                                         const uint8_t* img, const float* P,
                                                          Scales sc, float inv_batch, float* __restrict__ grad_partial,
                                                          float* __restrict__ loss_partial, int* __restrict__ status)
 {
   extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ uint64_t mbar;
+  __shared__ uint64_t mbar, mbar_w3, mbar_w2;
   __shared__ uint32_t tslot;
   __shared__ int      err;
   __shared__ float    red[128];
-  const int           tid = threadIdx.x, warp = tid >> 5, r = tid & 127, half = tid >> 7;
+  const int           tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid & 127, half = tid >> 7;
   const int           c0  = 32 * half;  // this thread's first column in the 64-column epilogues
 
-  // The point's pair (half 0) is gathered first, from its row of the epoch's
-  // visiting order, so that the loads' latency passes while the operand
-  // regions below are set up.
+  // The point's pair (half 0), from its row of the epoch's visiting order.
   const long j     = first + (long)blockIdx.x * 128 + r;
   const bool valid = j < n;
   float      x[9], y[6];
   if (half == 0) {
     const long idx = valid ? (long)((stride_a * j + offset_b) % n) : 0;
 #pragma unroll
-    for (int q = 0; q < 9; q++) x[q] = X[9 * idx + q];
+    for (int q = 0; q < 9; q++) x[q] = __ldg(&X[9 * idx + q]);
 #pragma unroll
-    for (int q = 0; q < 6; q++) y[q] = Y[6 * idx + q];
+    for (int q = 0; q < 6; q++) y[q] = __ldg(&Y[6 * idx + q]);
   }
-
   if (warp == 0) {
     tmem_alloc(&tslot, tr::kCols);
     tmem_relinquish();
   }
   if (tid == 0) {
     mbar_init(&mbar, 1);
+    mbar_init(&mbar_w3, 1);
+    mbar_init(&mbar_w2, 1);
     err = 0;
   }
-  // constant operand regions (zero rows, ones rows), weight images, biases
-  {
-    uint4 z = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < (tr::W - tr::AOP) / 16; i += kTrainThreads) reinterpret_cast<uint4*>(sm + tr::AOP)[i] = z;
-    const uint4* src = reinterpret_cast<const uint4*>(img);
-    for (int i = tid; i < kImgBytes / 16; i += kTrainThreads) reinterpret_cast<uint4*>(sm + tr::W)[i] = src[i];
-    float* bias = reinterpret_cast<float*>(sm + tr::B);
-    if (tid < kHid) bias[tid] = P[ob2 + tid];
-    if (tid < kOut) bias[64 + tid] = P[ob3 + tid];
-  }
-  __syncthreads();
-  if (half == 0) {
-    store_bf16(sm + tr::BOP, 96, r, 128, 1.0f);
-    store_bf16(sm + tr::BOP3, 64, r, 128, 1.0f);
-  }
-  const float* b2 = reinterpret_cast<const float*>(sm + tr::B);
-  const float* b3 = b2 + 64;
-  const uint32_t tb = tslot;
-  Sync           sy{&mbar, 0u, &err};
-
   // ---- the point (half 0: its input row and target) ----
   float t[6];
   if (half == 0) {
@@ -261,15 +267,34 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(const float* __restrict
     }
     float row[kInX];
     input_row(xs, row);
-    for (int k0 = 0; k0 < kInX; k0 += 8) store_chunk(sm + tr::X, r, k0, kInX, row + k0);
-    for (int q = 0; q < kInX; q++)
-      if (q < 10 || (q >= 16 && q < 25)) store_bf16(sm + tr::BOP, 64 + q, r, 128, row[q]);
+    for (int k0 = 0; k0 < kInX; k0 += 8) store_chunk(sm + tr::F, r, tr::cX + k0, tr::kF, row + k0);
+  }
+  // ---- what the previous step's Adam launch wrote: weight images, biases ----
+  wait_prerequisites();
+  launch_dependents();  // (not before the wait: this step's Adam launch reads the state that the previous one wrote)
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(img);
+    for (int i = tid; i < kImgBytes / 16; i += kTrainThreads) reinterpret_cast<uint4*>(sm + tr::W)[i] = __ldcg(src + i);
+    float* bias = reinterpret_cast<float*>(sm + tr::B);
+    if (tid < kHid) bias[tid] = __ldcg(&P[ob2 + tid]);
+    if (tid < kOut) bias[64 + tid] = __ldcg(&P[ob3 + tid]);
   }
   publish_operands();
+  const float*   b2 = reinterpret_cast<const float*>(sm + tr::B);
+  const float*   b3 = b2 + 64;
+  const uint32_t tb = tslot;
+  Sync           sy{&mbar, 0u, &err};
+  float* const   G  = grad_partial + (long)blockIdx.x * kParams;
+  const uint8_t* Xop = sm + tr::F + tr::cX * 16;  // column c of a row tile starts 16 c bytes in
+  const uint8_t* A1op = sm + tr::F + tr::cA1 * 16;
+  const uint8_t* A2op = sm + tr::F + tr::cA2 * 16;
+  const uint8_t* D1op = sm + tr::D + tr::cD1 * 16;
+  const uint8_t* D2op = sm + tr::D + tr::cD2 * 16;
+  const uint8_t* D3op = sm + tr::D + tr::cD3 * 16;
 
   // ---- forward ----
   if (tid == 0) {
-    gemm(tb + tr::cZ1, sm + tr::X, kInX, sm + tr::W + kOffW1, kInX, kHid, kInX, false);
+    gemm(tb + tr::cZ1, Xop, tr::kF, sm + tr::W + kOffW1, kInX, kHid, kInX, false);
     mma_commit(&mbar);
   }
   if (!await_mma(sy)) goto cleanup;
@@ -277,12 +302,11 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(const float* __restrict
     float z[32];
     ld_row(tb, tr::cZ1 + c0, 2, z);
     for (int q = 0; q < 32; q++) z[q] = act(z[q]);
-    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::A1, r, c0 + k0, kHid, z + k0);
-    for (int q = 0; q < 32; q++) store_bf16(sm + tr::BOP, c0 + q, r, 128, z[q]);
+    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::F, r, tr::cA1 + c0 + k0, tr::kF, z + k0);
   }
   publish_operands();
   if (tid == 0) {
-    gemm(tb + tr::cZ2, sm + tr::A1, kHid, sm + tr::W + kOffW2, kHid, kHid, kHid, false);
+    gemm(tb + tr::cZ2, A1op, tr::kF, sm + tr::W + kOffW2, kHid, kHid, kHid, false);
     mma_commit(&mbar);
   }
   if (!await_mma(sy)) goto cleanup;
@@ -290,12 +314,11 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(const float* __restrict
     float z[32];
     ld_row(tb, tr::cZ2 + c0, 2, z);
     for (int q = 0; q < 32; q++) z[q] = act(z[q] + b2[c0 + q]);
-    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::A2, r, c0 + k0, kHid, z + k0);
-    for (int q = 0; q < 32; q++) store_bf16(sm + tr::BOP3, c0 + q, r, 128, z[q]);
+    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::F, r, tr::cA2 + c0 + k0, tr::kF, z + k0);
   }
   publish_operands();
   if (tid == 0) {
-    gemm(tb + tr::cZ3, sm + tr::A2, kHid, sm + tr::W + kOffW3, kHid, kOutX, kHid, false);
+    gemm(tb + tr::cZ3, A2op, tr::kF, sm + tr::W + kOffW3, kHid, kOutX, kHid, false);
     mma_commit(&mbar);
   }
   if (!await_mma(sy)) goto cleanup;
@@ -310,73 +333,88 @@ __global__ void __launch_bounds__(kTrainThreads) k_train(const float* __restrict
       g[q] = 2.0f * d * inv_batch;
     }
     red[r] = lsum;
-    for (int k0 = 0; k0 < 16; k0 += 8) store_chunk(sm + tr::DZ3, r, k0, kOutX, g + k0);
-    for (int q = 0; q < kOut; q++) store_bf16(sm + tr::AOP3, q, r, 128, g[q]);
+    for (int k0 = 0; k0 < 16; k0 += 8) store_chunk(sm + tr::D, r, tr::cD3 + k0, tr::kD, g + k0);
   }
   publish_operands();
   // ---- backward ----
   if (tid == 0) {
-    gemm(tb + tr::cDA2, sm + tr::DZ3, kOutX, sm + tr::W + kOffW3t, kOutX, kHid, kOutX, false);
+    gemm(tb + tr::cDA, D3op, tr::kD, sm + tr::W + kOffW3t, kOutX, kHid, kOutX, false);
     mma_commit(&mbar);
+    gemm_points(tb + tr::cGW3, Xop, tr::kF, D3op, tr::kD, kOutX);  // rows 0-31 X (its ones: b3), 32-95 A2
+    mma_commit(&mbar_w3);
   }
   if (!await_mma(sy)) goto cleanup;
   {
     float da[32], z[32];
-    ld_row(tb, tr::cDA2 + c0, 2, da);
+    ld_row(tb, tr::cDA + c0, 2, da);
     ld_row(tb, tr::cZ2 + c0, 2, z);
     for (int q = 0; q < 32; q++) da[q] *= act_grad(z[q] + b2[c0 + q]);
-    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::DZ2, r, c0 + k0, kHid, da + k0);
-    for (int q = 0; q < 32; q++) store_bf16(sm + tr::AOP, c0 + q, r, 128, da[q]);
+    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::D, r, tr::cD2 + c0 + k0, tr::kD, da + k0);
   }
   publish_operands();
   if (tid == 0) {
-    gemm(tb + tr::cDA1, sm + tr::DZ2, kHid, sm + tr::W + kOffW2t, kHid, kHid, kHid, false);
+    gemm(tb + tr::cDA, D2op, tr::kD, sm + tr::W + kOffW2t, kHid, kHid, kHid, false);
     mma_commit(&mbar);
+    gemm_points(tb + tr::cGW2, A1op, tr::kF, D2op, tr::kD, kHid);  // rows 0-63 A1, 64-95 X (its ones: b2)
+    mma_commit(&mbar_w2);
+  }
+  // W3's gradient, while the data gradient is formed
+  if (!mbar_wait(&mbar_w3, 0u)) atomicOr(&err, 1);
+  fence_after_sync();
+  if (half == 1 && warp < 7) {
+    float w[16];
+    ld_row(tb, tr::cGW3, 1, w);
+    if (warp == 4) {
+      if (lane == tr::kOnes - tr::cX)
+        for (int o = 0; o < kOut; o++) G[ob3 + o] = w[o];
+    } else {
+      for (int o = 0; o < kOut; o++) G[oW3 + o * kHid + (r - 32)] = w[o];
+    }
   }
   if (!await_mma(sy)) goto cleanup;
   {
     float da[32], z[32];
-    ld_row(tb, tr::cDA1 + c0, 2, da);
+    ld_row(tb, tr::cDA + c0, 2, da);
     ld_row(tb, tr::cZ1 + c0, 2, z);
-    for (int q = 0; q < 32; q++) store_bf16(sm + tr::AOP, 64 + c0 + q, r, 128, da[q] * act_grad(z[q]));
+    for (int q = 0; q < 32; q++) da[q] *= act_grad(z[q]);
+    for (int k0 = 0; k0 < 32; k0 += 8) store_chunk(sm + tr::D, r, tr::cD1 + c0 + k0, tr::kD, da + k0);
   }
   publish_operands();
-  // weight gradients: sums over the 128 points of the tile (K = points)
   if (tid == 0) {
-    gemm(tb + tr::cGW, sm + tr::AOP, 128, sm + tr::BOP, 128, 112, 128, false);
-    gemm(tb + tr::cGW3, sm + tr::AOP3, 128, sm + tr::BOP3, 128, 80, 128, false);
+    gemm_points(tb + tr::cGW1, A1op, tr::kF, D1op, tr::kD, kHid);  // rows 64-95 X
     mma_commit(&mbar);
   }
-  if (!await_mma(sy)) goto cleanup;
-  {
-    float* G = grad_partial + (long)blockIdx.x * kParams;
-    if (half == 0) {
-      // row r of the [112] block: W2 and b2 gradients (rows < 64), W1 and b1 (rows >= 64)
-      float v[112];
-      ld_row(tb, tr::cGW, 7, v);
-      if (r < 64) {
-        for (int q = 0; q < 64; q++) G[oW2 + r * 64 + q] = v[q];
-        G[ob2 + r] = v[96];
-      } else {
-        const int o = r - 64;
-        for (int q = 0; q < 9; q++) G[oW1 + o * 9 + q] = v[64 + q] + v[64 + 16 + q];
-        G[ob1 + o] = v[64 + 9];
-      }
-    } else if (warp == 4) {  // rows 0..31 of the W3 block: W3 and b3 gradients of rows < 6
-      float w3[80];
-      ld_row(tb, tr::cGW3, 5, w3);
-      if (r < kOut) {
-        for (int q = 0; q < 64; q++) G[oW3 + r * 64 + q] = w3[q];
-        G[ob3 + r] = w3[64];
-      }
+  // W2's gradient, while W1's is formed: this half's 32 neurons
+  if (!mbar_wait(&mbar_w2, 0u)) atomicOr(&err, 1);
+  fence_after_sync();
+  if ((warp & 3) < 3) {
+    float w[32];
+    ld_row(tb, tr::cGW2 + c0, 2, w);
+    if (r < 64) {
+      for (int q = 0; q < 32; q++) G[oW2 + (c0 + q) * kHid + r] = w[q];
+    } else if (r == tr::kOnes) {
+      for (int q = 0; q < 32; q++) G[ob2 + c0 + q] = w[q];
     }
   }
-  __syncthreads();
-  for (int w = 64; w > 0; w >>= 1) {
-    if (tid < w) red[tid] += red[tid + w];
-    __syncthreads();
+  if (half == 1 && tid < 192) {  // the tile's loss, summed in a fixed order by two warps
+    float l = red[tid - 128] + red[tid - 64];
+    red[tid - 128] = l;
   }
-  if (tid == 0) loss_partial[blockIdx.x] = red[0];
+  if (!await_mma(sy)) goto cleanup;
+  if ((warp & 3) == 2) {  // rows 64-95: inputs X; the input's two terms are lanes q and 16 + q
+    float w[32];
+    ld_row(tb, tr::cGW1 + c0, 2, w);
+    for (int q = 0; q < 32; q++) {
+      const float lo = __shfl_down_sync(0xffffffffu, w[q], 16);
+      if (lane < kIn) G[oW1 + (c0 + q) * kIn + lane] = w[q] + lo;
+      else if (lane == 9) G[ob1 + c0 + q] = w[q];
+    }
+  } else if (warp == 0) {
+    float l = red[lane] + red[lane + 32];
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) l += __shfl_down_sync(0xffffffffu, l, w);
+    if (lane == 0) loss_partial[blockIdx.x] = l;
+  }
 
 cleanup:
   if (tid == 0 && err) {
@@ -412,40 +450,49 @@ __device__ __forceinline__ void store_images(int i, float w, uint8_t* __restrict
 
 // Deterministic reduction of the per-CTA gradients, an Adam step on the FP32
 // master parameters, and the new parameters' BF16 operand-image entries.
-// Eight lanes share a parameter: lane j sums the partials of CTAs j, j + 8,
-// ... in order (loads issued four at a time ahead of the in-order sum), and
-// three butterfly steps combine the eight sums in a fixed order, so every
-// run gives the same bits while a launch has many loads in flight.
-constexpr int kAdamLanes = 8;
-__global__ void k_adam(int ncta, const float* __restrict__ grad_partial, float* __restrict__ P,
-                       float* __restrict__ m1, float* __restrict__ m2, float lr, float beta1, float beta2,
-                       float eps, float bc1, float bc2, uint8_t* __restrict__ img)
+// Bound: the latency of the partials' loads.  Eight warps share 32 parameters:
+// warp j sums the partials of CTAs j, j + 8, ... in order (a 128-byte row per
+// load, up to 20 in flight ahead of the in-order sum), and the eight sums are
+// combined in a fixed order, so every run gives the same bits.
+constexpr int kAdamWarps = 8, kAdamAhead = 20;
+__global__ void __launch_bounds__(32 * kAdamWarps) k_adam(int ncta, const float* grad_partial, float* __restrict__ P,
+                                                          float* __restrict__ m1, float* __restrict__ m2, float lr,
+                                                          float beta1, float beta2, float eps, float bc1, float bc2,
+                                                          uint8_t* __restrict__ img)
 {
-  const long t   = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int  i   = (int)(t / kAdamLanes), sub = (int)(t % kAdamLanes);
-  const bool own = i < kParams;
-  float      g   = 0.0f;
+  __shared__ float sums[kAdamWarps][32];
+  const int        lane = threadIdx.x & 31, sub = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  const bool       own = i < kParams;
+  launch_dependents();
+  // (the state is the previous Adam launch's, which had ended when this step's training launch let this one start)
+  float a0 = 0.0f, b0 = 0.0f, p0 = 0.0f;
+  if (sub == 0 && own) a0 = m1[i], b0 = m2[i], p0 = P[i];
+  wait_prerequisites();
+  float g = 0.0f;
   if (own) {
     const float* gp = grad_partial + i;
-    int          c  = sub;
-    for (; c + 3 * kAdamLanes < ncta; c += 4 * kAdamLanes) {
-      const float p0 = gp[(long)c * kParams], p1 = gp[(long)(c + kAdamLanes) * kParams],
-                  p2 = gp[(long)(c + 2 * kAdamLanes) * kParams], p3 = gp[(long)(c + 3 * kAdamLanes) * kParams];
-      g += p0;
-      g += p1;
-      g += p2;
-      g += p3;
-    }
-    for (; c < ncta; c += kAdamLanes) g += gp[(long)c * kParams];
-  }
+    for (int c = sub; c < ncta; c += kAdamAhead * kAdamWarps) {
+      float v[kAdamAhead];
 #pragma unroll
-  for (int o = 1; o < kAdamLanes; o <<= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-  if (!own || sub != 0) return;
-  float a = beta1 * m1[i] + (1.0f - beta1) * g;
-  float b = beta2 * m2[i] + (1.0f - beta2) * g * g;
-  m1[i]   = a;
-  m2[i]   = b;
-  const float w = P[i] - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+      for (int k = 0; k < kAdamAhead; k++)
+        if (c + k * kAdamWarps < ncta) v[k] = __ldcg(&gp[(long)(c + k * kAdamWarps) * kParams]);
+#pragma unroll
+      for (int k = 0; k < kAdamAhead; k++)
+        if (c + k * kAdamWarps < ncta) g += v[k];
+    }
+  }
+  sums[sub][lane] = g;
+  __syncthreads();
+  if (sub != 0 || !own) return;
+  float s[kAdamWarps];
+#pragma unroll
+  for (int k = 0; k < kAdamWarps; k++) s[k] = sums[k][lane];
+  g = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+  const float a = fmaf(1.0f - beta1, g, beta1 * a0);
+  const float b = fmaf((1.0f - beta2) * g, g, beta2 * b0);
+  m1[i]         = a;
+  m2[i]         = b;
+  const float w = p0 - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
   P[i]          = w;
   store_images(i, w, img);
 }
@@ -599,21 +646,38 @@ cudaError_t setup_kernels()
   return cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, inf::SMEM);
 }
 
+// `overlap`: the launch may begin before the previous kernel of the stream has
+// ended (it waits for it before it reads or writes what the two share).
+template <class... Params, class... Args>
+static cudaError_t launch_overlapped(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s, bool overlap,
+                                     Args... args)
+{
+  cudaLaunchAttribute attr;
+  attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg                          = {};
+  cfg.gridDim                                     = dim3((unsigned)grid);
+  cfg.blockDim                                    = dim3((unsigned)block);
+  cfg.dynamicSmemBytes                            = smem;
+  cfg.stream                                      = s;
+  cfg.attrs                                       = &attr;
+  cfg.numAttrs                                    = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 cudaError_t launch_train(int tiles, const float* X, const float* Y, long n, long first, long stride_a, long offset_b,
                          const uint8_t* img, const float* P, const Scales& sc, float inv_batch, float* grad_partial,
-                         float* loss_partial, int* status, cudaStream_t s)
+                         float* loss_partial, int* status, bool after_adam, cudaStream_t s)
 {
-  k_train<<<tiles, kTrainThreads, tr::SMEM, s>>>(X, Y, n, first, stride_a, offset_b, img, P, sc, inv_batch, grad_partial,
-                                       loss_partial, status);
-  return cudaGetLastError();
+  return launch_overlapped(k_train, tiles, kTrainThreads, tr::SMEM, s, after_adam, X, Y, n, first, stride_a, offset_b, img, P,
+                           sc, inv_batch, grad_partial, loss_partial, status);
 }
 
 cudaError_t launch_adam(int ncta, const float* grad_partial, float* P, float* m1, float* m2, float lr, float beta1,
                         float beta2, float eps, float bc1, float bc2, uint8_t* img, cudaStream_t s)
 {
-  k_adam<<<(kParams * kAdamLanes + 255) / 256, 256, 0, s>>>(ncta, grad_partial, P, m1, m2, lr, beta1, beta2, eps,
-                                                             bc1, bc2, img);
-  return cudaGetLastError();
+  return launch_overlapped(k_adam, (kParams + 31) / 32, 32 * kAdamWarps, 0, s, true, ncta, grad_partial, P, m1, m2, lr, beta1,
+                           beta2, eps, bc1, bc2, img);
 }
 
 cudaError_t launch_sum_gradient(int ncta, const float* grad_partial, float* g, cudaStream_t s)

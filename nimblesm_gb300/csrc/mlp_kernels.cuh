@@ -16,11 +16,13 @@ cudaError_t launch_residual_moment(long n, const float* X, const float* Y, float
                                    double* partial, int blocks, cudaStream_t s);
 cudaError_t launch_images(const float* P, uint8_t* img, cudaStream_t s);
 // One training step over `tiles` tiles of 128 points: point j = first + tile*128 + lane
-// is sample (stride_a * j + offset_b) mod n.
+// is sample (stride_a * j + offset_b) mod n.  after_adam: the stream's previous
+// kernel is a launch_adam, which this one may overlap until it needs the
+// weights (the pairs, written before, are read ahead of that).
 cudaError_t launch_train(int tiles, const float* X, const float* Y, long n, long first, long stride_a, long offset_b,
                          const uint8_t* img, const float* P, const Scales& sc, float inv_batch, float* grad_partial,
-                         float* loss_partial, int* status, cudaStream_t s);
-// Sum of the per-CTA gradients, Adam step, and the updated parameters' BF16
+                         float* loss_partial, int* status, bool after_adam, cudaStream_t s);
+// Right after launch_train: sum of the per-CTA gradients, Adam step, and the updated parameters' BF16
 // operand-image entries (img, written in place).
 cudaError_t launch_adam(int ncta, const float* grad_partial, float* P, float* m1, float* m2, float lr, float beta1,
                         float beta2, float eps, float bc1, float bc2, uint8_t* img, cudaStream_t s);

@@ -58,6 +58,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// Added to the above: both operands MN-major (bits 15 and 16).  Without swizzle
+// such an operand is stored as the same 128-byte core matrices, 8 K-rows of 8
+// consecutive MN elements; SBO is then the distance between MN-adjacent core
+// matrices and LBO that between K-adjacent ones.
+constexpr uint32_t kIdescMnMajor = (1u << 15) | (1u << 16);
+
 // ---- tensor memory ----
 // Allocation by one full warp; the allocated base address is written to
 // shared memory at `slot`.
@@ -115,6 +121,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v)
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---- programmatic dependent launch ----
+// The stream's next kernel, if launched so, may start; and wait for the end
+// (and the writes) of the previous one.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count)

@@ -207,3 +207,25 @@ def test_closure_over_the_full_schedule():
           f"energy drift {drift:.3e} (FP64 plain {drift64:.3e}), fallbacks {fallbacks}")
     assert e_u < 1e-3
     assert abs(drift) < 1e-2
+
+
+@pytest.mark.parametrize("pairs, tiles", [(100, 1), (128, 2), (20_001, 160), (51_163, 400)])
+def test_one_training_step_is_adam_on_the_gradient(pairs, tiles):
+    """A step over one partial tile, an empty second one, a last wave of tiles
+    and more tiles than the GPU holds at once: from zero moments the step is
+    lr g / (|g| + eps), g the gradient of the whole set (summed in another
+    order: 2^-24 sqrt(tiles) relative to the largest terms, so entries within
+    1e-3 of the largest are held to 1e-3 of a step)."""
+    m = E.MLPClosure(K, G, seed=2)
+    m.generate(pairs, seed=5)
+    P0, _ = m.params()
+    H, Y = m.training_sample(0, pairs)
+    g, loss = m.gradient(H, Y)
+    lr = 2e-3
+    final = m.train(epochs=1, batch_tiles=tiles, lr=lr)
+    P1, _ = m.params()
+    assert abs(final * 6.0 - loss) <= 1e-5 * loss
+    big = np.abs(g) > 1e-3 * np.abs(g).max()
+    step = P0 - lr * np.sign(g) - P1  # one step of the schedule runs at the full rate
+    assert np.abs(step[big]).max() <= 1e-3 * lr
+    m.close()
