@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256, sizeof(TF) == 4 ? 5 : 4) k_node_update(No
       v[i]   = axpy<kExact>(s.half, acc[i], a.v[i * ld + n]);
       u[i]   = a.u[i * ld + n];
     }
-    if (s.is_output && slot >= 0) apply_bc(bc, s.delta, a.bc_expr_val ? a.bc_expr_val + (long)slot * 3 : nullptr, u, v);
+    if (s.is_output && slot >= 0) apply_bc(bc, s.delta, a.bc_expr_post ? a.bc_expr_post + (long)slot * 3 : nullptr, u, v);
   } else {
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256, sizeof(TF) == 4 ? 5 : 4) k_node_update(No
     const StepSched s = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
 #pragma unroll
     for (int i = 0; i < 3; i++) v[i] = axpy<kExact>(s.half, acc[i], v[i]);
-    const double* ev = a.bc_expr_val ? a.bc_expr_val + ((long)a.num_bc_slots + slot) * 3 : nullptr;
+    const double* ev = a.bc_expr_pre ? a.bc_expr_pre + (long)slot * 3 : nullptr;
     if (slot >= 0) apply_bc(bc, s.delta, ev, u, v);
 #pragma unroll
     for (int i = 0; i < 3; i++) u[i] = axpy<kExact>(s.delta, v[i], u[i]);
@@ -261,27 +261,25 @@ cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream)
   return cudaGetLastError();
 }
 
-__global__ void k_bc_expr_values(NodeArgs a, const int* __restrict__ slot_node, BcExprTable ex, double* __restrict__ out)
+// One thread per (slot, component) and step (grid row): a program's latency on
+// the FP64 pipe (a sine takes about 15 us) is that of one evaluation however
+// many steps are evaluated at once.
+__global__ void k_bc_expr_values(BcExprSteps q, BcExprTable ex, double* __restrict__ out)
 {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.num_bc_slots) return;
-  const NodeBC bc    = a.bcs[s];
-  const int    n     = slot_node[s];
-  const int    group = a.node_group ? a.node_group[n] : 0;
-  for (int level = 0; level < 2; level++) {
-    const int k = level == 0 ? a.k_post : a.k_pre;
-    if (k < 0) continue;
-    const double t = a.sched[(long)(*a.step_base + k) * a.num_groups + group].time;
-    for (int c = 0; c < 3; c++)
-      if (bc.expr[c] >= 0) out[((long)level * a.num_bc_slots + s) * 3 + c] = eval_bc_expression(ex, bc.expr[c], n, t);
-  }
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * q.num_slots) return;
+  const int s = t / 3, c = t % 3, prog = q.bcs[s].expr[c];
+  if (prog < 0) return;
+  const int    n     = q.slot_node[s];
+  const int    group = q.node_group ? q.node_group[n] : 0;
+  const double time  = q.sched[(long)(*q.step_base + q.k + blockIdx.y) * q.num_groups + group].time;
+  out[(long)blockIdx.y * 3 * q.num_slots + t] = eval_bc_expression(ex, prog, n, time);
 }
 
-cudaError_t launch_bc_expr_values(const NodeArgs& a, const int* slot_node, const BcExprTable& ex, double* out,
-                                  cudaStream_t stream)
+cudaError_t launch_bc_expr_values(const BcExprSteps& q, int steps, const BcExprTable& ex, double* out, cudaStream_t stream)
 {
-  if (a.num_bc_slots == 0) return cudaSuccess;
-  k_bc_expr_values<<<grid_for(a.num_bc_slots, 128), 128, 0, stream>>>(a, slot_node, ex, out);
+  if (q.num_slots == 0 || steps == 0) return cudaSuccess;
+  k_bc_expr_values<<<dim3(grid_for(3L * q.num_slots, 128), steps), 128, 0, stream>>>(q, ex, out);
   return cudaGetLastError();
 }
 

@@ -39,6 +39,9 @@ int cuda_fail(cudaError_t e, const char* where)
     if (_e != cudaSuccess) return cuda_fail(_e, #call);   \
   } while (0)
 
+// Largest half of a model's table of expression values.
+constexpr size_t kBcExprBytes = 8 << 20;
+
 long pad(long n, long q) { return (n + q - 1) / q * q; }
 
 struct BcLine {
@@ -123,7 +126,10 @@ struct nsm_model {
   int                      num_bc_slots = 0;          // nodes with a kinematic condition
   int*                     d_bc_slot_node = nullptr;  // [num_bc_slots] their node ids
   bool                     bc_has_expr = false;       // some kinematic condition is an expression
-  double*                  d_bc_expr_val = nullptr;   // [2][num_bc_slots][3] values per node launch
+  // their values, evaluated for bc_expr_rows steps of a launch sequence at a
+  // time: [2 * bc_expr_rows][num_bc_slots][3], the halves in turn
+  double*                  d_bc_expr_val = nullptr;
+  int                      bc_expr_rows = 0;
   int*                d_bc_slot = nullptr;
   NodeBC*             d_bcs = nullptr;
   int*                d_ibc_slot = nullptr;
@@ -254,8 +260,10 @@ int upload_bcs(nsm_model* m)
         NSM_CUDA(cudaMalloc(&m->d_bc_slot_node, sizeof(int) * slot_node.size()));
         NSM_CUDA(cudaMemcpyAsync(m->d_bc_slot_node, slot_node.data(), sizeof(int) * slot_node.size(),
                                  cudaMemcpyHostToDevice, m->stream));
-        NSM_CUDA(cudaMalloc(&m->d_bc_expr_val, sizeof(double) * 6 * slot_node.size()));
-        NSM_CUDA(cudaMemsetAsync(m->d_bc_expr_val, 0, sizeof(double) * 6 * slot_node.size(), m->stream));
+        const size_t row = sizeof(double) * 3 * slot_node.size();
+        m->bc_expr_rows  = (int)std::min<size_t>(m->graph_steps, std::max<size_t>(1, kBcExprBytes / row));
+        NSM_CUDA(cudaMalloc(&m->d_bc_expr_val, row * 2 * m->bc_expr_rows));
+        NSM_CUDA(cudaMemsetAsync(m->d_bc_expr_val, 0, row * 2 * m->bc_expr_rows, m->stream));
       }
     }
     NSM_CUDA(cudaStreamSynchronize(m->stream));  // host vectors go out of scope
@@ -335,6 +343,13 @@ nsm::BcExprTable expr_table(const nsm_model* m)
   return nsm::BcExprTable{m->d_expr_code, m->d_expr_start, m->d_X, m->ld_n};
 }
 
+// The row of expression values of schedule offset k, or null.
+const double* bc_expr_row(const nsm_model* m, int k)
+{
+  if (!m->bc_has_expr || k < 0) return nullptr;
+  return m->d_bc_expr_val + (size_t)(k % (2 * m->bc_expr_rows)) * 3 * m->num_bc_slots;
+}
+
 nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
 {
   nsm::NodeArgs a;
@@ -367,8 +382,8 @@ nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
   a.closure_first = m->closure_first;
   a.num_exact     = m->num_exact;
   a.node_off      = m->d_node_off;
-  a.bc_expr_val   = m->bc_has_expr ? m->d_bc_expr_val : nullptr;
-  a.num_bc_slots  = m->num_bc_slots;
+  a.bc_expr_post  = bc_expr_row(m, k_post);
+  a.bc_expr_pre   = bc_expr_row(m, k_pre);
   return a;
 }
 
@@ -459,16 +474,19 @@ std::pair<cudaEvent_t, cudaEvent_t> next_events(std::vector<std::pair<cudaEvent_
   return pool[used++];
 }
 
-// One node launch of the time loop, after the values of its expression
-// conditions when there are any.
-cudaError_t node_step(nsm_model* m, int k_post, int k_pre)
+// One node launch of a sequence of K steps, after the values of the expression
+// conditions of the steps from k_pre on where a new group of them begins (the
+// step finished has its own in the other half).
+cudaError_t node_step(nsm_model* m, int k_post, int k_pre, int K)
 {
-  const nsm::NodeArgs a = node_args(m, k_post, k_pre, 0);
-  if (m->bc_has_expr) {
-    cudaError_t e = nsm::launch_bc_expr_values(a, m->d_bc_slot_node, expr_table(m), m->d_bc_expr_val, m->stream);
+  if (m->bc_has_expr && k_pre >= 0 && k_pre % m->bc_expr_rows == 0) {
+    const nsm::BcExprSteps q{m->num_bc_slots, m->d_bc_slot_node, m->d_bcs, m->d_sched,
+                             m->d_step_base,  m->d_node_group,   m->S,     k_pre};
+    double* out = m->d_bc_expr_val + (size_t)(k_pre % (2 * m->bc_expr_rows)) * 3 * m->num_bc_slots;
+    cudaError_t e = nsm::launch_bc_expr_values(q, std::min(m->bc_expr_rows, K - k_pre), expr_table(m), out, m->stream);
     if (e != cudaSuccess) return e;
   }
-  return nsm::launch_node_update(a, m->stream);
+  return nsm::launch_node_update(node_args(m, k_post, k_pre, 0), m->stream);
 }
 
 // Launch sequence of a chunk of K schedule steps starting at the device base:
@@ -476,7 +494,7 @@ cudaError_t node_step(nsm_model* m, int k_post, int k_pre)
 cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
 {
   cudaError_t e;
-  if ((e = node_step(m, -1, 0)) != cudaSuccess) return e;
+  if ((e = node_step(m, -1, 0, K)) != cudaSuccess) return e;
   for (int k = 0; k < K; k++) {
     if (timed) {
       auto ev = next_events(m->ev_elem, m->ev_elem_used);
@@ -485,11 +503,11 @@ cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
       cudaEventRecord(ev.second, m->stream);
       auto en = next_events(m->ev_node, m->ev_node_used);
       cudaEventRecord(en.first, m->stream);
-      if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
+      if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1, K)) != cudaSuccess) return e;
       cudaEventRecord(en.second, m->stream);
     } else {
       if ((e = launch_element(m, k, k + 1 == K)) != cudaSuccess) return e;
-      if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1)) != cudaSuccess) return e;
+      if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1, K)) != cudaSuccess) return e;
     }
   }
   return nsm::launch_advance_base(m->d_step_base, K, m->stream);

@@ -138,3 +138,28 @@ def test_random_expressions_against_the_reference_parser():
                 assert ours == ref or (np.isnan(ours) and np.isnan(ref)), (text, pt, ours, ref)
                 checked += 1
     assert checked > 900  # most of them parse
+
+
+@pytest.mark.gpu
+def test_values_evaluated_for_several_steps_at_once():
+    """The same run in launch sequences of 100 steps (7,225 driven nodes: their
+    values for 48 steps at a time, three groups in the table's two halves), of
+    7 steps, and of 1 step: bitwise the same state."""
+    from nimblesm_gb300.mesh import Problem, cube_mesh
+    n = 84
+    coords, conn = cube_mesh(n)
+    keep = conn.max(axis=1) < 2 * (n + 1) ** 2  # one layer of elements
+    coords, conn = coords[:2 * (n + 1) ** 2], conn[keep]
+    p = Problem(coords=coords, conn=conn, node_sets={"bottom": np.arange((n + 1) ** 2, dtype=np.int32)})
+    p.bcs = [BoundaryCondition.parse('prescribed_velocity bottom z "0.5 * sin(2e5 * t) * (1 + x * y)"'),
+             BoundaryCondition.parse('prescribed_displacement bottom x "1e-5 * t"')]
+    out = []
+    for graph_steps in (100, 7, 1):
+        m = E.Model(p, graph_steps=graph_steps)
+        m.begin(130 * 4e-7, 130, 10)
+        m.advance(130)
+        out.append((m.GetVectorNodeData("displacement"), m.GetVectorNodeData("velocity")))
+        m.close()
+    assert np.abs(out[0][0]).max() > 0
+    for u, v in out[1:]:
+        assert np.array_equal(u, out[0][0]) and np.array_equal(v, out[0][1])
