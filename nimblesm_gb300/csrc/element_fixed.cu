@@ -24,7 +24,6 @@
 // An element outside the fixed-point domain is evaluated by the FP64 code
 // (element_work), records included.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 
 #include "element_work.cuh"
@@ -196,6 +195,8 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
   int id[2];
   load_ids(g, id);
   stage_geo(0, g);
+  wait_prerequisites();  // the node kernel that writes u
+  launch_dependents();
   stage_u(0, id);
   cp_async_commit();
   if (g + g_step < g_end) load_ids(g + g_step, id);
@@ -399,25 +400,20 @@ template <bool kStore, bool kHasElastic>
 static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
   constexpr int     bytes = kStore ? kStageBytesStore : kStageBytes;
-  // set once per device; repeated by a thread that races the first, to the same values
   static std::atomic<unsigned long long> configured{0};
-  int               dev = 0;
-  cudaError_t       err = cudaGetDevice(&dev);
+  cudaError_t err = once_per_device(configured, [] {
+    cudaError_t e =
+        cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * bytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return e;
+  });
   if (err != cudaSuccess) return err;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(configured.load(std::memory_order_acquire) & bit)) {
-    err = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * bytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (err != cudaSuccess) return err;
-    configured.fetch_or(bit, std::memory_order_release);
-  }
   const int  warps  = l.block == 64 ? 2 : 4;
   const long groups = ((a.E + 7L) >> 3) - (a.e_begin >> 3);
   const int  per_sm = l.persistent ? l.blocks_per_sm : (kStore ? 3 : 4) * (4 / warps);
   const long grid   = std::min<long>((groups + warps - 1) / warps, (long)per_sm * num_sms());
-  k_element_fixed<kStore, kHasElastic><<<(int)grid, 32 * warps, warps * bytes, stream>>>(a);
-  return cudaGetLastError();
+  return launch_overlapped(k_element_fixed<kStore, kHasElastic>, (int)grid, 32 * warps, warps * bytes, stream, a.overlap != 0, a);
 }
 
 cudaError_t launch_element_fp64(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)

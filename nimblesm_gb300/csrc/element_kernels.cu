@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(128, 3) k_element_staged(ElementArgs a)
   if (e < a.E) stage_conn(a, e, reinterpret_cast<int*>(cur + kStageValues * B), B);
   cp_async_commit();
   cp_async_wait_all();
+  wait_prerequisites();  // the node kernel that writes u
+  launch_dependents();
   if (e < a.E) stage_nodes(a, reinterpret_cast<const int*>(cur + kStageValues * B), cur, B);
   if (e + stride < a.E) stage_conn(a, e + stride, reinterpret_cast<int*>(nxt + kStageValues * B), B);
   cp_async_commit();
@@ -173,8 +175,7 @@ cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cu
   int grid           = grid_for(a.E - a.e_begin, block);
   const int g        = (l.blocks_per_sm > 0 ? l.blocks_per_sm : 1) * num_sms();
   if (g < grid) grid = g;
-  k_element_staged<<<grid, block, smem, stream>>>(b);
-  return cudaGetLastError();
+  return launch_overlapped(k_element_staged, grid, block, smem, stream, a.overlap != 0, b);
 }
 
 // Energies of the current state, FP64 whatever the element precision:

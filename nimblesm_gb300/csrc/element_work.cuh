@@ -78,11 +78,12 @@ __device__ __forceinline__ bool positive(double x) { return __double_as_longlong
 __device__ __forceinline__ bool positive(float x) { return x > 0.0f; }
 
 // Nodal values of the element: FP64 form from the FP64 field, FP32 form from
-// the FP32 copy (no FP64 conversions, which would run on the FP64 pipe).
+// the FP32 copy (no FP64 conversions, which would run on the FP64 pipe).  The
+// FP64 field through ordinary loads: an overlapped launch reads it.
 template <typename T>
 __device__ __forceinline__ T load_node(const double* f64, const float* f32, long i);
 template <>
-__device__ __forceinline__ double load_node<double>(const double* f64, const float*, long i) { return __ldg(&f64[i]); }
+__device__ __forceinline__ double load_node<double>(const double* f64, const float*, long i) { return f64[i]; }
 template <>
 __device__ __forceinline__ float load_node<float>(const double*, const float* f32, long i) { return __ldg(&f32[i]); }
 

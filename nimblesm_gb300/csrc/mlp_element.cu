@@ -221,11 +221,13 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
     return (c < nchunks && e < a.E) ? __ldg(&a.conn[p * ld_e + e]) : -1;
   };
   auto values_of = [&](int id, float4& v) {
-    v = id >= 0 ? make_float4(__ldg(&a.uf[id]), __ldg(&a.uf[ld_n + id]), __ldg(&a.uf[2 * ld_n + id]), 0.0f)
+    v = id >= 0 ? make_float4(a.uf[id], a.uf[ld_n + id], a.uf[2 * ld_n + id], 0.0f)
                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // idle rows: zero displacement
   };
   int    id_next = node_of(blockIdx.x);
   float4 nv;
+  wait_prerequisites();  // the node kernel that writes u
+  launch_dependents();
   values_of(id_next, nv);
   for (long chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
     const long e     = chunk * el::kElems + el;
@@ -511,8 +513,7 @@ cudaError_t launch_element_mlp(const ElementArgs& a, const MlpElementArgs& m, cu
   const long chunks = (a.E + el::kElems - 1) / el::kElems;
   const long cap    = (long)num_sms() * (g_blocks_per_sm > 0 ? g_blocks_per_sm : 1);
   const int  grid   = (int)(chunks < cap ? chunks : cap);
-  k_element_mlp<<<grid, 128, el::SMEM, stream>>>(a, m);
-  return cudaGetLastError();
+  return launch_overlapped(k_element_mlp, grid, 128, el::SMEM, stream, a.overlap != 0, a, m);
 }
 
 }  // namespace mlp

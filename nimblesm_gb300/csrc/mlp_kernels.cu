@@ -646,25 +646,6 @@ cudaError_t setup_kernels()
   return cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, inf::SMEM);
 }
 
-// `overlap`: the launch may begin before the previous kernel of the stream has
-// ended (it waits for it before it reads or writes what the two share).
-template <class... Params, class... Args>
-static cudaError_t launch_overlapped(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s, bool overlap,
-                                     Args... args)
-{
-  cudaLaunchAttribute attr;
-  attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg                          = {};
-  cfg.gridDim                                     = dim3((unsigned)grid);
-  cfg.blockDim                                    = dim3((unsigned)block);
-  cfg.dynamicSmemBytes                            = smem;
-  cfg.stream                                      = s;
-  cfg.attrs                                       = &attr;
-  cfg.numAttrs                                    = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
-
 cudaError_t launch_train(int tiles, const float* X, const float* Y, long n, long first, long stride_a, long offset_b,
                          const uint8_t* img, const float* P, const Scales& sc, float inv_batch, float* grad_partial,
                          float* loss_partial, int* status, bool after_adam, cudaStream_t s)

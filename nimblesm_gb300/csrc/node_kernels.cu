@@ -92,17 +92,20 @@ __device__ __noinline__ double eval_bc_expression(const BcExprTable& ex, int pro
 // v; prescribed displacement sets v = (d - u) / delta when delta > 0.  The
 // magnitude is the line's constant or its expression's value at the node's
 // reference coordinates and time_current (`ev`, evaluated beforehand).
-__device__ __forceinline__ void apply_bc(const NodeBC& bc, double delta, const double* ev, const double u[3],
-                                         double v[3])
+// Components c0 .. c0 + kComps - 1.
+template <int kComps>
+__device__ __forceinline__ void apply_bc(const NodeBC& bc, double delta, const double* ev, int c0, const double u[kComps],
+                                         double v[kComps])
 {
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
+  for (int i = 0; i < kComps; i++) {
+    const int k = c0 + i;
     if (bc.kind[k] == 0 || (bc.kind[k] == 2 && !(delta > 0.0))) continue;
     const double value = bc.expr[k] < 0 ? bc.value[k] : ev[k];
     if (bc.kind[k] == 1) {
-      v[k] = value;
+      v[i] = value;
     } else {
-      v[k] = __ddiv_rn(__dadd_rn(value, -u[k]), delta);
+      v[i] = __ddiv_rn(__dadd_rn(value, -u[i]), delta);
     }
   }
 }
@@ -121,39 +124,47 @@ __device__ __forceinline__ double axpy(double s, double x, double y)
   return kExact ? __dadd_rn(y, __dmul_rn(s, x)) : fma(s, x, y);
 }
 
-// The assembled element force of node n: element contributions in increasing
-// element order, from the corner-major planes fe[(3 c + i) ld_e + e] (a row
-// of consecutive nodes reads consecutive elements of one plane per slot).
-template <typename TF, bool kExact>
-__device__ __forceinline__ void gather_force(const NodeArgs& a, int n, double f[3])
+// The first incidences of node n (all of them at a hex mesh's interior node)
+// from the slot-major copy, -1 past its last, and whether it has more.
+constexpr int kFirst = 8;
+__device__ __forceinline__ bool load_incidences(const NodeArgs& a, int n, int ec[kFirst])
 {
-  const TF* fe    = reinterpret_cast<const TF*>(a.fe);
-  TF        fs[3] = {TF(0), TF(0), TF(0)};
-  // the first 8 incidences (all of them at a hex mesh's interior node) from
-  // the slot-major copy: every load issued before the first sum, the sums in
-  // the same order as the rest from the CSR below
-  constexpr int  kFirst = 8;
-  const bool     more   = (__ldg(&a.node_more[n >> 5]) >> (n & 31)) & 1u;
-  int            ec[kFirst];
 #pragma unroll
   for (int j = 0; j < kFirst; j++) ec[j] = __ldg(&a.node_slots[(long)j * a.ld_n + n]);
-  TF x[kFirst][3];
+  return (__ldg(&a.node_more[n >> 5]) >> (n & 31)) & 1u;
+}
+
+// The assembled element force of node n, components c0 ...: element
+// contributions in increasing element order, from the corner-major planes
+// fe[(3 c + i) ld_e + e] (a row of consecutive nodes reads consecutive
+// elements of one plane per slot).
+template <typename TF, bool kExact, int kComps>
+__device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int ec[kFirst], bool more, int c0,
+                                             double f[kComps])
+{
+  const TF* fe = reinterpret_cast<const TF*>(a.fe) + c0 * a.ld_e;
+  TF        fs[kComps];
+  // every load issued before the first sum, the sums in the same order as the
+  // rest from the CSR below
+  TF x[kFirst][kComps];
 #pragma unroll
   for (int j = 0; j < kFirst; j++)
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-      x[j][i] = ec[j] >= 0 ? __ldg(&fe[((ec[j] & 7) * 3 + i) * a.ld_e + (ec[j] >> 3)]) : TF(0);
+    for (int i = 0; i < kComps; i++)
+      x[j][i] = ec[j] >= 0 ? fe[((ec[j] & 7) * 3 + i) * a.ld_e + (ec[j] >> 3)] : TF(0);
+#pragma unroll
+  for (int i = 0; i < kComps; i++) fs[i] = TF(0);
   // the first sum is 0 + x: x itself but for -0.0 (+0.0), an integer select
   // rather than an FP64 add in the exact form
   if (ec[0] >= 0) {
 #pragma unroll
-    for (int i = 0; i < 3; i++) fs[i] = kExact ? TF(plus_zero(double(x[0][i]))) : fs[i] + x[0][i];
+    for (int i = 0; i < kComps; i++) fs[i] = kExact ? TF(plus_zero(double(x[0][i]))) : fs[i] + x[0][i];
   }
 #pragma unroll
   for (int j = 1; j < kFirst; j++)
     if (ec[j] >= 0) {
 #pragma unroll
-      for (int i = 0; i < 3; i++) fs[i] = kExact ? TF(__dadd_rn(double(fs[i]), double(x[j][i]))) : fs[i] + x[j][i];
+      for (int i = 0; i < kComps; i++) fs[i] = kExact ? TF(__dadd_rn(double(fs[i]), double(x[j][i]))) : fs[i] + x[j][i];
     }
   const int k1 = more ? __ldg(&a.node_ptr[n + 1]) : 0;
   for (int k = more ? __ldg(&a.node_ptr[n]) + kFirst : 0; k < k1; k++) {
@@ -161,104 +172,151 @@ __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, double f[
     const long e  = ec >> 3;
     const int  c  = ec & 7;
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      const TF xi = __ldg(&fe[(c * 3 + i) * a.ld_e + e]);
+    for (int i = 0; i < kComps; i++) {
+      const TF xi = fe[(c * 3 + i) * a.ld_e + e];
       fs[i]       = kExact ? TF(__dadd_rn(double(fs[i]), double(xi))) : fs[i] + xi;
     }
   }
 #pragma unroll
-  for (int i = 0; i < 3; i++) f[i] = double(fs[i]);
+  for (int i = 0; i < kComps; i++) f[i] = double(fs[i]);
 }
 
-template <typename TF, bool kExact>
-__global__ void __launch_bounds__(256, sizeof(TF) == 4 ? 5 : 4) k_node_update(NodeArgs a)
+// kComps = 3: a thread per node.  kComps = 1: a thread per node and component
+// (blockIdx.y), with everything that the element kernel does not write read
+// ahead of the wait for it; for meshes that one wave of blocks covers, where a
+// step waits for latency: a third of the serial FP64 operations (64 clocks
+// each for a warp by itself), and the loads of state and schedule overlap the
+// element kernel's end.  (Three components that far ahead would spill.)
+template <typename TF, bool kExact, int kComps>
+__global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 4)) k_node_update(NodeArgs a)
 {
-  const int n = a.n_begin + blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr bool kAhead = kComps == 1;
+  const int      n      = a.n_begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.N) return;
+  const int  c0 = kComps == 1 ? blockIdx.y : 0;
   const long ld = a.ld_n;
-  double     u[3], v[3], acc[3];
+  double     u[kComps], v[kComps], acc[kComps];
   const int  slot  = a.bc_slot[n];
   const int  group = a.node_group ? __ldg(&a.node_group[n]) : 0;
   NodeBC     bc;
   if (slot >= 0) bc = a.bcs[slot];
+  const bool closes = a.closure && group >= a.closure_first;
+  int        ec[kFirst];
+  bool       more = false;
+  StepSched  post, pre;
+  double     im = 0.0;
+  auto       load_state = [&] {
+    if (a.k_post >= 0) {
+      post = a.sched[(long)(*a.step_base + a.k_post) * a.num_groups + group];
+      im   = a.inv_mass[n];
+    }
+#pragma unroll
+    for (int i = 0; i < kComps; i++) {
+      v[i] = a.v[(c0 + i) * ld + n];
+      u[i] = a.u[(c0 + i) * ld + n];
+    }
+  };
+  if ((a.k_post >= 0 || a.gather_only) && !closes) more = load_incidences(a, n, ec);
+  // (u and v are the previous node launch's, which had ended when the element
+  // kernel let this one start)
+  if (kAhead && !a.gather_only) {
+    load_state();
+    if (a.k_pre >= 0) pre = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
+  }
+  wait_prerequisites();
+  launch_dependents();
 
   if (a.k_post >= 0 || a.gather_only) {
     // ModelData::ComputeInternalForce: zero, then element contributions in
     // increasing element order (src/nimble_model_data.cc:620-667,
     // src/nimble_block.cc:373-383).
-    double f[3];
-    if (a.closure && group >= a.closure_first) {
+    double f[kComps];
+    if (closes) {
       // UqModel::ApplyClosure (src/uq/nimble_uq.cc:327-345): f = f_0 c_0, then
       // f += f_k c_k over the exact samples, from the same assembled forces
       // the nominal and exact samples' own nodes compute
       const int     local = n - a.node_off[group];
       const double* c     = a.closure + (long)(group - a.closure_first) * (a.num_exact + 1);
-      double        fk[3];
-      gather_force<TF, kExact>(a, a.node_off[0] + local, fk);
+      double        fk[kComps];
+      more = load_incidences(a, a.node_off[0] + local, ec);
+      gather_force<TF, kExact, kComps>(a, a.node_off[0] + local, ec, more, c0, fk);
 #pragma unroll
-      for (int i = 0; i < 3; i++) f[i] = kExact ? __dmul_rn(fk[i], c[0]) : fk[i] * c[0];
+      for (int i = 0; i < kComps; i++) f[i] = kExact ? __dmul_rn(fk[i], c[0]) : fk[i] * c[0];
       for (int k = 1; k <= a.num_exact; k++) {
-        gather_force<TF, kExact>(a, a.node_off[k] + local, fk);
+        more = load_incidences(a, a.node_off[k] + local, ec);
+        gather_force<TF, kExact, kComps>(a, a.node_off[k] + local, ec, more, c0, fk);
 #pragma unroll
-        for (int i = 0; i < 3; i++) f[i] = kExact ? __dadd_rn(f[i], __dmul_rn(fk[i], c[k])) : fma(fk[i], c[k], f[i]);
+        for (int i = 0; i < kComps; i++)
+          f[i] = kExact ? __dadd_rn(f[i], __dmul_rn(fk[i], c[k])) : fma(fk[i], c[k], f[i]);
       }
     } else {
-      gather_force<TF, kExact>(a, n, f);
+      gather_force<TF, kExact, kComps>(a, n, ec, more, c0, f);
     }
     // f_int (and a, below) are read by nothing inside a launch sequence: the
     // sequence's last launch (k_pre < 0) leaves them for the host's queries
     if (a.gather_only || a.k_pre < 0) {
 #pragma unroll
-      for (int i = 0; i < 3; i++) a.f_int[i * ld + n] = f[i];
+      for (int i = 0; i < kComps; i++) a.f_int[(c0 + i) * ld + n] = f[i];
     }
     if (a.gather_only) return;
-    const StepSched s  = a.sched[(long)(*a.step_base + a.k_post) * a.num_groups + group];
-    const double    im = a.inv_mass[n];
+    if (!kAhead) load_state();
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
+    for (int i = 0; i < kComps; i++) {
       // a = (1/m) (f_int + f_ext), f_ext = 0 (src/integrators/explicit_time_integrator.cc:250-257)
       acc[i] = kExact ? __dmul_rn(im, plus_zero(f[i])) : im * f[i];
-      v[i]   = axpy<kExact>(s.half, acc[i], a.v[i * ld + n]);
-      u[i]   = a.u[i * ld + n];
+      v[i]   = axpy<kExact>(post.half, acc[i], v[i]);
     }
-    if (s.is_output && slot >= 0) apply_bc(bc, s.delta, a.bc_expr_post ? a.bc_expr_post + (long)slot * 3 : nullptr, u, v);
+    if (post.is_output && slot >= 0)
+      apply_bc<kComps>(bc, post.delta, a.bc_expr_post ? a.bc_expr_post + (long)slot * 3 : nullptr, c0, u, v);
   } else {
+    if (!kAhead) load_state();
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      acc[i] = a.a[i * ld + n];
-      v[i]   = a.v[i * ld + n];
-      u[i]   = a.u[i * ld + n];
-    }
+    for (int i = 0; i < kComps; i++) acc[i] = a.a[(c0 + i) * ld + n];
   }
   if (a.k_pre >= 0) {
     // v^{n+1/2} = v^n + dt/2 a^n; BCs; u^{n+1} = u^n + dt v^{n+1/2}; BCs
     // (src/integrators/explicit_time_integrator.cc:200-223)
-    const StepSched s = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
+    if (!kAhead) pre = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
 #pragma unroll
-    for (int i = 0; i < 3; i++) v[i] = axpy<kExact>(s.half, acc[i], v[i]);
+    for (int i = 0; i < kComps; i++) v[i] = axpy<kExact>(pre.half, acc[i], v[i]);
     const double* ev = a.bc_expr_pre ? a.bc_expr_pre + (long)slot * 3 : nullptr;
-    if (slot >= 0) apply_bc(bc, s.delta, ev, u, v);
+    if (slot >= 0) apply_bc<kComps>(bc, pre.delta, ev, c0, u, v);
 #pragma unroll
-    for (int i = 0; i < 3; i++) u[i] = axpy<kExact>(s.delta, v[i], u[i]);
-    if (slot >= 0) apply_bc(bc, s.delta, ev, u, v);
+    for (int i = 0; i < kComps; i++) u[i] = axpy<kExact>(pre.delta, v[i], u[i]);
+    if (slot >= 0) apply_bc<kComps>(bc, pre.delta, ev, c0, u, v);
   }
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    a.u[i * ld + n] = u[i];
-    a.v[i * ld + n] = v[i];
-    if (a.k_post >= 0 && a.k_pre < 0) a.a[i * ld + n] = acc[i];
-    if (sizeof(TF) == 4 && a.uf != nullptr) a.uf[i * ld + n] = (float)u[i];  // FP32 forms only
+  for (int i = 0; i < kComps; i++) {
+    a.u[(c0 + i) * ld + n] = u[i];
+    a.v[(c0 + i) * ld + n] = v[i];
+    if (a.k_post >= 0 && a.k_pre < 0) a.a[(c0 + i) * ld + n] = acc[i];
+    if (sizeof(TF) == 4 && a.uf != nullptr) a.uf[(c0 + i) * ld + n] = (float)u[i];  // FP32 forms only
   }
+}
+
+template <typename TF, bool kExact>
+static cudaError_t launch_small(const NodeArgs& a, int count, cudaStream_t stream)
+{
+  // The element kernels take all of an SM's shared memory; with the same split
+  // of L1 here, an SM need not drain to change it between the two (a 4,096
+  // element step with overlapped launches: 16.5 us with differing splits).
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t err = once_per_device(configured, [] {
+    return cudaFuncSetAttribute(k_node_update<TF, kExact, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  });
+  if (err != cudaSuccess) return err;
+  const int block = count <= 64 * 152 ? 64 : 256;  // the smallest meshes over more SMs
+  return launch_overlapped(k_node_update<TF, kExact, 1>, dim3(grid_for(count, block), 3), block, 0, stream, a.overlap != 0, a);
 }
 
 cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream)
 {
-  if (a.N <= a.n_begin) return cudaSuccess;
-  if (a.fe_is_float)
-    k_node_update<float, false><<<grid_for(a.N - a.n_begin, 256), 256, 0, stream>>>(a);
-  else
-    k_node_update<double, true><<<grid_for(a.N - a.n_begin, 256), 256, 0, stream>>>(a);
-  return cudaGetLastError();
+  const int count = a.N - a.n_begin;
+  if (count <= 0) return cudaSuccess;
+  if (count <= kSmallNodes)
+    return a.fe_is_float ? launch_small<float, false>(a, count, stream) : launch_small<double, true>(a, count, stream);
+  return launch_overlapped(a.fe_is_float ? k_node_update<float, false, 3> : k_node_update<double, true, 3>,
+                           dim3(grid_for(count, 256)), 256, 0, stream, a.overlap != 0, a);
 }
 
 // One thread per (slot, component) and step (grid row): a program's latency on
@@ -309,7 +367,7 @@ __global__ void k_apply_bc(int N, long ld_n, const int* __restrict__ bc_slot, co
   double        ev[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) ev[k] = bc.expr[k] >= 0 ? eval_bc_expression(ex, bc.expr[k], n, time) : 0.0;
-  apply_bc(bc, delta, ev, uu, vv);
+  apply_bc<3>(bc, delta, ev, 0, uu, vv);
 #pragma unroll
   for (int i = 0; i < 3; i++) v[i * ld_n + n] = vv[i];
 }

@@ -8,6 +8,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <atomic>
 #include <stdint.h>
 
 namespace nsm {
@@ -92,7 +94,50 @@ struct ExprOp {
 constexpr int kExprStack = 16;  // operand stack of the evaluators; deeper programs are refused
 __host__ __device__ constexpr bool expr_is_unary(int code) { return code >= kExNeg && code <= kExNot; }
 
+// Runs `set` for the current device the first time (threads that race the
+// first repeat it, to the same effect).
+template <class F>
+inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, F set)
+{
+  int         dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  if ((err = set()) == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return err;
+}
+
 inline int grid_for(long n, int block) { return (int)((n + block - 1) / block); }
+
+// Programmatic dependent launch: a kernel launched by launch_overlapped may
+// start before the stream's previous kernel has ended.  It must call
+// wait_prerequisites() before it touches what that kernel writes (and read
+// that through ordinary loads, not the read-only path), and call
+// launch_dependents() only after that: its own successor may then rely on
+// everything before this kernel being complete.  What no kernel of a sequence
+// writes (geometry, connectivity, schedule, masses) may be read ahead of the
+// wait.
+#ifdef __CUDACC__
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... Params, class... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t s, bool overlap,
+                                     Args... args)
+{
+  cudaLaunchAttribute attr;
+  attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg                          = {};
+  cfg.gridDim                                     = grid;
+  cfg.blockDim                                    = dim3((unsigned)block);
+  cfg.dynamicSmemBytes                            = smem;
+  cfg.stream                                      = s;
+  cfg.attrs                                       = &attr;
+  cfg.numAttrs                                    = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+#endif
 
 // 4- and 8-byte asynchronous copies global -> shared (per-thread copy groups),
 // used to stage the next element's nodal values while the current one computes.

@@ -109,6 +109,7 @@ struct ElementArgs {
   const StepSched*  sched;      // schedule (nullable: outside the time loop)
   const int*        step_base;  // device step counter
   int               k;          // schedule offset of this step
+  int               overlap;    // the stream's previous kernel is the node kernel of the same sequence
   int*              status;
 };
 
@@ -172,6 +173,7 @@ struct NodeArgs {
   int               k_post;   // schedule offset of the step being finished, or -1
   int               k_pre;    // schedule offset of the step being started, or -1
   int               gather_only; // only f_int = gather(fe); no state update
+  int               overlap;    // the stream's previous kernel is the element kernel of the step being finished
   double*           u;
   double*           v;
   double*           a;
@@ -190,6 +192,11 @@ struct NodeArgs {
   const double*     bc_expr_pre;
 };
 
+// Nodes up to which a node launch gives a thread one component: the threads of
+// a wave (4 blocks of 256 on each of the chip's 152 SMs) over 3.  The launches
+// of a step overlap for such meshes (above, the kernels want different splits
+// of L1: the FP32 step of a mesh without locality went from 89 to 109 us).
+constexpr int kSmallNodes = 4 * 256 * 152 / 3;
 cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream);
 // The kinematic slots' expressions at their nodes (slot_node) and at the
 // schedule's times of `steps` steps from offset k: out [steps][num_slots][3].

@@ -122,12 +122,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v)
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// ---- programmatic dependent launch ----
-// The stream's next kernel, if launched so, may start; and wait for the end
-// (and the writes) of the previous one.
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count)
 {

@@ -91,3 +91,27 @@ def test_qoi_and_autotune():
     ref.begin(final, steps, 0)
     ref.advance(steps)
     assert np.array_equal(ref.state()["u"], st["u"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_sizes_on_both_sides_of_the_launch_rules(precision):
+    """Meshes that the node kernel takes a component per thread (50,653 nodes,
+    and 343 with overlapped element launches), and the ensemble of them, a node
+    per thread: bitwise the same state."""
+    probs = [cube_problem(36, jitter=0.2, seed=1), cube_problem(6, jitter=0.2, seed=2), cube_problem(10, jitter=0.2, seed=3)]
+    steps = 12
+    ens = E.Model(probs, precision=precision)
+    dt = 0.5 * ens.sample_time_steps()
+    ens.begin(steps * dt, steps, 5)
+    ens.advance(steps)
+    u, v, f = (ens.GetVectorNodeData(k) for k in ("displacement", "velocity", "internal_force"))
+    for g, p in enumerate(probs):
+        m = E.Model(p, precision=precision, graph_steps=5)
+        m.begin(steps * dt[g], steps, 5)
+        m.advance(steps)
+        s = ens.sample_slice(g)
+        assert np.array_equal(m.GetVectorNodeData("displacement"), u[s])
+        assert np.array_equal(m.GetVectorNodeData("velocity"), v[s])
+        assert np.array_equal(m.GetVectorNodeData("internal_force"), f[s])
+        m.close()
+    ens.close()
