@@ -98,6 +98,7 @@ def test_sizes_on_both_sides_of_the_launch_rules(precision):
     """Meshes that the node kernel takes a component per thread (50,653 nodes,
     and 343 with overlapped element launches), and the ensemble of them, a node
     per thread: bitwise the same state."""
+    from nimblesm_gb300.mesh import cube_problem
     probs = [cube_problem(36, jitter=0.2, seed=1), cube_problem(6, jitter=0.2, seed=2), cube_problem(10, jitter=0.2, seed=3)]
     steps = 12
     ens = E.Model(probs, precision=precision)
