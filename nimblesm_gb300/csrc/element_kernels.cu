@@ -33,10 +33,12 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_element(ElementArgs a)
 // nothing staged is held in registers.  Copy groups are per thread and each
 // thread reads only its own columns: no block barrier is needed.
 
-// Per thread and slot: kStageValues floats (values 0..23 u, 24..47 X), then
-// 8 connectivity entries; column stride B.  Two slots, for the element being
-// computed and the next one.
-constexpr int kStageWords = kStageValues + 8;
+// Per thread and slot: kStageValues 16-byte records (0..7 u, 8..15 X), then 8
+// connectivity entries; column stride B.  Two slots, for the element being
+// computed and the next one.  One record per node and field: in a mesh without
+// locality every gathered value is a 32-byte sector of its own, and three
+// 4-byte planes per field made that three times as many.
+constexpr int kStageBytes = kStageValues * 16 + 8 * 4;
 
 __device__ __forceinline__ void stage_conn(const ElementArgs& a, long e, int* col, int B)
 {
@@ -44,47 +46,50 @@ __device__ __forceinline__ void stage_conn(const ElementArgs& a, long e, int* co
   for (int n = 0; n < 8; n++) cp_async4(col + n * B, a.conn + n * a.ld_e + e);
 }
 
-__device__ __forceinline__ void stage_nodes(const ElementArgs& a, const int* conn_col, float* col, int B)
+__device__ __forceinline__ void stage_nodes(const ElementArgs& a, const int* conn_col, float4* col, int B)
 {
 #pragma unroll
   for (int n = 0; n < 8; n++) {
     const int id = conn_col[n * B];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      cp_async4(col + (n * 3 + k) * B, a.uf + k * a.ld_n + id);
-      cp_async4(col + (24 + n * 3 + k) * B, a.Xf + k * a.ld_n + id);
-    }
+    cp_async16(col + n * B, a.uf + id);
+    cp_async16(col + (8 + n) * B, a.Xf + id);
   }
 }
 
 __global__ void __launch_bounds__(128, 3) k_element_staged(ElementArgs a)
 {
-  extern __shared__ float stage_mem[];  // [2][kStageWords][blockDim.x]
+  extern __shared__ __align__(16) uint8_t stage_mem[];  // [2][16][blockDim.x] float4, then [2][8][blockDim.x] int
   const int  B      = blockDim.x;
   const long stride = (long)gridDim.x * B;
-  const int  slot   = kStageWords * B;
-  float*     cur    = stage_mem + threadIdx.x;  // slot of the element being computed
-  float*     nxt    = cur + slot;               // slot of the next one
+  float4*    cur    = reinterpret_cast<float4*>(stage_mem) + threadIdx.x;  // the element being computed
+  float4*    nxt    = cur + kStageValues * B;                              // the next one
+  int*       ccur   = reinterpret_cast<int*>(stage_mem + 2 * kStageValues * 16 * B) + threadIdx.x;
+  int*       cnxt   = ccur + 8 * B;
   long       e      = a.e_begin + blockIdx.x * (long)B + threadIdx.x;
   // prologue: connectivity of e (waited for), its nodal values and the
   // connectivity of e + stride in flight
-  if (e < a.E) stage_conn(a, e, reinterpret_cast<int*>(cur + kStageValues * B), B);
+  if (e < a.E) stage_conn(a, e, ccur, B);
   cp_async_commit();
   cp_async_wait_all();
   wait_prerequisites();  // the node kernel that writes u
   launch_dependents();
-  if (e < a.E) stage_nodes(a, reinterpret_cast<const int*>(cur + kStageValues * B), cur, B);
-  if (e + stride < a.E) stage_conn(a, e + stride, reinterpret_cast<int*>(nxt + kStageValues * B), B);
+  if (e < a.E) stage_nodes(a, ccur, cur, B);
+  if (e + stride < a.E) stage_conn(a, e + stride, cnxt, B);
   cp_async_commit();
   for (; e < a.E; e += stride) {
     cp_async_wait_all();  // this element's values and the next one's connectivity
-    if (e + stride < a.E) stage_nodes(a, reinterpret_cast<const int*>(nxt + kStageValues * B), nxt, B);
-    if (e + 2 * stride < a.E) stage_conn(a, e + 2 * stride, reinterpret_cast<int*>(cur + kStageValues * B), B);
+    if (e + stride < a.E) stage_nodes(a, cnxt, nxt, B);
+    if (e + 2 * stride < a.E) stage_conn(a, e + 2 * stride, ccur, B);
     cp_async_commit();
     element_work<float, false>(a, (int)e, StagedNodes{cur, B});
-    float* t = cur;
-    cur      = nxt;
-    nxt      = t;
+    // a whole warp's tile has been read before a lane's next copies arrive in it
+    if (a.store_ip != kStoreNever && e - (threadIdx.x & 31) + 32 <= a.E) __syncwarp();
+    float4* t = cur;
+    cur       = nxt;
+    nxt       = t;
+    int* c    = ccur;
+    ccur      = cnxt;
+    cnxt      = c;
   }
   cp_async_wait_all();
 }
@@ -159,10 +164,10 @@ cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cu
     }
     return cudaGetLastError();
   }
-  const size_t smem  = 2 * kStageWords * block * sizeof(float);
+  const size_t smem  = 2 * kStageBytes * block;
   static bool  configured = false;
-  if (!configured) {  // 56 KB at 128 threads: above the default 48 KB of dynamic shared memory
-    const int   most = 2 * kStageWords * 128 * (int)sizeof(float);
+  if (!configured) {  // 72 KB at 128 threads: above the default 48 KB of dynamic shared memory
+    const int   most = 2 * kStageBytes * 128;
     cudaError_t err  = cudaSuccess;
     err = cudaFuncSetAttribute(k_element_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (err == cudaSuccess)
@@ -320,16 +325,17 @@ cudaError_t launch_group_max_abs(int count, const int* nodes, const double* fiel
   return cudaGetLastError();
 }
 
-__global__ void k_to_float(long n, const double* __restrict__ src, float* __restrict__ dst)
+// FP64 planes to the FP32 form's records {x, y, z, 0} of the nodes.
+__global__ void k_to_records(int N, long ld_n, const double* __restrict__ src, float4* __restrict__ dst)
 {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)src[i];
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < N) dst[n] = make_float4((float)src[n], (float)src[ld_n + n], (float)src[2 * ld_n + n], 0.0f);
 }
 
-cudaError_t launch_to_float(long n, const double* src, float* dst, cudaStream_t stream)
+cudaError_t launch_to_records(int N, long ld_n, const double* src, float4* dst, cudaStream_t stream)
 {
-  if (n == 0) return cudaSuccess;
-  k_to_float<<<grid_for(n, 256), 256, 0, stream>>>(n, src, dst);
+  if (N == 0) return cudaSuccess;
+  k_to_records<<<grid_for(N, 256), 256, 0, stream>>>(N, ld_n, src, dst);
   return cudaGetLastError();
 }
 
@@ -341,13 +347,13 @@ __global__ void k_node_soa_to_aos(int N, long ld_n, const double* __restrict__ s
 }
 
 __global__ void k_node_aos_to_soa(int N, long ld_n, const double* __restrict__ src, double* __restrict__ dst,
-                                  float* __restrict__ dstf)
+                                  float4* __restrict__ dstf)
 {
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= 3L * N) return;
   const double x = src[i];
   dst[(i % 3) * ld_n + i / 3] = x;
-  if (dstf) dstf[(i % 3) * ld_n + i / 3] = (float)x;
+  if (dstf) reinterpret_cast<float*>(dstf + i / 3)[i % 3] = (float)x;
 }
 
 cudaError_t launch_node_soa_to_aos(int N, long ld_n, const double* src, double* dst, cudaStream_t stream)
@@ -357,7 +363,7 @@ cudaError_t launch_node_soa_to_aos(int N, long ld_n, const double* src, double* 
   return cudaGetLastError();
 }
 
-cudaError_t launch_node_aos_to_soa(int N, long ld_n, const double* src, double* dst, float* dstf,
+cudaError_t launch_node_aos_to_soa(int N, long ld_n, const double* src, double* dst, float4* dstf,
                                    cudaStream_t stream)
 {
   if (N == 0) return cudaSuccess;

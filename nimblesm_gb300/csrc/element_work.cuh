@@ -4,6 +4,8 @@
 // and the reasons for its form are in hex_math.cuh.
 #pragma once
 
+#include <type_traits>
+
 #include "hex_math.cuh"
 #include "nsm_kernels.cuh"
 
@@ -51,9 +53,16 @@ __device__ __forceinline__ uint4 pack16(const double* v, int c)
   return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
 }
 
+// A warp's tile: contiguous, or rows of 32 chunks `row` chunks apart.
+struct Tile {
+  uint4* p;
+  int    row;
+  __device__ __forceinline__ uint4& operator[](int i) const { return p[(i >> 5) * row + (i & 31)]; }
+};
+
 // dst: the first lane's block; all 32 lanes of the warp take part.
 template <int kChunks, typename T>
-__device__ __forceinline__ void warp_store(uint4* __restrict__ dst, const T* v, uint4* tile, int lane)
+__device__ __forceinline__ void warp_store(uint4* __restrict__ dst, const T* v, const Tile& tile, int lane)
 {
   __syncwarp();  // the tile's previous contents have been read
 #pragma unroll
@@ -77,18 +86,10 @@ __device__ __forceinline__ bool finite_bits(float x) { return isfinite(x); }
 __device__ __forceinline__ bool positive(double x) { return __double_as_longlong(x) > 0; }
 __device__ __forceinline__ bool positive(float x) { return x > 0.0f; }
 
-// Nodal values of the element: FP64 form from the FP64 field, FP32 form from
-// the FP32 copy (no FP64 conversions, which would run on the FP64 pipe).  The
-// FP64 field through ordinary loads: an overlapped launch reads it.
-template <typename T>
-__device__ __forceinline__ T load_node(const double* f64, const float* f32, long i);
-template <>
-__device__ __forceinline__ double load_node<double>(const double* f64, const float*, long i) { return f64[i]; }
-template <>
-__device__ __forceinline__ float load_node<float>(const double*, const float* f32, long i) { return __ldg(&f32[i]); }
-
-// Where an element's nodal values come from.  GlobalNodes: gathered from the
-// node planes through the connectivity.  StagedNodes: this thread's slots of a
+// Where an element's nodal values come from.  GlobalNodes: gathered through
+// the connectivity, from the FP64 field's planes or, in the FP32 form, from
+// the FP32 copies (no FP64 conversions, which would run on the FP64 pipe), one
+// 16-byte record per node and field.  StagedNodes: this thread's slots of a
 // shared-memory stage that cp.async filled one element ahead (FP32 form).
 template <typename T>
 struct GlobalNodes {
@@ -99,19 +100,42 @@ struct GlobalNodes {
 #pragma unroll
     for (int n = 0; n < 8; n++) id[n] = __ldg(&a.conn[n * a.ld_e + e]);
   }
-  __device__ __forceinline__ T u(int n, int k) const { return load_node<T>(a.u, a.uf, k * a.ld_n + id[n]); }
-  __device__ __forceinline__ T X(int n, int k) const { return __ldg(&a.Xf[k * a.ld_n + id[n]]); }
+  __device__ __forceinline__ void u(int n, T x[3]) const
+  {
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) x[k] = a.u[k * a.ld_n + id[n]];  // (an overlapped launch's: ordinary loads)
+    } else {
+      const float4 v = a.uf[id[n]];
+      x[0] = v.x, x[1] = v.y, x[2] = v.z;
+    }
+  }
+  __device__ __forceinline__ void X(int n, T x[3]) const
+  {
+    const float4 v = __ldg(&a.Xf[id[n]]);
+    x[0] = v.x, x[1] = v.y, x[2] = v.z;
+  }
+  __device__ __forceinline__ Tile tile(uint4* own) const { return Tile{own, 32}; }
 };
 
-// Stage layout: [48][blockDim] floats per element slot, values 0..23 u
-// (node-major, 3 components), 24..47 X; thread t owns column t, so the lanes of
-// a warp read consecutive words.
-constexpr int kStageValues = 48;
+// Stage layout: [16][blockDim] float4 per element slot, 0..7 the nodes' u,
+// 8..15 X; thread t owns column t, so the lanes of a warp read consecutive
+// chunks.  Once the values are read the first rows serve as the warp's tile.
+constexpr int kStageValues = 16;
 struct StagedNodes {
-  const float* s;  // this thread's column of the stage
-  int          B;  // column stride (threads per block)
-  __device__ __forceinline__ float u(int n, int k) const { return s[(n * 3 + k) * B]; }
-  __device__ __forceinline__ float X(int n, int k) const { return s[(24 + n * 3 + k) * B]; }
+  float4* s;  // this thread's column of the stage
+  int     B;  // column stride (threads per block)
+  __device__ __forceinline__ void u(int n, float x[3]) const
+  {
+    const float4 v = s[n * B];
+    x[0] = v.x, x[1] = v.y, x[2] = v.z;
+  }
+  __device__ __forceinline__ void X(int n, float x[3]) const
+  {
+    const float4 v = s[(8 + n) * B];
+    x[0] = v.x, x[1] = v.y, x[2] = v.z;
+  }
+  __device__ __forceinline__ Tile tile(uint4*) const { return Tile{reinterpret_cast<uint4*>(s - (threadIdx.x & 31)), B}; }
 };
 
 // FP64 form: reference geometry precomputed (geo planes).  FP32 form: the
@@ -130,18 +154,14 @@ __device__ __forceinline__ void element_work(const ElementArgs& a, const int e, 
   {
     T x[8][3];
 #pragma unroll
-    for (int n = 0; n < 8; n++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) x[n][k] = nodes.u(n, k);
+    for (int n = 0; n < 8; n++) nodes.u(n, x[n]);
     nodal_gradient<T>(x, Gu);
   }
   T GX[3][3][2][2];
   if constexpr (!kPrecomputedGeo) {
     T x[8][3];
 #pragma unroll
-    for (int n = 0; n < 8; n++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) x[n][k] = nodes.X(n, k);
+    for (int n = 0; n < 8; n++) nodes.X(n, x[n]);
     nodal_gradient<T>(x, GX);
   }
 
@@ -174,11 +194,12 @@ __device__ __forceinline__ void element_work(const ElementArgs& a, const int e, 
   // partial warp or a single lane by itself
   constexpr int kRecChunks = kIpRecord * (int)sizeof(T) / 16;
   constexpr int kTile      = tile_chunks<kRecChunks>();
-  __shared__ uint4 tiles[kWarp ? 4 : 1][kWarp ? kTile : 1];  // blocks of at most 128 threads
+  constexpr bool   kOwnTile = kWarp && !std::is_same<Nodes, StagedNodes>::value;
+  __shared__ uint4 tiles[kOwnTile ? 4 : 1][kOwnTile ? kTile : 1];  // blocks of at most 128 threads
   const int        lane   = threadIdx.x & 31;
   const long       e0     = (long)e - lane;  // the warp's elements are e0 .. e0 + 31
   const bool       whole  = kWarp && e0 + 32 <= a.E;
-  uint4*           tile   = tiles[kWarp ? (threadIdx.x >> 5) & 3 : 0];
+  const Tile       tile   = nodes.tile(tiles[kOwnTile ? (threadIdx.x >> 5) & 3 : 0]);
 
 #pragma unroll
   for (int p = 0; p < 8; p++) {

@@ -221,8 +221,7 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
     return (c < nchunks && e < a.E) ? __ldg(&a.conn[p * ld_e + e]) : -1;
   };
   auto values_of = [&](int id, float4& v) {
-    v = id >= 0 ? make_float4(a.uf[id], a.uf[ld_n + id], a.uf[2 * ld_n + id], 0.0f)
-                : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // idle rows: zero displacement
+    v = id >= 0 ? a.uf[id] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // idle rows: zero displacement
   };
   int    id_next = node_of(blockIdx.x);
   float4 nv;
@@ -454,8 +453,8 @@ __global__ void k_closure_geometry(ElementArgs a, float* __restrict__ geo)
 #pragma unroll
   for (int n = 0; n < 8; n++) {
     const int id = __ldg(&a.conn[n * a.ld_e + e]);
-#pragma unroll
-    for (int k = 0; k < 3; k++) x[n][k] = __ldg(&a.Xf[k * a.ld_n + id]);
+    const float4 v = __ldg(&a.Xf[id]);
+    x[n][0] = v.x, x[n][1] = v.y, x[n][2] = v.z;
   }
   float DX[3][3], G0[3][3], det0;
   point_gradient(x, w, DX);

@@ -290,7 +290,10 @@ __global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 
     a.u[(c0 + i) * ld + n] = u[i];
     a.v[(c0 + i) * ld + n] = v[i];
     if (a.k_post >= 0 && a.k_pre < 0) a.a[(c0 + i) * ld + n] = acc[i];
-    if (sizeof(TF) == 4 && a.uf != nullptr) a.uf[(c0 + i) * ld + n] = (float)u[i];  // FP32 forms only
+  }
+  if (sizeof(TF) == 4 && a.uf != nullptr) {  // FP32 forms only
+    if constexpr (kComps == 3) a.uf[n] = make_float4((float)u[0], (float)u[1], (float)u[2], 0.0f);
+    else reinterpret_cast<float*>(a.uf + n)[c0] = (float)u[0];
   }
 }
 

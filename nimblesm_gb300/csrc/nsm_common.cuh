@@ -139,7 +139,7 @@ inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, int b
 }
 #endif
 
-// 4- and 8-byte asynchronous copies global -> shared (per-thread copy groups),
+// 4-, 8- and 16-byte asynchronous copies global -> shared (per-thread copy groups),
 // used to stage the next element's nodal values while the current one computes.
 #ifdef __CUDACC__
 __device__ __forceinline__ void cp_async4(void* dst, const void* src)
@@ -151,6 +151,11 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src)
 {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src)
+{
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }

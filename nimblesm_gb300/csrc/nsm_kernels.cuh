@@ -90,8 +90,8 @@ struct ElementArgs {
   long          ld_e, ld_n;
   const int*    conn;      // [8][ld_e]
   const double* u;         // [3][ld_n] displacement (FP64 form)
-  const float*  uf;        // [3][ld_n] FP32 copy of u (FP32 form)
-  const float*  Xf;        // [3][ld_n] FP32 copy of X (FP32 form)
+  const float4* uf;        // [ld_n] FP32 copy of u, {x, y, z, 0} (FP32 form)
+  const float4* Xf;        // [ld_n] FP32 copy of X (FP32 form)
   const double* geo;       // [8 * kGeoPerPoint][ld_e] (FP64 form only)
   const long long* geo_fixed;      // fixed-point geometry (FP64 form only; element_fixed.cu)
   const struct FixedMaterial* fixed_mats;  // materials in fixed point
@@ -178,7 +178,7 @@ struct NodeArgs {
   double*           v;
   double*           a;
   double*           f_int;
-  float*            uf;       // FP32 copy of u kept in step (FP32 form), or null
+  float4*           uf;       // FP32 copy of u kept in step (FP32 form), or null
   // UQ closure (samples of one mesh): samples closure_first.. have no
   // elements; their force is c0 f_0 + sum_k c_k f_k over samples 0..num_exact
   // at the same local node (closure [sample - closure_first][num_exact + 1]).
@@ -234,10 +234,10 @@ cudaError_t launch_group_max_abs(int count, const int* nodes, const double* fiel
 // which: 0 = F ([E][8][9]), 1 = sigma ([E][8][6]).
 cudaError_t launch_ip_to_aos(int E, long ld_e, const void* ip, int src_is_float, int which, double* dst,
                              cudaStream_t stream);
-cudaError_t launch_to_float(long n, const double* src, float* dst, cudaStream_t stream);
+cudaError_t launch_to_records(int N, long ld_n, const double* src, float4* dst, cudaStream_t stream);
 cudaError_t launch_node_soa_to_aos(int N, long ld_n, const double* src, double* dst, cudaStream_t stream);
-// dstf (nullable): also an FP32 copy of the planes, same layout.
-cudaError_t launch_node_aos_to_soa(int N, long ld_n, const double* src, double* dst, float* dstf,
+// dstf (nullable): also the FP32 form's records of the nodes.
+cudaError_t launch_node_aos_to_soa(int N, long ld_n, const double* src, double* dst, float4* dstf,
                                    cudaStream_t stream);
 
 // Records the calling thread's nsm_last_error() text and returns `code`

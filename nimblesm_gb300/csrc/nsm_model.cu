@@ -81,8 +81,8 @@ struct nsm_model {
   unsigned char*      d_elem_left = nullptr;
   void*   d_ip = nullptr;   // [8][ld_e][16] per-point F and sigma records
   void*   d_fe = nullptr;   // [24][ld_e] element nodal forces, corner-major planes (3 c + i)
-  float*  d_Xf = nullptr;   // FP32 copies of X and u (FP32 form)
-  float*  d_uf = nullptr;
+  float4* d_Xf = nullptr;   // FP32 copies of X and u (FP32 form), {x, y, z, 0} per node
+  float4* d_uf = nullptr;
   int*    d_status = nullptr;
   int*    d_step_base = nullptr;
   double* d_scratch = nullptr;  // energy partials / setup temporaries
@@ -398,7 +398,7 @@ nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
 cudaError_t sync_uf(nsm_model* m)
 {
   if (!m->d_uf) return cudaSuccess;
-  return nsm::launch_to_float(3 * m->ld_n, m->d_u, m->d_uf, m->stream);
+  return nsm::launch_to_records(m->N, m->ld_n, m->d_u, m->d_uf, m->stream);
 }
 
 bool has_callbacks(const nsm_model* m)
@@ -665,9 +665,9 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
   NSM_CUDA_B(nsm::launch_ip_identity(E, m->ld_e, m->d_ip, m->precision == NSM_PRECISION_FP64 ? 0 : 1, m->stream));
   NSM_CUDA_B(cudaMemsetAsync(m->d_fe, 0, eb * 24 * m->ld_e, m->stream));
   if (m->precision == NSM_PRECISION_FP32_MIXED) {
-    NSM_CUDA_B(cudaMalloc(&m->d_Xf, sizeof(float) * 3 * m->ld_n));
-    NSM_CUDA_B(cudaMalloc(&m->d_uf, sizeof(float) * 3 * m->ld_n));
-    NSM_CUDA_B(cudaMemsetAsync(m->d_uf, 0, sizeof(float) * 3 * m->ld_n, m->stream));
+    NSM_CUDA_B(cudaMalloc(&m->d_Xf, sizeof(float4) * m->ld_n));
+    NSM_CUDA_B(cudaMalloc(&m->d_uf, sizeof(float4) * m->ld_n));
+    NSM_CUDA_B(cudaMemsetAsync(m->d_uf, 0, sizeof(float4) * m->ld_n, m->stream));
   }
   NSM_CUDA_B(cudaMalloc(&m->d_status, sizeof(int)));
   NSM_CUDA_B(cudaMemsetAsync(m->d_status, 0, sizeof(int), m->stream));
@@ -736,7 +736,7 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     NSM_CUDA_B(cudaMemcpyAsync(m->d_conn, conn_soa.data(), sizeof(int) * conn_soa.size(), cudaMemcpyHostToDevice,
                                m->stream));
     NSM_CUDA_B(cudaMemcpyAsync(m->d_X, X.data(), sizeof(double) * X.size(), cudaMemcpyHostToDevice, m->stream));
-    if (m->d_Xf) NSM_CUDA_B(nsm::launch_to_float(3 * m->ld_n, m->d_X, m->d_Xf, m->stream));
+    if (m->d_Xf) NSM_CUDA_B(nsm::launch_to_records(m->N, m->ld_n, m->d_X, m->d_Xf, m->stream));
     NSM_CUDA_B(cudaMemcpyAsync(m->d_node_ptr, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice,
                                m->stream));
     if (E > 0)
