@@ -292,12 +292,21 @@ __device__ __forceinline__ void element_work(const ElementArgs& a, const int e, 
       fv[n * 3 + i] = f[n][i];
       finite        = finite & finite_bits(f[n][i]);
     }
-  // corner-major planes fe[(3 c + i) ld_e + e]: each store instruction writes
-  // 32 consecutive elements of one plane, and the node kernel's gather of a
-  // row of nodes reads 32 consecutive elements of one plane
-  T* fe = reinterpret_cast<T*>(a.fe) + e;
+  bool planes = true;
+  if constexpr (sizeof(T) == 4) {
+    planes = a.fe_slot == nullptr;
+    if (!planes) {
 #pragma unroll
-  for (int q = 0; q < 24; q++) fe[(size_t)q * ld_e] = fv[q];
+      for (int n = 0; n < 8; n++)
+        reinterpret_cast<float4*>(a.fe)[__ldg(&a.fe_slot[n * ld_e + e])] =
+            make_float4(fv[3 * n], fv[3 * n + 1], fv[3 * n + 2], 0.0f);
+    }
+  }
+  if (planes) {
+    T* fe = reinterpret_cast<T*>(a.fe) + e;
+#pragma unroll
+    for (int q = 0; q < 24; q++) fe[(size_t)q * ld_e] = fv[q];
+  }
   if (bad || !finite) atomicOr(a.status, (bad ? NSM_STATUS_BAD_JACOBIAN : 0) | (finite ? 0 : NSM_STATUS_NONFINITE));
 }
 

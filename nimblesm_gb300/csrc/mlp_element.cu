@@ -420,10 +420,14 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
       for (int i = 0; i < 3; i++) g1[i] = fmaf(-mode_sign[ax], __shfl_xor_sync(0xffffffffu, g1[i], flip), g1[i]);
     }
     if (valid) {
-      float* fo = reinterpret_cast<float*>(a.fe) + (size_t)(3 * p) * ld_e + e;  // corner-major planes
-      fo[0]      = g1[0];
-      fo[ld_e]   = g1[1];
-      fo[2 * ld_e] = g1[2];
+      if (a.fe_slot) {
+        reinterpret_cast<float4*>(a.fe)[__ldg(&a.fe_slot[p * ld_e + e])] = make_float4(g1[0], g1[1], g1[2], 0.0f);
+      } else {
+        float* fo    = reinterpret_cast<float*>(a.fe) + (size_t)(3 * p) * ld_e + e;
+        fo[0]        = g1[0];
+        fo[ld_e]     = g1[1];
+        fo[2 * ld_e] = g1[2];
+      }
       if (!isfinite(g1[0]) || !isfinite(g1[1]) || !isfinite(g1[2])) status |= NSM_STATUS_NONFINITE;
     }
   }

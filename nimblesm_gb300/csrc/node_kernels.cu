@@ -124,34 +124,58 @@ __device__ __forceinline__ double axpy(double s, double x, double y)
   return kExact ? __dadd_rn(y, __dmul_rn(s, x)) : fma(s, x, y);
 }
 
-// The first incidences of node n (all of them at a hex mesh's interior node)
-// from the slot-major copy, -1 past its last, and whether it has more.
+// The first incidences of node n (all of them at a hex mesh's interior node),
+// -1 past its last, and whether it has more: 8 e + corner from the slot-major
+// copy, or (kRecords) the place of the force record.
 constexpr int kFirst = 8;
-__device__ __forceinline__ bool load_incidences(const NodeArgs& a, int n, int ec[kFirst])
+template <bool kRecords>
+__device__ __forceinline__ bool load_incidences(const NodeArgs& a, int n, int at[kFirst])
 {
+  if constexpr (kRecords) {
+    const int count = __ldg(&a.node_ptr[n + 1]) - __ldg(&a.node_ptr[n]);
 #pragma unroll
-  for (int j = 0; j < kFirst; j++) ec[j] = __ldg(&a.node_slots[(long)j * a.ld_n + n]);
-  return (__ldg(&a.node_more[n >> 5]) >> (n & 31)) & 1u;
+    for (int j = 0; j < kFirst; j++) at[j] = j < count ? j * (int)a.ld_n + n : -1;
+    return count > kFirst;
+  } else {
+#pragma unroll
+    for (int j = 0; j < kFirst; j++) at[j] = __ldg(&a.node_slots[(long)j * a.ld_n + n]);
+    return (__ldg(&a.node_more[n >> 5]) >> (n & 31)) & 1u;
+  }
+}
+
+// Components c0 ... of force record `at`.
+template <int kComps>
+__device__ __forceinline__ void load_record(const NodeArgs& a, int at, int c0, float x[kComps])
+{
+  const float4* row = reinterpret_cast<const float4*>(a.fe) + at;
+  if constexpr (kComps == 1) {
+    x[0] = reinterpret_cast<const float*>(row)[c0];
+  } else {
+    const float4 v = *row;
+    x[0] = v.x, x[1] = v.y, x[2] = v.z;
+  }
 }
 
 // The assembled element force of node n, components c0 ...: element
-// contributions in increasing element order, from the corner-major planes
-// fe[(3 c + i) ld_e + e] (a row of consecutive nodes reads consecutive
-// elements of one plane per slot).
-template <typename TF, bool kExact, int kComps>
+// contributions in increasing element order.
+template <typename TF, bool kExact, int kComps, bool kRecords>
 __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int ec[kFirst], bool more, int c0,
                                              double f[kComps])
 {
-  const TF* fe = reinterpret_cast<const TF*>(a.fe) + c0 * a.ld_e;
+  const TF* fe = reinterpret_cast<const TF*>(a.fe) + c0 * a.ld_e;  // planes
   TF        fs[kComps];
   // every load issued before the first sum, the sums in the same order as the
   // rest from the CSR below
   TF x[kFirst][kComps];
 #pragma unroll
   for (int j = 0; j < kFirst; j++)
+    if constexpr (kRecords) {
+      if (ec[j] >= 0) load_record<kComps>(a, ec[j], c0, x[j]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kComps; i++)
-      x[j][i] = ec[j] >= 0 ? fe[((ec[j] & 7) * 3 + i) * a.ld_e + (ec[j] >> 3)] : TF(0);
+      for (int i = 0; i < kComps; i++)
+        x[j][i] = ec[j] >= 0 ? fe[((ec[j] & 7) * 3 + i) * a.ld_e + (ec[j] >> 3)] : TF(0);
+    }
 #pragma unroll
   for (int i = 0; i < kComps; i++) fs[i] = TF(0);
   // the first sum is 0 + x: x itself but for -0.0 (+0.0), an integer select
@@ -171,9 +195,11 @@ __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int
     const int  ec = __ldg(&a.node_inc[k]);
     const long e  = ec >> 3;
     const int  c  = ec & 7;
+    TF         xk[kComps];
+    if constexpr (kRecords) load_record<kComps>(a, __ldg(&a.fe_slot[c * a.ld_e + e]), c0, xk);
 #pragma unroll
     for (int i = 0; i < kComps; i++) {
-      const TF xi = fe[(c * 3 + i) * a.ld_e + e];
+      const TF xi = kRecords ? xk[i] : fe[(c * 3 + i) * a.ld_e + e];
       fs[i]       = kExact ? TF(__dadd_rn(double(fs[i]), double(xi))) : fs[i] + xi;
     }
   }
@@ -187,8 +213,8 @@ __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int
 // step waits for latency: a third of the serial FP64 operations (64 clocks
 // each for a warp by itself), and the loads of state and schedule overlap the
 // element kernel's end.  (Three components that far ahead would spill.)
-template <typename TF, bool kExact, int kComps>
-__global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 4)) k_node_update(NodeArgs a)
+template <typename TF, bool kExact, int kComps, bool kRecords>
+__global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecords ? 5 : 4) k_node_update(NodeArgs a)
 {
   constexpr bool kAhead = kComps == 1;
   const int      n      = a.n_begin + blockIdx.x * blockDim.x + threadIdx.x;
@@ -216,7 +242,7 @@ __global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 
       u[i] = a.u[(c0 + i) * ld + n];
     }
   };
-  if ((a.k_post >= 0 || a.gather_only) && !closes) more = load_incidences(a, n, ec);
+  if ((a.k_post >= 0 || a.gather_only) && !closes) more = load_incidences<kRecords>(a, n, ec);
   // (u and v are the previous node launch's, which had ended when the element
   // kernel let this one start)
   if (kAhead && !a.gather_only) {
@@ -238,19 +264,19 @@ __global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 
       const int     local = n - a.node_off[group];
       const double* c     = a.closure + (long)(group - a.closure_first) * (a.num_exact + 1);
       double        fk[kComps];
-      more = load_incidences(a, a.node_off[0] + local, ec);
-      gather_force<TF, kExact, kComps>(a, a.node_off[0] + local, ec, more, c0, fk);
+      more = load_incidences<kRecords>(a, a.node_off[0] + local, ec);
+      gather_force<TF, kExact, kComps, kRecords>(a, a.node_off[0] + local, ec, more, c0, fk);
 #pragma unroll
       for (int i = 0; i < kComps; i++) f[i] = kExact ? __dmul_rn(fk[i], c[0]) : fk[i] * c[0];
       for (int k = 1; k <= a.num_exact; k++) {
-        more = load_incidences(a, a.node_off[k] + local, ec);
-        gather_force<TF, kExact, kComps>(a, a.node_off[k] + local, ec, more, c0, fk);
+        more = load_incidences<kRecords>(a, a.node_off[k] + local, ec);
+        gather_force<TF, kExact, kComps, kRecords>(a, a.node_off[k] + local, ec, more, c0, fk);
 #pragma unroll
         for (int i = 0; i < kComps; i++)
           f[i] = kExact ? __dadd_rn(f[i], __dmul_rn(fk[i], c[k])) : fma(fk[i], c[k], f[i]);
       }
     } else {
-      gather_force<TF, kExact, kComps>(a, n, ec, more, c0, f);
+      gather_force<TF, kExact, kComps, kRecords>(a, n, ec, more, c0, f);
     }
     // f_int (and a, below) are read by nothing inside a launch sequence: the
     // sequence's last launch (k_pre < 0) leaves them for the host's queries
@@ -297,7 +323,7 @@ __global__ void __launch_bounds__(256, kComps == 1 ? 4 : (sizeof(TF) == 4 ? 5 : 
   }
 }
 
-template <typename TF, bool kExact>
+template <typename TF, bool kExact, bool kRecords>
 static cudaError_t launch_small(const NodeArgs& a, int count, cudaStream_t stream)
 {
   // The element kernels take all of an SM's shared memory; with the same split
@@ -305,21 +331,28 @@ static cudaError_t launch_small(const NodeArgs& a, int count, cudaStream_t strea
   // element step with overlapped launches: 16.5 us with differing splits).
   static std::atomic<unsigned long long> configured{0};
   cudaError_t err = once_per_device(configured, [] {
-    return cudaFuncSetAttribute(k_node_update<TF, kExact, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return cudaFuncSetAttribute(k_node_update<TF, kExact, 1, kRecords>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
   if (err != cudaSuccess) return err;
   const int block = count <= 64 * 152 ? 64 : 256;  // the smallest meshes over more SMs
-  return launch_overlapped(k_node_update<TF, kExact, 1>, dim3(grid_for(count, block), 3), block, 0, stream, a.overlap != 0, a);
+  return launch_overlapped(k_node_update<TF, kExact, 1, kRecords>, dim3(grid_for(count, block), 3), block, 0, stream, a.overlap != 0, a);
+}
+
+template <typename TF, bool kExact, bool kRecords>
+static cudaError_t launch_nodes(const NodeArgs& a, cudaStream_t stream)
+{
+  const int count = a.N - a.n_begin;
+  if (count <= 0) return cudaSuccess;
+  if (count <= kSmallNodes) return launch_small<TF, kExact, kRecords>(a, count, stream);
+  return launch_overlapped(k_node_update<TF, kExact, 3, kRecords>, dim3(grid_for(count, 256)), 256, 0, stream,
+                           a.overlap != 0, a);
 }
 
 cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream)
 {
-  const int count = a.N - a.n_begin;
-  if (count <= 0) return cudaSuccess;
-  if (count <= kSmallNodes)
-    return a.fe_is_float ? launch_small<float, false>(a, count, stream) : launch_small<double, true>(a, count, stream);
-  return launch_overlapped(a.fe_is_float ? k_node_update<float, false, 3> : k_node_update<double, true, 3>,
-                           dim3(grid_for(count, 256)), 256, 0, stream, a.overlap != 0, a);
+  if (a.fe_is_float)
+    return a.fe_slot ? launch_nodes<float, false, true>(a, stream) : launch_nodes<float, false, false>(a, stream);
+  return launch_nodes<double, true, false>(a, stream);
 }
 
 // One thread per (slot, component) and step (grid row): a program's latency on

@@ -78,6 +78,16 @@ cudaError_t launch_derived_element(int E, long ld_e, const int* conn, const doub
 // stores; a warp writes 2 or 4 KB contiguous.
 constexpr int kIpRecord = 16;
 
+// Element nodal forces, in one of two layouts:
+//   planes [24][ld_e], plane 3 c + i component i of corner c: elements write
+//     them coalesced, and a warp's gather reads consecutive elements where
+//     consecutive nodes lie in consecutive elements;
+//   records (FP32 forms with fe_slot) {x, y, z, 0} where the node reads them:
+//     its j-th incidence at j ld_n + n, the ones past its eighth after all of
+//     those.  The node kernel reads them coalesced, and the element's write
+//     scatters one record per corner where the planes' gather would read three
+//     sectors per incidence.
+
 // When an element launch writes the records: on the schedule's output steps,
 // always, or never (a step inside a launch sequence, whose records the next
 // step overwrites before anything can read them).
@@ -104,7 +114,8 @@ struct ElementArgs {
   int           num_groups;      // samples (rows of the schedule)
   int           persistent;      // 0: one thread per element; 1: grid-stride over elements
   void*         ip;        // [8][ld_e][16] per-point records (T)
-  void*         fe;        // [ld_e][24] element nodal forces, corner-major (T)
+  void*         fe;        // element nodal forces (T)
+  const int*    fe_slot;   // [8][ld_e] record of each corner; null: planes (FP64 form: always)
   int               store_ip;   // kStore*
   const StepSched*  sched;      // schedule (nullable: outside the time loop)
   const int*        step_base;  // device step counter
@@ -162,6 +173,7 @@ struct NodeArgs {
   const int*        node_slots;
   const unsigned*   node_more;
   const void*       fe;       // element nodal forces (double or float)
+  const int*        fe_slot;  // as in ElementArgs
   int               fe_is_float;
   const double*     inv_mass;
   const int*        bc_slot;  // [N] -1 or index into bcs

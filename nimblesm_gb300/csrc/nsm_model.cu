@@ -80,7 +80,8 @@ struct nsm_model {
   nsm::FixedMaterial* d_fixed_mats = nullptr;
   unsigned char*      d_elem_left = nullptr;
   void*   d_ip = nullptr;   // [8][ld_e][16] per-point F and sigma records
-  void*   d_fe = nullptr;   // [24][ld_e] element nodal forces, corner-major planes (3 c + i)
+  void*   d_fe = nullptr;   // element nodal forces, planes or records
+  int*    d_fe_slot = nullptr;  // [8][ld_e] (records)
   float4* d_Xf = nullptr;   // FP32 copies of X and u (FP32 form), {x, y, z, 0} per node
   float4* d_uf = nullptr;
   int*    d_status = nullptr;
@@ -173,7 +174,7 @@ void free_all(nsm_model* m)
   m->graphs.clear();
   void* ptrs[] = {m->d_conn, m->d_node_ptr, m->d_node_inc, m->d_node_slots, m->d_node_more, m->d_X,     m->d_u,         m->d_v,     m->d_a,
                   m->d_f,    m->d_fext,     m->d_mass,     m->d_inv_mass, m->d_geo,    m->d_ip,    m->d_Xf,
-                  m->d_uf,   m->d_fe,   m->d_status,   m->d_step_base, m->d_scratch, m->d_stage,  m->d_out,   m->d_bc_slot,
+                  m->d_uf,   m->d_fe,   m->d_fe_slot,   m->d_status,   m->d_step_base, m->d_scratch, m->d_stage,  m->d_out,   m->d_bc_slot,
                   m->d_bcs,  m->d_ibc_slot, m->d_ibcs,     m->d_sched, m->d_group_out, m->d_elem_group,
                   m->d_node_group, m->d_elem_off, m->d_mats, m->d_fallbacks, m->d_node_off, m->d_closure,
                   m->d_stage_out, m->d_expr_code, m->d_expr_start, m->d_bc_slot_node, m->d_bc_expr_val,
@@ -325,6 +326,7 @@ nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
   a.model     = m->model;
   a.ip        = m->d_ip;
   a.fe        = m->d_fe;
+  a.fe_slot   = m->d_fe_slot;
   a.elem_group = m->d_elem_group;
   a.mats       = m->d_mats;
   a.num_groups = m->S;
@@ -367,6 +369,7 @@ nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
   a.node_slots  = m->d_node_slots;
   a.node_more   = m->d_node_more;
   a.fe          = m->d_fe;
+  a.fe_slot     = m->d_fe_slot;
   a.fe_is_float = m->precision == NSM_PRECISION_FP64 ? 0 : 1;
   a.inv_mass    = m->d_inv_mass;
   a.bc_slot     = m->d_bc_slot;
@@ -555,6 +558,47 @@ int         nsm_abi_version(void) { return NSM_ABI_VERSION; }
 
 namespace {
 
+// Whether the FP32 forms' element forces are kept as records where the nodes
+// read them rather than as planes over elements: the 32-byte sectors that warps
+// of the element and the node kernel touch either way, summed over about 100
+// evenly spaced groups of 32 consecutive nodes and of 32 consecutive elements.
+// Numbered along the axes a mesh keeps planes; with its nodes and elements
+// shuffled, 151,951 elements take 27 + 27 us a step (element + node launch) in
+// planes and 30 + 16 in records, 72^3 52 + 47 and 67 + 28.  The scattered half
+// sectors have to be joined in L2: 80^3 (68 MB of records) takes 125 us either
+// way and 100^3 285 in planes and 300 in records, so records past 48 MB are
+// left alone.  In FP64 (32-byte records) 151,951 elements take 135 us in planes
+// and 140 in records: planes always.
+constexpr long kMaxForceRecords = (48L << 20) / (long)sizeof(float4);
+bool force_records_pay(int N, int E, long ld_n, const std::vector<int>& slots, const int* conn)
+{
+  const int        step = std::max(1, std::max(N, E) / 32 / 100) * 32;
+  long             planes = 0, records = 0;
+  std::vector<int> s;
+  auto             distinct = [&] {
+    std::sort(s.begin(), s.end());
+    return (long)(std::unique(s.begin(), s.end()) - s.begin());
+  };
+  for (int n0 = 0; n0 + 32 <= N; n0 += step)
+    for (int j = 0; j < 8; j++) {
+      s.clear();
+      for (int n = n0; n < n0 + 32; n++) {
+        const int ec = slots[(size_t)j * ld_n + n];
+        if (ec >= 0) s.push_back(ec >> 6 << 3 | (ec & 7));  // 8 elements of plane 3 c (+ i)
+      }
+      records += (long)s.size() / 2;
+      planes += 3 * distinct();
+    }
+  for (int e0 = 0; e0 + 32 <= E; e0 += step)
+    for (int c = 0; c < 8; c++) {
+      s.clear();
+      for (int e = e0; e < e0 + 32; e++) s.push_back(conn[8 * (size_t)e + c] / 2);  // whichever slot
+      planes += 3 * 4;
+      records += 4 + distinct();  // the table, the records
+    }
+  return records < planes;
+}
+
 // One handle over S samples: the samples' meshes are concatenated (node and
 // element ids offset per sample) and each node carries its sample's time
 // schedule.  Materials: `num_mats` entries, element e uses
@@ -660,10 +704,8 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
   NSM_CUDA_B(cudaMalloc(&m->d_inv_mass, sizeof(double) * m->ld_n));
   NSM_CUDA_B(cudaMalloc(&m->d_geo, sizeof(double) * 8 * nsm::kGeoPerPoint * m->ld_e));
   NSM_CUDA_B(cudaMalloc(&m->d_ip, eb * nsm::kIpRecord * 8 * m->ld_e));
-  NSM_CUDA_B(cudaMalloc(&m->d_fe, eb * 24 * m->ld_e));
   NSM_CUDA_B(cudaMemsetAsync(m->d_ip, 0, eb * nsm::kIpRecord * 8 * m->ld_e, m->stream));
   NSM_CUDA_B(nsm::launch_ip_identity(E, m->ld_e, m->d_ip, m->precision == NSM_PRECISION_FP64 ? 0 : 1, m->stream));
-  NSM_CUDA_B(cudaMemsetAsync(m->d_fe, 0, eb * 24 * m->ld_e, m->stream));
   if (m->precision == NSM_PRECISION_FP32_MIXED) {
     NSM_CUDA_B(cudaMalloc(&m->d_Xf, sizeof(float4) * m->ld_n));
     NSM_CUDA_B(cudaMalloc(&m->d_uf, sizeof(float4) * m->ld_n));
@@ -727,6 +769,24 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
       for (int j = 0; j < 8 && ptr[n] + j < ptr[n + 1]; j++) slots[(size_t)j * m->ld_n + n] = inc[ptr[n] + j];
       if (ptr[n + 1] - ptr[n] > 8) more[n >> 5] |= 1u << (n & 31);
     }
+    size_t           fe_values = (size_t)24 * m->ld_e;
+    std::vector<int> at;
+    long             past = 8 * m->ld_n;  // records so far
+    for (int n = 0; n < N; n++) past += std::max(0, ptr[n + 1] - ptr[n] - 8);
+    if (m->precision == NSM_PRECISION_FP32_MIXED && past <= kMaxForceRecords &&
+        force_records_pay(N, E, m->ld_n, slots, gconn.data())) {
+      fe_values = (size_t)past * 4;
+      past      = 8 * m->ld_n;
+      at.assign((size_t)8 * m->ld_e, 0);
+      for (int n = 0; n < N; n++)
+        for (int k = ptr[n]; k < ptr[n + 1]; k++)
+          at[(size_t)(inc[k] & 7) * m->ld_e + (inc[k] >> 3)] =
+              (int)(k - ptr[n] < 8 ? (k - ptr[n]) * m->ld_n + n : past++);
+      NSM_CUDA_B(cudaMalloc(&m->d_fe_slot, sizeof(int) * at.size()));
+      NSM_CUDA_B(cudaMemcpyAsync(m->d_fe_slot, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, m->stream));
+    }
+    NSM_CUDA_B(cudaMalloc(&m->d_fe, eb * fe_values));
+    NSM_CUDA_B(cudaMemsetAsync(m->d_fe, 0, eb * fe_values, m->stream));
     if (m->ld_n > 0) {
       NSM_CUDA_B(cudaMemcpyAsync(m->d_node_slots, slots.data(), sizeof(int) * slots.size(), cudaMemcpyHostToDevice,
                                  m->stream));
