@@ -207,6 +207,91 @@ __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int
   for (int i = 0; i < kComps; i++) f[i] = double(fs[i]);
 }
 
+// UqModel::ApplyClosure (src/uq/nimble_uq.cc:327-345) for a node of an
+// approximate sample: f = f_0 c_0, then f += f_k c_k over the exact samples,
+// force(k) being sample k's at the same local node.
+template <bool kExact, typename Force>
+__device__ __forceinline__ double close_force(const NodeArgs& a, int group, Force force)
+{
+  const double* c  = a.closure + (long)(group - a.closure_first) * (a.num_exact + 1);
+  double        fk = force(0);
+  double        f  = kExact ? __dmul_rn(fk, c[0]) : fk * c[0];
+  for (int k = 1; k <= a.num_exact; k++) {
+    fk = force(k);
+    f  = kExact ? __dadd_rn(f, __dmul_rn(fk, c[k])) : fma(fk, c[k], f);
+  }
+  return f;
+}
+
+// What a node's update reads besides its force, components c0 ....
+template <int kComps>
+struct NodeState {
+  double    u[kComps], v[kComps];
+  double    im = 0.0;
+  StepSched post, pre;
+
+  __device__ __forceinline__ void load(const NodeArgs& a, int n, int c0, int group)
+  {
+    if (a.k_post >= 0) {
+      post = a.sched[(long)(*a.step_base + a.k_post) * a.num_groups + group];
+      im   = a.inv_mass[n];
+    }
+#pragma unroll
+    for (int i = 0; i < kComps; i++) {
+      v[i] = a.v[(c0 + i) * a.ld_n + n];
+      u[i] = a.u[(c0 + i) * a.ld_n + n];
+    }
+  }
+  __device__ __forceinline__ void load_pre(const NodeArgs& a, int group)
+  {
+    if (a.k_pre >= 0) pre = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
+  }
+};
+
+// The end of the step finished, from its assembled forces.
+template <bool kExact, int kComps>
+__device__ __forceinline__ void end_step(const NodeArgs& a, int n, int c0, int slot, const NodeBC& bc,
+                                         const double f[kComps], NodeState<kComps>& s, double acc[kComps])
+{
+#pragma unroll
+  for (int i = 0; i < kComps; i++) {
+    // a = (1/m) (f_int + f_ext), f_ext = 0 (src/integrators/explicit_time_integrator.cc:250-257)
+    acc[i] = kExact ? __dmul_rn(s.im, plus_zero(f[i])) : s.im * f[i];
+    s.v[i] = axpy<kExact>(s.post.half, acc[i], s.v[i]);
+  }
+  if (s.post.is_output && slot >= 0)
+    apply_bc<kComps>(bc, s.post.delta, a.bc_expr_post ? a.bc_expr_post + (long)slot * 3 : nullptr, c0, s.u, s.v);
+}
+
+// The beginning of the step started, and the stores of the state.
+template <typename TF, bool kExact, int kComps>
+__device__ __forceinline__ void begin_step(const NodeArgs& a, int n, int c0, int slot, const NodeBC& bc,
+                                           NodeState<kComps>& s, const double acc[kComps])
+{
+  const long ld = a.ld_n;
+  if (a.k_pre >= 0) {
+    // v^{n+1/2} = v^n + dt/2 a^n; BCs; u^{n+1} = u^n + dt v^{n+1/2}; BCs
+    // (src/integrators/explicit_time_integrator.cc:200-223)
+#pragma unroll
+    for (int i = 0; i < kComps; i++) s.v[i] = axpy<kExact>(s.pre.half, acc[i], s.v[i]);
+    const double* ev = a.bc_expr_pre ? a.bc_expr_pre + (long)slot * 3 : nullptr;
+    if (slot >= 0) apply_bc<kComps>(bc, s.pre.delta, ev, c0, s.u, s.v);
+#pragma unroll
+    for (int i = 0; i < kComps; i++) s.u[i] = axpy<kExact>(s.pre.delta, s.v[i], s.u[i]);
+    if (slot >= 0) apply_bc<kComps>(bc, s.pre.delta, ev, c0, s.u, s.v);
+  }
+#pragma unroll
+  for (int i = 0; i < kComps; i++) {
+    a.u[(c0 + i) * ld + n] = s.u[i];
+    a.v[(c0 + i) * ld + n] = s.v[i];
+    if (a.k_post >= 0 && a.k_pre < 0) a.a[(c0 + i) * ld + n] = acc[i];
+  }
+  if (sizeof(TF) == 4 && a.uf != nullptr) {  // FP32 forms only
+    if constexpr (kComps == 3) a.uf[n] = make_float4((float)s.u[0], (float)s.u[1], (float)s.u[2], 0.0f);
+    else reinterpret_cast<float*>(a.uf + n)[c0] = (float)s.u[0];
+  }
+}
+
 // kComps = 3: a thread per node.  kComps = 1: a thread per node and component
 // (blockIdx.y), with everything that the element kernel does not write read
 // ahead of the wait for it; for meshes that one wave of blocks covers, where a
@@ -219,35 +304,25 @@ __global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecor
   constexpr bool kAhead = kComps == 1;
   const int      n      = a.n_begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.N) return;
-  const int  c0 = kComps == 1 ? blockIdx.y : 0;
-  const long ld = a.ld_n;
-  double     u[kComps], v[kComps], acc[kComps];
+  const int  c0    = kComps == 1 ? blockIdx.y : 0;
+  const long ld    = a.ld_n;
   const int  slot  = a.bc_slot[n];
   const int  group = a.node_group ? __ldg(&a.node_group[n]) : 0;
   NodeBC     bc;
   if (slot >= 0) bc = a.bcs[slot];
-  const bool closes = a.closure && group >= a.closure_first;
-  int        ec[kFirst];
-  bool       more = false;
-  StepSched  post, pre;
-  double     im = 0.0;
-  auto       load_state = [&] {
-    if (a.k_post >= 0) {
-      post = a.sched[(long)(*a.step_base + a.k_post) * a.num_groups + group];
-      im   = a.inv_mass[n];
-    }
-#pragma unroll
-    for (int i = 0; i < kComps; i++) {
-      v[i] = a.v[(c0 + i) * ld + n];
-      u[i] = a.u[(c0 + i) * ld + n];
-    }
-  };
+  int               ec[kFirst];
+  bool              more = false;
+  double            acc[kComps];
+  NodeState<kComps> s;
+  // under the UQ closure a thread of a small mesh assembles the forces that it
+  // needs by itself
+  const bool closes = kComps == 1 && a.closure && group >= a.closure_first;
   if ((a.k_post >= 0 || a.gather_only) && !closes) more = load_incidences<kRecords>(a, n, ec);
   // (u and v are the previous node launch's, which had ended when the element
   // kernel let this one start)
   if (kAhead && !a.gather_only) {
-    load_state();
-    if (a.k_pre >= 0) pre = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
+    s.load(a, n, c0, group);
+    s.load_pre(a, group);
   }
   wait_prerequisites();
   launch_dependents();
@@ -258,23 +333,13 @@ __global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecor
     // src/nimble_block.cc:373-383).
     double f[kComps];
     if (closes) {
-      // UqModel::ApplyClosure (src/uq/nimble_uq.cc:327-345): f = f_0 c_0, then
-      // f += f_k c_k over the exact samples, from the same assembled forces
-      // the nominal and exact samples' own nodes compute
-      const int     local = n - a.node_off[group];
-      const double* c     = a.closure + (long)(group - a.closure_first) * (a.num_exact + 1);
-      double        fk[kComps];
-      more = load_incidences<kRecords>(a, a.node_off[0] + local, ec);
-      gather_force<TF, kExact, kComps, kRecords>(a, a.node_off[0] + local, ec, more, c0, fk);
-#pragma unroll
-      for (int i = 0; i < kComps; i++) f[i] = kExact ? __dmul_rn(fk[i], c[0]) : fk[i] * c[0];
-      for (int k = 1; k <= a.num_exact; k++) {
-        more = load_incidences<kRecords>(a, a.node_off[k] + local, ec);
-        gather_force<TF, kExact, kComps, kRecords>(a, a.node_off[k] + local, ec, more, c0, fk);
-#pragma unroll
-        for (int i = 0; i < kComps; i++)
-          f[i] = kExact ? __dadd_rn(f[i], __dmul_rn(fk[i], c[k])) : fma(fk[i], c[k], f[i]);
-      }
+      f[0] = close_force<kExact>(a, group, [&](int k) {
+        const int exact = a.node_off[k] + n - a.node_off[group];
+        double    fk[1];
+        more = load_incidences<kRecords>(a, exact, ec);
+        gather_force<TF, kExact, 1, kRecords>(a, exact, ec, more, c0, fk);
+        return fk[0];
+      });
     } else {
       gather_force<TF, kExact, kComps, kRecords>(a, n, ec, more, c0, f);
     }
@@ -285,41 +350,69 @@ __global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecor
       for (int i = 0; i < kComps; i++) a.f_int[(c0 + i) * ld + n] = f[i];
     }
     if (a.gather_only) return;
-    if (!kAhead) load_state();
-#pragma unroll
-    for (int i = 0; i < kComps; i++) {
-      // a = (1/m) (f_int + f_ext), f_ext = 0 (src/integrators/explicit_time_integrator.cc:250-257)
-      acc[i] = kExact ? __dmul_rn(im, plus_zero(f[i])) : im * f[i];
-      v[i]   = axpy<kExact>(post.half, acc[i], v[i]);
-    }
-    if (post.is_output && slot >= 0)
-      apply_bc<kComps>(bc, post.delta, a.bc_expr_post ? a.bc_expr_post + (long)slot * 3 : nullptr, c0, u, v);
+    if (!kAhead) s.load(a, n, c0, group);
+    end_step<kExact, kComps>(a, n, c0, slot, bc, f, s, acc);
   } else {
-    if (!kAhead) load_state();
+    if (!kAhead) s.load(a, n, c0, group);
 #pragma unroll
     for (int i = 0; i < kComps; i++) acc[i] = a.a[(c0 + i) * ld + n];
   }
-  if (a.k_pre >= 0) {
-    // v^{n+1/2} = v^n + dt/2 a^n; BCs; u^{n+1} = u^n + dt v^{n+1/2}; BCs
-    // (src/integrators/explicit_time_integrator.cc:200-223)
-    if (!kAhead) pre = a.sched[(long)(*a.step_base + a.k_pre) * a.num_groups + group];
-#pragma unroll
-    for (int i = 0; i < kComps; i++) v[i] = axpy<kExact>(pre.half, acc[i], v[i]);
-    const double* ev = a.bc_expr_pre ? a.bc_expr_pre + (long)slot * 3 : nullptr;
-    if (slot >= 0) apply_bc<kComps>(bc, pre.delta, ev, c0, u, v);
-#pragma unroll
-    for (int i = 0; i < kComps; i++) u[i] = axpy<kExact>(pre.delta, v[i], u[i]);
-    if (slot >= 0) apply_bc<kComps>(bc, pre.delta, ev, c0, u, v);
+  if (!kAhead) s.load_pre(a, group);
+  begin_step<TF, kExact, kComps>(a, n, c0, slot, bc, s, acc);
+}
+
+// The samples of one mesh under the UQ closure, past small meshes: a block takes
+// 32 local nodes of all samples, a warp one sample and component of them at a
+// time.  First the nominal and exact samples' forces are assembled, into f_int
+// (read back through L1), then every node is updated.  Bound by the FP64 pipe,
+// 64 clocks per warp and instruction on a quarter of an SM; a thread per node
+// with each approximate node assembling the full samples' forces again is
+// three times as many of its instructions with two exact samples.  15,625
+// nodes of 11 samples (8 approximate): 41 -> 25 us, 35,937 of 12: 96 -> 48;
+// 15,625 of 5 (1 approximate): 24.5 -> 16.3.  At most 12 warps: 6 or 8 and 16
+// take 26 and 49 to 54 us for the first two.  Small meshes wait for latency
+// instead, and this order lengthens the chain of a step: 216 nodes of 8
+// samples 12.8 us a step against 11.3, 4,913 of 10 21.6 against 19.3.
+constexpr int kUqWarps = 12;
+template <typename TF, bool kExact, bool kRecords>
+__global__ void __launch_bounds__(32 * kUqWarps, 3) k_node_update_uq(NodeArgs a)
+{
+  const int  local = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int  warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const bool in = local < a.local_nodes;
+  const long ld = a.ld_n;
+  wait_prerequisites();
+  launch_dependents();
+  for (int t = warp; t < 3 * (a.num_exact + 1) && in; t += warps) {
+    const int  n = __ldg(&a.node_off[t / 3]) + local;
+    int        ec[kFirst];
+    const bool more = load_incidences<kRecords>(a, n, ec);
+    double     f[1];
+    gather_force<TF, kExact, 1, kRecords>(a, n, ec, more, t % 3, f);
+    a.f_int[(t % 3) * ld + n] = f[0];
   }
-#pragma unroll
-  for (int i = 0; i < kComps; i++) {
-    a.u[(c0 + i) * ld + n] = u[i];
-    a.v[(c0 + i) * ld + n] = v[i];
-    if (a.k_post >= 0 && a.k_pre < 0) a.a[(c0 + i) * ld + n] = acc[i];
-  }
-  if (sizeof(TF) == 4 && a.uf != nullptr) {  // FP32 forms only
-    if constexpr (kComps == 3) a.uf[n] = make_float4((float)u[0], (float)u[1], (float)u[2], 0.0f);
-    else reinterpret_cast<float*>(a.uf + n)[c0] = (float)u[0];
+  __syncthreads();
+  for (int t = warp; t < 3 * a.num_groups && in; t += warps) {
+    const int    group = t / 3, c0 = t % 3;
+    const int    n    = __ldg(&a.node_off[group]) + local;
+    const int    slot = a.bc_slot[n];
+    NodeBC       bc;
+    NodeState<1> s;
+    if (slot >= 0) bc = a.bcs[slot];
+    if (!a.gather_only) {
+      s.load(a, n, c0, group);
+      s.load_pre(a, group);
+    }
+    double f[1], acc[1];
+    if (group < a.closure_first) {
+      f[0] = a.f_int[c0 * ld + n];
+    } else {
+      f[0] = close_force<kExact>(a, group, [&](int k) { return a.f_int[c0 * ld + __ldg(&a.node_off[k]) + local]; });
+      if (a.gather_only || a.k_pre < 0) a.f_int[c0 * ld + n] = f[0];
+    }
+    if (a.gather_only) continue;
+    end_step<kExact, 1>(a, n, c0, slot, bc, f, s, acc);
+    begin_step<TF, kExact, 1>(a, n, c0, slot, bc, s, acc);
   }
 }
 
@@ -343,6 +436,12 @@ static cudaError_t launch_nodes(const NodeArgs& a, cudaStream_t stream)
 {
   const int count = a.N - a.n_begin;
   if (count <= 0) return cudaSuccess;
+  if (a.closure && count > kSmallNodes && (a.k_post >= 0 || a.gather_only)) {
+    const int tasks = 3 * a.num_groups, rounds = (tasks + kUqWarps - 1) / kUqWarps;
+    const int warps = (tasks + rounds - 1) / rounds;
+    return launch_overlapped(k_node_update_uq<TF, kExact, kRecords>, dim3(grid_for(a.local_nodes, 32)), 32 * warps, 0, stream,
+                             a.overlap != 0, a);
+  }
   if (count <= kSmallNodes) return launch_small<TF, kExact, kRecords>(a, count, stream);
   return launch_overlapped(k_node_update<TF, kExact, 3, kRecords>, dim3(grid_for(count, 256)), 256, 0, stream,
                            a.overlap != 0, a);

@@ -196,6 +196,7 @@ struct NodeArgs {
   // at the same local node (closure [sample - closure_first][num_exact + 1]).
   const double*     closure;  // or null
   int               closure_first, num_exact;
+  int               local_nodes;  // of every sample
   const int*        node_off; // [num_groups + 1] first node of each sample
   // expression-driven boundary conditions: their values [num_bc_slots][3] at
   // the step finished and at the step started (rows of launch_bc_expr_values),

@@ -390,6 +390,7 @@ nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
   a.closure       = m->d_closure;
   a.closure_first = m->closure_first;
   a.num_exact     = m->num_exact;
+  a.local_nodes   = m->node_off[1];
   a.node_off      = m->d_node_off;
   a.bc_expr_post  = bc_expr_row(m, k_post);
   a.bc_expr_pre   = bc_expr_row(m, k_pre);

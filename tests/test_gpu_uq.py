@@ -121,3 +121,38 @@ def test_uq_fp32_mixed():
         out[prec] = m.trajectories("displacement")
         m.close()
     assert rel(out["fp32"], out["fp64"]) < 1e-3
+
+
+@pytest.mark.parametrize("n,exact,approx", [(17, 3, 8), (22, 1, 3)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_closure_of_meshes_past_the_small_ones(n, exact, approx, precision):
+    """More nodes than one wave takes (69,984 and 60,835), the last block of
+    32 nodes in part, 36 and 15 warps' work to a block.  An approximate sample
+    whose coefficients select one exact sample runs as that sample does, bit
+    for bit; the others' forces at the end are the linear combination of the
+    full samples' (bitwise in FP64, whose products and sums are rounded one by
+    one)."""
+    p = cube_problem(n, jitter=0.2, seed=3)
+    rng = np.random.default_rng(n)
+    coef = rng.uniform(-0.5, 0.8, size=(approx, exact + 1))
+    coef[:exact] = np.eye(exact + 1)[1:]
+    spec = UqSpec([(0, "bulk_modulus", 2.0e10)], rng.uniform(-1, 1, size=(exact, 1)), rng.uniform(-1, 1, size=(approx, 1)),
+                  coef)
+    m = E.UqModel(p, spec, precision=precision, graph_steps=4)
+    assert m.trajectories("displacement").shape[0] * p.num_nodes > 4 * 256 * 152 // 3
+    m.begin(9 * 0.4 * critical_time_step(p), 9, 0)
+    m.advance(9)
+    for field in ("displacement", "velocity", "internal_force"):
+        x = m.trajectories(field)
+        assert np.abs(x).max() > 0.0
+        assert np.array_equal(x[1 + exact : 1 + 2 * exact], x[1 : 1 + exact]), field
+    f = m.trajectories("internal_force")
+    for s in range(exact, approx):
+        want = f[0] * coef[s, 0]
+        for k in range(exact):
+            want = want + f[1 + k] * coef[s, 1 + k]
+        if precision == "fp64":
+            assert np.array_equal(f[1 + exact + s], want)
+        else:  # fused: each of the products' roundings left out
+            assert np.abs(f[1 + exact + s] - want).max() <= 4 * exact * 2.0 ** -53 * np.abs(f[: 1 + exact]).max()
+    m.close()
