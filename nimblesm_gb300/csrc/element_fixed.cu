@@ -4,10 +4,10 @@
 //
 // Bound: the integer pipes and issue.  On the FP64 pipe the same work is 170
 // FP64 instructions per point at 16 clocks each per SM: 5.08 ms for 128^3
-// elements, pipe 89% busy.  Here it is about 1,500 integer instructions per
-// point, 380 of them wide products (one per clock and SM), the others at two
-// to four per clock: 1.24 ms, 1.84 ms with F and sigma stored (issue 52%,
-// multiplier 64%); one launch on 4,096 elements 12 us against 60 us.
+// elements, pipe 89% busy.  Here it is about 1,190 integer instructions per
+// point, 360 of them wide products (one per clock and SM), the others at two
+// to four per clock: 1.09 ms (issue 46%, multiplier 73%), 1.63 ms with F and sigma
+// stored; one launch on 4,096 elements 11 us against 60 us.
 //
 // Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
 // j-th of 8 consecutive elements), two points each, in a loop that is not
