@@ -6,7 +6,7 @@
 // FP64 instructions per point at 16 clocks each per SM: 5.08 ms for 128^3
 // elements, pipe 89% busy.  Here it is about 1,190 integer instructions per
 // point, 360 of them wide products (one per clock and SM), the others at two
-// to four per clock: 1.09 ms (issue 46%, multiplier 73%), 1.63 ms with F and sigma
+// to four per clock: 1.09 ms (issue 46%, multiplier 73%), 1.52 ms with F and sigma
 // stored; one launch on 4,096 elements 11 us against 60 us.
 //
 // Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
@@ -105,6 +105,14 @@ __device__ __forceinline__ i64 other(i64 x)
   return __shfl_xor_sync(0xffffffffu, x, kXor);
 }
 constexpr int kAcrossEta = 8, kAcrossZeta = 16;  // lane masks
+
+// x 2^e, the scale added to the exponent (a product is one more instruction of
+// 64 clocks a warp on the FP64 pipe, as the conversion is).
+__device__ __forceinline__ double scaled(i64 x, int e)
+{
+  const double d = (double)x;
+  return x == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+}
 
 // The element as a whole on the FP64 pipe, by one lane.
 __device__ __noinline__ void fallback_fp64(const ElementArgs& a, int e)
@@ -327,14 +335,13 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
         }
         if (store) {
           double       r[kIpRecord];
-          const double ss = __longlong_as_double((i64)(1023 - 62 + mat.exponent - ee) << 52);
 #pragma unroll
           for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int k = 0; k < 3; k++)
-              r[full_slot(i, k)] = (double)(pt.H[i][k] + (i == k ? fx::kOne : 0)) * (1.0 / 1152921504606846976.0);
+              r[full_slot(i, k)] = scaled(pt.H[i][k] + (i == k ? fx::kOne : 0), -60);
 #pragma unroll
-          for (int q = 0; q < 6; q++) r[9 + q] = (double)pt.sig[q] * ss;
+          for (int q = 0; q < 6; q++) r[9 + q] = scaled(pt.sig[q], mat.exponent - ee - 62);
           r[15] = 0.0;
           store_records(a, eb, sx, r, reinterpret_cast<uint4*>(stage + kStageTile), lane);
         }

@@ -349,7 +349,13 @@ __global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecor
 #pragma unroll
       for (int i = 0; i < kComps; i++) a.f_int[(c0 + i) * ld + n] = f[i];
     }
-    if (a.gather_only) return;
+    if (a.gather_only) {
+      if (a.f_rows) {
+#pragma unroll
+        for (int i = 0; i < kComps; i++) a.f_rows[3L * n + c0 + i] = f[i];
+      }
+      return;
+    }
     if (!kAhead) s.load(a, n, c0, group);
     end_step<kExact, kComps>(a, n, c0, slot, bc, f, s, acc);
   } else {

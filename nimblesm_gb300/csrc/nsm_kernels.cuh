@@ -190,6 +190,7 @@ struct NodeArgs {
   double*           v;
   double*           a;
   double*           f_int;
+  double*           f_rows;   // gather_only: f_int [N][3] too, or null
   float4*           uf;       // FP32 copy of u kept in step (FP32 form), or null
   // UQ closure (samples of one mesh): samples closure_first.. have no
   // elements; their force is c0 f_0 + sum_k c_k f_k over samples 0..num_exact

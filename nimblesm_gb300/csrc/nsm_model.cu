@@ -85,6 +85,7 @@ struct nsm_model {
   float4* d_Xf = nullptr;   // FP32 copies of X and u (FP32 form), {x, y, z, 0} per node
   float4* d_uf = nullptr;
   int*    d_status = nullptr;
+  int*    h_status = nullptr;  // pinned: a copy to pageable memory waits for the stream by itself first
   int*    d_step_base = nullptr;
   double* d_scratch = nullptr;  // energy partials / setup temporaries
   double* d_stage = nullptr;    // [3N] AoS staging for host copies
@@ -154,8 +155,8 @@ struct nsm_model {
   int                      host_chunks = -1;  // requested (-1: by size)
   int                      hp_k = 0;          // chunks the cut tables were built for
   std::vector<int>         hp_e, hp_in, hp_ready;
-  cudaStream_t             hp_stream[4] = {};  // copy in, elements (2), copy out
-  std::vector<cudaEvent_t> hp_ev;              // [0]: start; then per chunk: in, elements, gathered
+  cudaStream_t             hp_stream[5] = {};  // copy in, elements (2), copy out, into planes
+  std::vector<cudaEvent_t> hp_ev;              // [0]: start; then per chunk: in, in planes, elements, gathered
   double*                  d_stage_out = nullptr;
 
   // profiling
@@ -195,14 +196,15 @@ void free_all(nsm_model* m)
     cudaEventDestroy(e.second);
   }
   if (m->stream) cudaStreamDestroy(m->stream);
+  cudaFreeHost(m->h_status);
 }
 
 int read_status(nsm_model* m)
 {
-  int status = 0;
-  NSM_CUDA(cudaMemcpyAsync(&status, m->d_status, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  NSM_CUDA(cudaMemcpyAsync(m->h_status, m->d_status, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   NSM_CUDA(cudaMemsetAsync(m->d_status, 0, sizeof(int), m->stream));
   NSM_CUDA(cudaStreamSynchronize(m->stream));
+  const int status = *m->h_status;
   if (status & NSM_STATUS_BAD_JACOBIAN) return fail(NSM_ERR_BAD_JACOBIAN, "non-positive Jacobian (inverted element)");
   if (status & NSM_STATUS_NONFINITE) return fail(NSM_ERR_NONFINITE, "non-finite element force");
   if (status & NSM_STATUS_TIMEOUT) return fail(NSM_ERR_STATE, "a bounded tensor-core wait ran out (learned closure)");
@@ -306,7 +308,7 @@ double* field_ptr(nsm_model* m, int field)
 // launched after this step that overwrites its records.
 nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
 {
-  nsm::ElementArgs a;
+  nsm::ElementArgs a{};
   a.E         = m->E;
   a.e_begin   = 0;
   a.ld_e      = m->ld_e;
@@ -359,7 +361,7 @@ const double* bc_expr_row(const nsm_model* m, int k)
 
 nsm::NodeArgs node_args(nsm_model* m, int k_post, int k_pre, int gather_only)
 {
-  nsm::NodeArgs a;
+  nsm::NodeArgs a{};
   a.N           = m->N;
   a.n_begin     = 0;
   a.ld_n        = m->ld_n;
@@ -713,6 +715,7 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     NSM_CUDA_B(cudaMemsetAsync(m->d_uf, 0, sizeof(float4) * m->ld_n, m->stream));
   }
   NSM_CUDA_B(cudaMalloc(&m->d_status, sizeof(int)));
+  NSM_CUDA_B(cudaMallocHost(&m->h_status, sizeof(int)));
   NSM_CUDA_B(cudaMemsetAsync(m->d_status, 0, sizeof(int), m->stream));
   NSM_CUDA_B(cudaMalloc(&m->d_step_base, sizeof(int)));
   NSM_CUDA_B(cudaMemsetAsync(m->d_step_base, 0, sizeof(int), m->stream));
@@ -1150,9 +1153,11 @@ namespace {
 int host_chunk_count(const nsm_model* m)
 {
   if (m->closure || m->d_closure || has_callbacks(m)) return 1;
-  // default: measured fastest at 128^3 (FP64 8 chunks, 5.64 ms; FP32 4 chunks,
-  // 0.63 ms, where each chunk's launches weigh more against 0.37 ms of device work)
-  const int k_default = m->precision == NSM_PRECISION_FP64 ? 8 : 4;
+  // Chunks by default, measured (us per call, pinned arrays): FP32 64^3 elements
+  // 155 whole, 145 in 6, 153 in 8; 90^3 344, 256, 263; 128^3 893, 560, 545.
+  // FP64 64^3 337 whole, 313 in 4, 311 in 8; 90^3 823, 709, 711; 128^3 2,251,
+  // 1,843, 1,791.  40^3: 71 whole, 80 in 2 (FP32), 116 and 131 (FP64).
+  const int k_default = m->precision == NSM_PRECISION_FP64 ? 8 : 6;
   int       k         = m->host_chunks > 0 ? m->host_chunks : (m->E >= (1 << 18) ? k_default : 1);
   if (k > m->E) k = m->E > 0 ? m->E : 1;
   return k;
@@ -1188,14 +1193,17 @@ cudaError_t build_host_pipe(nsm_model* m, int K)
     const int* r   = std::lower_bound(node_last.data(), node_last.data() + N, m->hp_e[j]);
     m->hp_ready[j] = j == K ? N : (int)(r - node_last.data());
   }
-  if ((int)m->hp_ev.size() < 1 + 3 * K) {
+  if ((int)m->hp_ev.size() < 1 + 4 * K) {
     for (cudaEvent_t e : m->hp_ev) cudaEventDestroy(e);
-    m->hp_ev.assign(1 + 3 * K, nullptr);
+    m->hp_ev.assign(1 + 4 * K, nullptr);
     for (auto& e : m->hp_ev)
       if ((err = cudaEventCreateWithFlags(&e, cudaEventDisableTiming)) != cudaSuccess) return err;
   }
+  int low = 0, high = 0;
+  if ((err = cudaDeviceGetStreamPriorityRange(&low, &high)) != cudaSuccess) return err;
   for (auto& s : m->hp_stream)
-    if (!s && (err = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)) != cudaSuccess) return err;
+    if (!s && (err = cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, &s == &m->hp_stream[4] ? high : low)) != cudaSuccess)
+      return err;
   if (!m->d_stage_out && (err = cudaMalloc(&m->d_stage_out, sizeof(double) * 3 * (size_t)N)) != cudaSuccess)
     return err;
   m->hp_k = K;
@@ -1207,58 +1215,83 @@ cudaError_t build_host_pipe(nsm_model* m, int K)
 // bitwise the same.
 cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double* f_host, int K)
 {
-  cudaStream_t s_in = m->hp_stream[0], s_out = m->hp_stream[3];
+  cudaStream_t s_in = m->hp_stream[0], s_out = m->hp_stream[3], s_planes = m->hp_stream[4];
   cudaStream_t s_el[2] = {m->hp_stream[1], m->hp_stream[2]};
-  cudaEvent_t* ev      = m->hp_ev.data();  // ev[0] start; ev[1 + 3j + {0, 1, 2}] in, elements, gathered
+  cudaEvent_t* ev      = m->hp_ev.data();  // ev[0] start; ev[1 + 4j + {0, ..., 3}] in, in planes, elements, gathered
   cudaError_t  err     = cudaEventRecord(ev[0], m->stream);  // earlier work on the state is done first
   if (err == cudaSuccess) err = cudaStreamWaitEvent(s_in, ev[0], 0);
-  for (int j = 0; j < K && err == cudaSuccess; j++) {
-    const int n0 = m->hp_in[j], n1 = m->hp_in[j + 1];
-    if (n1 > n0) {
-      err = cudaMemcpyAsync(m->d_stage + 3L * n0, u_host + 3L * n0, sizeof(double) * 3 * (size_t)(n1 - n0),
-                            cudaMemcpyHostToDevice, s_in);
-      if (err == cudaSuccess)
-        err = nsm::launch_node_aos_to_soa(n1 - n0, m->ld_n, m->d_stage + 3L * n0, m->d_u + n0,
-                                          m->d_uf ? m->d_uf + n0 : nullptr, s_in);
-    }
-    if (err == cudaSuccess) err = cudaEventRecord(ev[1 + 3 * j], s_in);
-  }
-  for (int j = 0; j < K && err == cudaSuccess; j++) {
+  auto copy_in = [&](int j) -> cudaError_t {
+    const int   n0 = m->hp_in[j], n1 = m->hp_in[j + 1];
+    cudaError_t e  = cudaSuccess;
+    if (n1 > n0)
+      e = cudaMemcpyAsync(m->d_stage + 3L * n0, u_host + 3L * n0, sizeof(double) * 3 * (size_t)(n1 - n0),
+                          cudaMemcpyHostToDevice, s_in);
+    if (e == cudaSuccess) e = cudaEventRecord(ev[1 + 4 * j], s_in);
+    // (on a stream of their own: the planes' kernel waits for registers while a
+    // chunk's elements hold all of them, and the copies need not)
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s_planes, ev[1 + 4 * j], 0);
+    if (e == cudaSuccess && n1 > n0)
+      e = nsm::launch_node_aos_to_soa(n1 - n0, m->ld_n, m->d_stage + 3L * n0, m->d_u + n0,
+                                      m->d_uf ? m->d_uf + n0 : nullptr, s_planes);
+    return e != cudaSuccess ? e : cudaEventRecord(ev[2 + 4 * j], s_planes);
+  };
+  auto elements = [&](int j) -> cudaError_t {
     cudaStream_t s = s_el[j & 1];
-    err            = cudaStreamWaitEvent(s, ev[1 + 3 * j], 0);
-    if (err == cudaSuccess) {
-      nsm::ElementArgs a = element_args(m, -1, true);
-      a.e_begin          = m->hp_e[j];
-      a.E                = m->hp_e[j + 1];
-      err = m->precision == NSM_PRECISION_FP64 ? nsm::launch_element_fp64(a, m->elaunch, s)
-                                               : nsm::launch_element_fp32(a, m->elaunch, s);
-    }
-    if (err == cudaSuccess) err = cudaEventRecord(ev[2 + 3 * j], s);
-  }
-  for (int j = 0; j < K && err == cudaSuccess; j++) {
+    cudaError_t  e = cudaStreamWaitEvent(s, ev[2 + 4 * j], 0);
+    if (e != cudaSuccess) return e;
+    nsm::ElementArgs a = element_args(m, -1, true);
+    a.e_begin          = m->hp_e[j];
+    a.E                = m->hp_e[j + 1];
+    e = m->precision == NSM_PRECISION_FP64 ? nsm::launch_element_fp64(a, m->elaunch, s)
+                                           : nsm::launch_element_fp32(a, m->elaunch, s);
+    return e != cudaSuccess ? e : cudaEventRecord(ev[3 + 4 * j], s);
+  };
+  auto nodes_out = [&](int j) -> cudaError_t {
     // chunks 0..j done: the last one on each element stream
-    err = cudaStreamWaitEvent(m->stream, ev[2 + 3 * j], 0);
-    if (err == cudaSuccess && j > 0) err = cudaStreamWaitEvent(m->stream, ev[2 + 3 * (j - 1)], 0);
+    cudaError_t e = cudaStreamWaitEvent(m->stream, ev[3 + 4 * j], 0);
+    if (e == cudaSuccess && j > 0) e = cudaStreamWaitEvent(m->stream, ev[3 + 4 * (j - 1)], 0);
     const int r0 = m->hp_ready[j], r1 = m->hp_ready[j + 1];
-    if (err == cudaSuccess && r1 > r0) {
-      nsm::NodeArgs a = node_args(m, -1, -1, 1);
-      a.n_begin       = r0;
-      a.N             = r1;
-      err             = nsm::launch_node_update(a, m->stream);
-      if (err == cudaSuccess)
-        err = nsm::launch_node_soa_to_aos(r1 - r0, m->ld_n, m->d_f + r0, m->d_stage_out + 3L * r0, m->stream);
-    }
-    if (err == cudaSuccess) err = cudaEventRecord(ev[3 + 3 * j], m->stream);
-    if (err == cudaSuccess) err = cudaStreamWaitEvent(s_out, ev[3 + 3 * j], 0);
-    if (err == cudaSuccess && r1 > r0)
-      err = cudaMemcpyAsync(f_host + 3L * r0, m->d_stage_out + 3L * r0, sizeof(double) * 3 * (size_t)(r1 - r0),
-                            cudaMemcpyDeviceToHost, s_out);
+    if (e != cudaSuccess || r1 <= r0) return e;
+    nsm::NodeArgs a = node_args(m, -1, -1, 1);
+    a.n_begin       = r0;
+    a.N             = r1;
+    a.f_rows        = m->d_stage_out;
+    e               = nsm::launch_node_update(a, m->stream);
+    if (e == cudaSuccess) e = cudaEventRecord(ev[4 + 4 * j], m->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s_out, ev[4 + 4 * j], 0);
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(f_host + 3L * r0, m->d_stage_out + 3L * r0,
+                                              sizeof(double) * 3 * (size_t)(r1 - r0), cudaMemcpyDeviceToHost, s_out);
+  };
+  // chunk by chunk, two copies in ahead of a chunk's kernels
+  for (int j = 0; j < 2 && j < K && err == cudaSuccess; j++) err = copy_in(j);
+  for (int j = 0; j < K && err == cudaSuccess; j++) {
+    if (j + 2 < K) err = copy_in(j + 2);
+    if (err == cudaSuccess) err = elements(j);
+    if (err == cudaSuccess) err = nodes_out(j);
   }
   if (err == cudaSuccess) err = cudaStreamSynchronize(s_out);
   return err;
 }
 
 }  // namespace
+
+// The device's address of `bytes` at p when all of them are pinned host memory
+// of one allocation (or registration) that the device can address, else null.
+static double* pinned_view(const double* p, size_t bytes)
+{
+  if ((reinterpret_cast<uintptr_t>(p) & (alignof(double) - 1)) != 0) return nullptr;
+  cudaPointerAttributes first{}, last{};
+  const char* const     end = reinterpret_cast<const char*>(p) + bytes - 1;
+  if (cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+      (const char*)last.devicePointer - (const char*)first.devicePointer != (ptrdiff_t)(bytes - 1))
+    return nullptr;
+  return reinterpret_cast<double*>(first.devicePointer);
+}
 
 int nsm_set_host_chunks(nsm_model* m, int chunks)
 {
@@ -1285,13 +1318,21 @@ int nsm_compute_internal_force_host(nsm_model* m, const double* displacement, do
     NSM_CUDA(internal_force_pipelined(m, displacement, internal_force, K));
     return read_status(m);  // synchronizes
   }
-  const size_t bytes = sizeof(double) * 3 * m->N;
-  NSM_CUDA(cudaMemcpyAsync(m->d_stage, displacement, bytes, cudaMemcpyHostToDevice, m->stream));
-  NSM_CUDA(nsm::launch_node_aos_to_soa(m->N, m->ld_n, m->d_stage, m->d_u, m->d_uf, m->stream));
+  // Pinned arrays are read and written by the kernels that change the layout
+  // (13,824 elements, FP32: 50 -> 46 us; 64,000: 71 -> 64); others go through the
+  // staging array.
+  const size_t  bytes = sizeof(double) * 3 * m->N;
+  const double* u_in  = pinned_view(displacement, bytes);
+  double*       f_out = pinned_view(internal_force, bytes);
+  if (!u_in) {
+    NSM_CUDA(cudaMemcpyAsync(m->d_stage, displacement, bytes, cudaMemcpyHostToDevice, m->stream));
+    u_in = m->d_stage;
+  }
+  NSM_CUDA(nsm::launch_node_aos_to_soa(m->N, m->ld_n, u_in, m->d_u, m->d_uf, m->stream));
   NSM_CUDA(launch_element(m, -1, true));
   NSM_CUDA(nsm::launch_node_update(node_args(m, -1, -1, 1), m->stream));
-  NSM_CUDA(nsm::launch_node_soa_to_aos(m->N, m->ld_n, m->d_f, m->d_stage, m->stream));
-  NSM_CUDA(cudaMemcpyAsync(internal_force, m->d_stage, bytes, cudaMemcpyDeviceToHost, m->stream));
+  NSM_CUDA(nsm::launch_node_soa_to_aos(m->N, m->ld_n, m->d_f, f_out ? f_out : m->d_stage, m->stream));
+  if (!f_out) NSM_CUDA(cudaMemcpyAsync(internal_force, m->d_stage, bytes, cudaMemcpyDeviceToHost, m->stream));
   return read_status(m);  // synchronizes
 }
 
