@@ -273,7 +273,7 @@ class Model:
 
     # ---- ModelDataBase mirror ----
     def ComputeLumpedMass(self) -> np.ndarray:
-        m = np.zeros(self.problem.num_nodes)
+        m = np.empty(self.problem.num_nodes)
         _check(library().nsm_compute_lumped_mass(self._h, _d(m)))
         return m
 
@@ -289,7 +289,7 @@ class Model:
         _check(library().nsm_apply_kinematic_conditions(self._h, time_current, time_previous))
 
     def GetVectorNodeData(self, label) -> np.ndarray:
-        out = np.zeros((self.problem.num_nodes, 3))
+        out = np.empty((self.problem.num_nodes, 3))
         _check(library().nsm_get_node_field(self._h, FIELDS[label], _d(out)))
         return out
 
@@ -329,7 +329,7 @@ class Model:
 
     def ComputeInternalForceHost(self, displacement, out=None) -> np.ndarray:
         u = np.ascontiguousarray(displacement, dtype=np.float64)
-        f = out if out is not None else np.zeros((self.problem.num_nodes, 3))
+        f = out if out is not None else np.empty((self.problem.num_nodes, 3))
         _check(library().nsm_compute_internal_force_host(self._h, _d(u), _d(f)))
         return f
 
@@ -352,7 +352,7 @@ class Model:
 
     def GetIntegrationPointData(self):
         E = self.problem.num_elem
-        F, s = np.zeros((E, 8, 9)), np.zeros((E, 8, 6))
+        F, s = np.empty((E, 8, 9)), np.empty((E, 8, 6))
         _check(library().nsm_get_ip_data(self._h, _d(F), _d(s)))
         return F, s
 
@@ -361,7 +361,7 @@ class Model:
         gradient [E][9] of the current configuration
         (Block::ComputeDerivedElementData)."""
         E = self.problem.num_elem
-        vol, s, F = np.zeros(E), np.zeros((E, 6)), np.zeros((E, 9))
+        vol, s, F = np.empty(E), np.empty((E, 6)), np.empty((E, 9))
         _check(library().nsm_compute_derived_element_data(self._h, _d(vol), _d(s), _d(F)))
         return vol, s, F
 
