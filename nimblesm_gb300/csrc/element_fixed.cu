@@ -10,7 +10,8 @@
 // stored; one launch on 4,096 elements 11 us against 60 us.
 //
 // Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
-// j-th of 8 consecutive elements), two points each, in a loop that is not
+// j-th of 8 consecutive elements; in small meshes eight, with a point each), two
+// points each, in a loop that is not
 // unrolled: the code of one point stays in the instruction cache (four points
 // unrolled, two lanes per element, ran at 25% issue with instruction fetch the
 // largest stall), and a small mesh waits for two points in a row, not eight.
@@ -104,7 +105,7 @@ __device__ __forceinline__ i64 other(i64 x)
 {
   return __shfl_xor_sync(0xffffffffu, x, kXor);
 }
-constexpr int kAcrossEta = 8, kAcrossZeta = 16;  // lane masks
+constexpr int kAcrossXi = 4, kAcrossEta = 8, kAcrossZeta = 16;  // lane masks (xi: one point per lane)
 
 // x 2^e, the scale added to the exponent (a product is one more instruction of
 // 64 clocks a warp on the FP64 pipe, as the conversion is).
@@ -159,12 +160,18 @@ __device__ __forceinline__ void load_g0(const i64* gp, Limbs g0[3][3])
 }
 
 // kStore: F and sigma are formed and stored when the launch asks for it.
-// kElastic: some material of the model is elastic.
-template <bool kStore, bool kHasElastic>
+// kHasElastic: some material of the model is elastic.
+// kPoints: points per lane.  1 (small meshes; without records): two lanes share
+// what a lane does otherwise, each with one of the two points; the transforms
+// before and after are done by both.
+template <bool kStore, bool kHasElastic, int kPoints>
 __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementArgs a)
 {
+  static_assert(kPoints == 2 || (kPoints == 1 && !kStore), "points per lane");
+  constexpr int  kElems = 4 * kPoints;  // of a warp, half a geometry block or a whole one
   extern __shared__ __align__(128) uint8_t stage_all[];
-  const int      lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 7, y = (lane >> 3) & 1, z = lane >> 4;
+  const int      lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & (kElems - 1), y = (lane >> 3) & 1, z = lane >> 4;
+  const int      side = kPoints == 1 ? (lane >> 2) & 1 : 0;  // of this lane's point along xi
   const long     ld_e = a.ld_e, ld_n = a.ld_n;
   uint8_t* const stage = stage_all + warp * (kStore ? kStageBytesStore : kStageBytes);
   double* const  us    = reinterpret_cast<double*>(stage + kStageU) + lane;  // [2][6][32]
@@ -175,13 +182,13 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
   const int* const conn = a.conn + (long)(corner_of(0, y, 0) + 4 * z) * ld_e;
   const long       next_corner = (corner_of(1, y, 0) - corner_of(0, y, 0)) * ld_e;
 
-  // groups of 8 elements; those at the ends of [e_begin, E) may be partial
-  const long g_end = (a.E + 7) >> 3, g_step = (long)gridDim.x * (blockDim.x >> 5);
-  long       g     = (a.e_begin >> 3) + (long)blockIdx.x * (blockDim.x >> 5) + warp;
+  // groups of kElems elements; those at the ends of [e_begin, E) may be partial
+  const long g_end = (a.E + kElems - 1) / kElems, g_step = (long)gridDim.x * (blockDim.x >> 5);
+  long       g     = a.e_begin / kElems + (long)blockIdx.x * (blockDim.x >> 5) + warp;
   const long first = g;
   if (g >= g_end) return;
   auto load_ids = [&](long gr, int id[2]) {
-    const long e = min(gr * 8 + j, (long)a.E - 1);  // (spare lanes repeat the last element)
+    const long e = min(gr * kElems + j, (long)a.E - 1);  // (spare lanes repeat the last element)
     id[0]        = __ldg(&conn[e]);
     id[1]        = __ldg(&conn[e + next_corner]);
   };
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       for (int i = 0; i < 3; i++) cp_async8(us + (buf * 6 + i * 2 + bx) * 32, a.u + i * ld_n + id[bx]);
   };
   auto stage_geo = [&](int buf, long gr) {
-    if (lane == 0) tc::bulk_load(stage + buf * kGeoBytes, a.geo_fixed + gr * kGeoBlock, kGeoBytes, &bar[buf]);
+    if (lane == 0) tc::bulk_load(stage + buf * kGeoBytes, a.geo_fixed + gr * kElems / 8 * kGeoBlock, kGeoBytes, &bar[buf]);
   };
   if (lane == 0) {
     tc::mbar_init(&bar[0], 1);
@@ -224,10 +231,11 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       cp_async_commit();
       if (g + 2 * g_step < g_end) load_ids(g + 2 * g_step, id);
     }
-    const long       eb    = g * 8;
+    const long       eb    = g * kElems;
     const int        e     = (int)min(eb + j, (long)a.E - 1);
     const bool       valid = eb + j >= a.e_begin && eb + j < a.E;
-    i64* const       gs    = reinterpret_cast<i64*>(stage + buf * kGeoBytes) + lane;
+    // the lane's column of the block
+    i64* const       gs    = reinterpret_cast<i64*>(stage + buf * kGeoBytes) + (kPoints == 2 ? lane : (lane & 24) + (eb & 4) + j);
 
     // ---- displacements of the lane's two corners, at 2^sc ----
     u64 u[3][2];
@@ -292,9 +300,10 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         fx::lane_gradient(v[i], G[i]);
-        // (the second point's increments wait where the displacements were)
-        us_i[(buf * 6 + i) * 32]     = G[i].y1;
-        us_i[(buf * 6 + 3 + i) * 32] = G[i].z1;
+        if (kPoints == 2) {  // the second point's increments wait where the displacements were
+          us_i[(buf * 6 + i) * 32]     = G[i].y1;
+          us_i[(buf * 6 + 3 + i) * 32] = G[i].z1;
+        }
       }
     }
 
@@ -305,9 +314,13 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     // in its own geometry rows.
     i64              Q[3][3];
     const fx::Moduli mod{mat.half_k, mat.shear, mat.lambda, mat.exponent, mat.model};
-    i64*             gp = gs;
+    i64*             gp = gs + side * kGeoPoint * 32;
+    if (side) {
+#pragma unroll
+      for (int i = 0; i < 3; i++) G[i].y += G[i].y1, G[i].z += G[i].z1;
+    }
 #pragma unroll 1
-    for (int sx = 0; sx < 2; sx++, gp += kGeoPoint * 32) {
+    for (int sx = 0; sx < kPoints; sx++, gp += kGeoPoint * 32) {
       i64 P[3][3];
       {
         Limbs g0[3][3];
@@ -350,7 +363,10 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       Limbs g0[3][3];
       load_g0(gp, g0);
       fx::point_force(g0, P, Q);
-      if (sx == 0) {
+      if (kPoints == 1) {
+#pragma unroll
+        for (int q = 0; q < 9; q++) gp[q * 32] = Q[q / 3][q % 3];
+      } else if (sx == 0) {
 #pragma unroll
         for (int q = 0; q < 9; q++) gp[q * 32] = Q[q / 3][q % 3];
 #pragma unroll
@@ -365,6 +381,11 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     const int    ef    = (int)ge + mat.exponent - ee - (elastic ? fx::kElasticForce : 0);
     const double scale = __longlong_as_double((i64)(1023 + ef) << 52);
     double       f[2][3];
+    if (kPoints == 1) {  // both lanes' forces
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 9; q++) Q[q / 3][q % 3] = gs[(kGeoPoint + q) * 32];
+    }
 #pragma unroll
     for (int i = 0; i < 3; i++) {
       const i64      qx = gs[i * 32], qy = gs[(3 + i) * 32], qz = gs[(6 + i) * 32];
@@ -378,57 +399,68 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       f[0][i] = (double)(od - ev) * scale;
       f[1][i] = (double)(-od - ev) * scale;
     }
+    if (kPoints == 1) bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossXi);
     bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossEta);
     bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossZeta);
     if (bad == 0 && valid) {
       double* const fe = reinterpret_cast<double*>(a.fe) + e;
 #pragma unroll
       for (int bx = 0; bx < 2; bx++)
+        if (kPoints == 2 || bx == side) {
 #pragma unroll
-        for (int i = 0; i < 3; i++) fe[(size_t)(3 * (corner_of(bx, y, 0) + 4 * z) + i) * ld_e] = f[bx][i];
+          for (int i = 0; i < 3; i++) fe[(size_t)(3 * (corner_of(bx, y, 0) + 4 * z) + i) * ld_e] = f[bx][i];
+        }
     }
     // which elements are left to the FP64 code
     any_bad |= bad;
-    if (y == 0 && z == 0 && valid) a.elem_left[e] = bad != 0;
+    if (y == 0 && z == 0 && side == 0 && valid) a.elem_left[e] = bad != 0;
     tc::fence_proxy_async();  // this lane's writes to the block come before the next copy into it
     __syncwarp();             // this group's staged data are read, its records written
   }
   // (after the loop: a call inside it would spill the loop's state)
-  if (__any_sync(0xffffffffu, any_bad != 0) && y == 0 && z == 0)
+  if (__any_sync(0xffffffffu, any_bad != 0) && y == 0 && z == 0 && side == 0)
     for (g = first; g < g_end; g += g_step) {
-      const long e = g * 8 + j;
+      const long e = g * kElems + j;
       if (e >= a.e_begin && e < a.E && a.elem_left[e]) fallback_fp64(a, (int)e);
     }
 }
 
 // Blocks of 128 threads, four warps, four blocks per SM (three where records
 // are stored): 16 warps of 128 registers and 14 KB of staging.
-template <bool kStore, bool kHasElastic>
+template <bool kStore, bool kHasElastic, int kPoints>
 static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
   constexpr int     bytes = kStore ? kStageBytesStore : kStageBytes;
   static std::atomic<unsigned long long> configured{0};
   cudaError_t err = once_per_device(configured, [] {
     cudaError_t e =
-        cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * bytes);
+        cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic, kPoints>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * bytes);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      e = cudaFuncSetAttribute(k_element_fixed<kStore, kHasElastic, kPoints>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return e;
   });
   if (err != cudaSuccess) return err;
   const int  warps  = l.block == 64 ? 2 : 4;
-  const long groups = ((a.E + 7L) >> 3) - (a.e_begin >> 3);
+  constexpr int kElems = 4 * kPoints;
+  const long groups = (a.E + kElems - 1L) / kElems - a.e_begin / kElems;
   const int  per_sm = l.persistent ? l.blocks_per_sm : (kStore ? 3 : 4) * (4 / warps);
   const long grid   = std::min<long>((groups + warps - 1) / warps, (long)per_sm * num_sms());
-  return launch_overlapped(k_element_fixed<kStore, kHasElastic>, (int)grid, 32 * warps, warps * bytes, stream, a.overlap != 0, a);
+  return launch_overlapped(k_element_fixed<kStore, kHasElastic, kPoints>, (int)grid, 32 * warps, warps * bytes, stream, a.overlap != 0, a);
 }
 
+// One point per lane as long as that gives none of the chip's schedulers (four
+// per SM) a second warp of 4 elements: a step of 100 elements 7.6 us with two
+// points per lane, 6.4 with one; 1,728 elements 8.8 and 7.7 (elastic blocks
+// beside neo-Hookean ones 11.6 and 10.6); 4,096 9.7 and 9.9 (13.0 and 12.6);
+// 8,000 12.0 and 13.2.
 cudaError_t launch_element_fp64(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
   if (a.E <= a.e_begin) return cudaSuccess;
-  if (a.store_ip == kStoreNever)
-    return a.has_elastic ? launch_fixed<false, true>(a, l, stream) : launch_fixed<false, false>(a, l, stream);
-  return a.has_elastic ? launch_fixed<true, true>(a, l, stream) : launch_fixed<true, false>(a, l, stream);
+  if (a.store_ip != kStoreNever)
+    return a.has_elastic ? launch_fixed<true, true, 2>(a, l, stream) : launch_fixed<true, false, 2>(a, l, stream);
+  if (a.E - a.e_begin <= 4 * 4 * num_sms())
+    return a.has_elastic ? launch_fixed<false, true, 1>(a, l, stream) : launch_fixed<false, false, 1>(a, l, stream);
+  return a.has_elastic ? launch_fixed<false, true, 2>(a, l, stream) : launch_fixed<false, false, 2>(a, l, stream);
 }
 
 }  // namespace nsm

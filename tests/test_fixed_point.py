@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from nimblesm_gb300 import engine as E
-from nimblesm_gb300.mesh import Problem, cube_mesh
+from nimblesm_gb300.mesh import Material, Problem, cube_mesh
 from oracle import oracle as O
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -106,3 +106,33 @@ def test_a_node_without_a_number_is_reported():
     with pytest.raises(E.EngineError):
         m.ComputeInternalForceHost(bad)
     assert np.array_equal(m.ComputeInternalForceHost(u), f)  # and the handle still works
+
+
+@pytest.mark.gpu
+# a lane's share of the element changes past one warp of 4 elements per
+# scheduler of the chip (2,432 elements)
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 2432, 2433])
+@pytest.mark.parametrize("elastic", [False, True])
+def test_one_point_per_lane_gives_the_bits_of_two(n, elastic):
+    """The first of two steps in one sequence stores no records and may take
+    the kernel of one point per lane; a step by itself stores them, with two.
+    Some elements strain beyond the fixed-point domain."""
+    p, rng = strip(n, 11 + n)
+    h = 1.0 / n
+    dt = 0.3 * h * np.sqrt(p.density / p.bulk_modulus)
+    p.v_init = rng.normal(0, 1e-3 * h / dt, p.coords.shape)
+    p.v_init[p.conn[::3].ravel()] += rng.uniform(-0.08, 0.08, (p.conn[::3].size, 3)) * h / dt
+    if elastic:
+        kind = [Material(m, p.density, p.bulk_modulus, p.shear_modulus) for m in ("elastic", "neohookean")]
+        p.blocks, p.elem_block = (kind, (np.arange(n) >= (n + 1) // 2).astype(np.int32)) if n > 1 else (kind[:1], np.zeros(1, np.int32))
+    states = []
+    for parts in ((2,), (1, 1)):
+        m = E.Model(p)
+        m.begin(2 * dt, 2, 0)
+        for k in parts:
+            m.advance(k)
+        states.append(m.state())
+        m.close()
+    assert np.abs(states[0]["f_int"]).max() > 0.0
+    for key in states[0]:
+        assert np.array_equal(states[0][key], states[1][key]), key
