@@ -8,6 +8,7 @@
 // multiply-adds -- on this chip FP64 operations, not bytes, bound a node
 // update, and the exact rounding of the reference buys nothing when the forces
 // themselves are FP32.
+#include "fixed_sum.cuh"
 #include "nsm_kernels.cuh"
 
 namespace nsm {
@@ -157,15 +158,17 @@ __device__ __forceinline__ void load_record(const NodeArgs& a, int at, int c0, f
 }
 
 // The assembled element force of node n, components c0 ...: element
-// contributions in increasing element order.
+// contributions in increasing element order, the first eight of the FP64 form
+// as one sum in fixed point (sum8; on the FP64 pipe their additions were half
+// of the launch's: 128^3 elements 183 -> 130 us, 15,625 nodes of 11 samples
+// 24.5 -> 22).
 template <typename TF, bool kExact, int kComps, bool kRecords>
 __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int ec[kFirst], bool more, int c0,
                                              double f[kComps])
 {
   const TF* fe = reinterpret_cast<const TF*>(a.fe) + c0 * a.ld_e;  // planes
   TF        fs[kComps];
-  // every load issued before the first sum, the sums in the same order as the
-  // rest from the CSR below
+  // every load issued before the first sum
   TF x[kFirst][kComps];
 #pragma unroll
   for (int j = 0; j < kFirst; j++)
@@ -176,20 +179,24 @@ __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int
       for (int i = 0; i < kComps; i++)
         x[j][i] = ec[j] >= 0 ? fe[((ec[j] & 7) * 3 + i) * a.ld_e + (ec[j] >> 3)] : TF(0);
     }
+  if constexpr (kExact) {
 #pragma unroll
-  for (int i = 0; i < kComps; i++) fs[i] = TF(0);
-  // the first sum is 0 + x: x itself but for -0.0 (+0.0), an integer select
-  // rather than an FP64 add in the exact form
-  if (ec[0] >= 0) {
+    for (int i = 0; i < kComps; i++) {
+      double y[kFirst];
 #pragma unroll
-    for (int i = 0; i < kComps; i++) fs[i] = kExact ? TF(plus_zero(double(x[0][i]))) : fs[i] + x[0][i];
-  }
-#pragma unroll
-  for (int j = 1; j < kFirst; j++)
-    if (ec[j] >= 0) {
-#pragma unroll
-      for (int i = 0; i < kComps; i++) fs[i] = kExact ? TF(__dadd_rn(double(fs[i]), double(x[j][i]))) : fs[i] + x[j][i];
+      for (int j = 0; j < kFirst; j++) y[j] = x[j][i];
+      fs[i] = fx::sum8(y);
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kComps; i++) fs[i] = TF(0);
+#pragma unroll
+    for (int j = 0; j < kFirst; j++)
+      if (ec[j] >= 0) {
+#pragma unroll
+        for (int i = 0; i < kComps; i++) fs[i] += x[j][i];
+      }
+  }
   const int k1 = more ? __ldg(&a.node_ptr[n + 1]) : 0;
   for (int k = more ? __ldg(&a.node_ptr[n]) + kFirst : 0; k < k1; k++) {
     const int  ec = __ldg(&a.node_inc[k]);
@@ -375,8 +382,9 @@ __global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecor
 // with each approximate node assembling the full samples' forces again is
 // three times as many of its instructions with two exact samples.  15,625
 // nodes of 11 samples (8 approximate): 41 -> 25 us, 35,937 of 12: 96 -> 48;
-// 15,625 of 5 (1 approximate): 24.5 -> 16.3.  At most 12 warps: 6 or 8 and 16
-// take 26 and 49 to 54 us for the first two.  Small meshes wait for latency
+// 15,625 of 5 (1 approximate): 24.5 -> 16.3 (with FP64 additions in the
+// assembly; 22, 43 and 14.5 without).  At most 12 warps: 6 or 8 and 16 took 26
+// and 49 to 54 us for the first two.  Small meshes wait for latency
 // instead, and this order lengthens the chain of a step: 216 nodes of 8
 // samples 12.8 us a step against 11.3, 4,913 of 10 21.6 against 19.3.
 constexpr int kUqWarps = 12;

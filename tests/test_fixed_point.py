@@ -43,6 +43,26 @@ def test_fixed_point_is_no_less_exact_than_fp64(tmp_path):
         assert float(s_fixed) <= max(float(s_fp64), ROUNDING), (model, rigid, strain)
 
 
+def test_sums_of_eight_are_no_less_exact_than_fp64(tmp_path):
+    """The node kernel's sum of up to eight element forces: over the largest of
+    them, within the rounding of the sum (2^-53 of at most 8 times it) and eight
+    numbers cut at 2^-59 of its power of two, and never further off than FP64
+    additions; infinities, NaN and zeros exactly as those."""
+    nvcc = shutil.which(os.environ.get("NVCC", "nvcc"))
+    if nvcc is None:
+        pytest.skip("nvcc not found")
+    exe = str(tmp_path / "fixed_sum_check")
+    subprocess.run([nvcc, "-O2", "-std=c++17", os.path.join(HERE, "fixed_sum_check.cc"), "-o", exe], check=True,
+                   capture_output=True)
+    r = subprocess.run([exe, "20000", "5"], capture_output=True, text=True, check=True)
+    rows = [line.split() for line in r.stdout.splitlines()]
+    assert len(rows) == 8
+    for kind, fixed, fp64 in rows:
+        assert float(fixed) <= float(fp64), kind
+        if kind not in ("tiny", "huge"):  # those are FP64 additions
+            assert float(fixed) <= 2.0 ** -53 * 8 + 8 * 2.0 ** -59, kind
+
+
 def strip(n, seed):
     """n jittered elements in a row along x."""
     coords, conn = cube_mesh(1)
