@@ -15,9 +15,14 @@
 //     p with the sum for node p (21 shuffles, no shared memory).
 // The CTAs are persistent: each loads the operand images once and walks
 // chunks of 16 elements.  The three layers use the same 64 tensor-memory
-// columns in turn, so up to 8 CTAs fit the 512 columns of an SM.  The biases
-// of layers 2 and 3 are written into the accumulator by one extra K = 16 MMA
-// before the layer's own (bias_mma), so no thread adds a bias.
+// columns in turn, so up to 8 CTAs fit the 512 columns of an SM, and 7 its
+// shared memory and registers.  The biases of layers 2 and 3 are written into
+// the accumulator by one extra K = 16 MMA before the layer's own (bias_mma), so
+// no thread adds a bias.
+// Bound: the chain gather, three MMA rounds with their epilogues, forces (1,150
+// instructions per point, 140 of them on the special-function unit: issue 52%),
+// so the more CTAs the better: 262,144 elements 117 us with 7 of 32.2 KB, 121
+// with 6 of 34.6 KB.
 // Points outside the training envelope take the plain neo-Hookean stress
 // (FP32) and are counted.
 #include <cuda_runtime.h>
@@ -37,11 +42,13 @@ namespace el {
 // 8 KB, and the per-warp node staging (4 elements x 8 nodes x 32 B) sits in
 // the warp's own X rows (bytes [2048 w, 2048 w + 1024)).
 constexpr int A    = 0;
-constexpr int W    = A + 128 * kHid * 2;  // W1x, W2, W3x images
-constexpr int ONE  = W + kOffW2t;         // [8][16] ones in columns 0-2, read by every 8-row group (SBO 0)
-constexpr int B2b  = ONE + 256;           // [64][16]: three-term BF16 split of b2 in columns 0-2
-constexpr int B3b  = B2b + 2048;          // [16][16]: of b3 (rows 0-5)
-constexpr int SMEM = B3b + 512;
+constexpr int ONE  = A + 128 * kHid * 2;  // [8][8] ones in columns 0-2, read by every 8-row group (SBO 0)
+constexpr int W    = ONE + 128;           // W1x, W2, W3x images
+constexpr int ZERO = W + kOffW3 + 16 * kHid;  // columns 8-15 beside ONE: rows 8-15 of W3x, which has six
+constexpr int B2b  = W + kOffW2t;         // [64][8]: three-term BF16 split of b2 in columns 0-2
+constexpr int B3b  = B2b + 1024;          // [16][8]: of b3 (rows 0-5)
+constexpr int BAR  = B3b + 256;           // the barrier, the tensor-memory address, the timeout record
+constexpr int SMEM = BAR + 64;
 constexpr int kStageWarp = 2048;          // bytes between the warps' staging areas
 constexpr uint32_t kCols = 64;
 constexpr int kElems = 16;                // elements per chunk
@@ -90,12 +97,15 @@ __device__ __forceinline__ float bias_term(float v, int t)
 }
 // D = ones * bias^T (one K = 16 step, overwriting D): every accumulator row
 // starts at the layer's FP32 bias, and the layer's MMAs accumulate onto it.
-// The A operand is one [8][16] core-matrix pair with ones in columns 0-2;
-// its stride between 8-row groups is 0, so all 128 rows read the same 256
-// bytes.  The B operand holds the bias's three-term split in columns 0-2.
-__device__ __forceinline__ void bias_mma(uint32_t d, const uint8_t* ones, const uint8_t* bias, int N)
+// The A operand is one core matrix with ones in columns 0-2 and a zero one
+// beside it; its stride between 8-row groups is 0, so all 128 rows read the
+// same 256 bytes.  The B operand holds the bias's three-term split in columns
+// 0-2, and (distance 0 along K) the same numbers again in columns 8-15, which
+// meet A's zeros.
+__device__ __forceinline__ void bias_mma(uint32_t d, const uint8_t* sm, const uint8_t* bias, int N)
 {
-  mma_bf16(d, smem_desc(smem_addr(ones), kLBO, 0), smem_desc(smem_addr(bias), kLBO, 256), idesc_bf16_f32(128, N), false);
+  mma_bf16(d, smem_desc(smem_addr(sm + el::ONE), el::ZERO - el::ONE, 0), smem_desc(smem_addr(bias), 0, 128),
+           idesc_bf16_f32(128, N), false);
 }
 // Hidden-layer epilogue: 64 accumulator columns of this thread's row, read as
 // two 32-column halves (two tensor-memory loads per wait) -> act(z) -> BF16
@@ -169,12 +179,12 @@ __device__ __forceinline__ int rec_slot(int row, int c)
   return ((row ^ ((row >> 3) & 1)) << 2) + (c ^ ((row >> 1) & 3));
 }
 
-__global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElementArgs m)
+__global__ void __launch_bounds__(128, 7) k_element_mlp(ElementArgs a, MlpElementArgs m)
 {
   extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ uint64_t mbar;
-  __shared__ uint32_t tslot;
-  __shared__ int      err;
+  uint64_t&           mbar  = *reinterpret_cast<uint64_t*>(sm + el::BAR);
+  uint32_t&           tslot = *reinterpret_cast<uint32_t*>(sm + el::BAR + 8);
+  int&                err   = *reinterpret_cast<int*>(sm + el::BAR + 12);
   const int           r = threadIdx.x, warp = r >> 5, lane = r & 31;
   const int           p = r & 7, el = r >> 3;
   const long          ld_e = a.ld_e, ld_n = a.ld_n;
@@ -191,11 +201,11 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
     // the layers' BF16 weight images
     const uint4* src = reinterpret_cast<const uint4*>(m.img);
     for (int i = r; i < kOffW2t / 16; i += 128) reinterpret_cast<uint4*>(sm + el::W)[i] = src[i];
-    for (int i = r; i < 64 * 16; i += 128) {
-      const int n = i / 16, k = i % 16;
-      store_bf16(sm + el::B2b, n, k, 16, k < 3 ? bias_term(m.P[ob2 + n], k) : 0.0f);
-      if (n < 16) store_bf16(sm + el::B3b, n, k, 16, (k < 3 && n < kOut) ? bias_term(m.P[ob3 + n], k) : 0.0f);
-      if (n < 8) store_bf16(sm + el::ONE, n, k, 16, k < 3 ? 1.0f : 0.0f);
+    for (int i = r; i < 64 * 8; i += 128) {
+      const int n = i / 8, k = i % 8;
+      store_bf16(sm + el::B2b, n, k, 8, k < 3 ? bias_term(m.P[ob2 + n], k) : 0.0f);
+      if (n < 16) store_bf16(sm + el::B3b, n, k, 8, (k < 3 && n < kOut) ? bias_term(m.P[ob3 + n], k) : 0.0f);
+      if (n < 8) store_bf16(sm + el::ONE, n, k, 8, k < 3 ? 1.0f : 0.0f);
     }
   }
   fence_before_sync();
@@ -287,7 +297,7 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
     // ---- layer 2 ----
     if (!publish(&err)) break;
     if (r == 0) {
-      bias_mma(tb, sm + el::ONE, sm + el::B2b, kHid);
+      bias_mma(tb, sm, sm + el::B2b, kHid);
       layer(tb, sm + el::A, kHid, sm + el::W + kOffW2, kHid, true);
       mma_commit(&mbar);
     }
@@ -297,7 +307,7 @@ __global__ void __launch_bounds__(128, 6) k_element_mlp(ElementArgs a, MlpElemen
     // ---- layer 3 ----
     if (!publish(&err)) break;
     if (r == 0) {
-      bias_mma(tb, sm + el::ONE, sm + el::B3b, kOutX);
+      bias_mma(tb, sm, sm + el::B3b, kOutX);
       layer(tb, sm + el::A, kHid, sm + el::W + kOffW3, kOutX, true);
       mma_commit(&mbar);
     }
