@@ -40,28 +40,28 @@ METRIC = "hex8 IP stress updates/sec, plain FP64 vs mixed/MLP at <=1e-3 rel. dis
 UNIT = "IP-updates/s"
 SCHEDULE_STEPS = 2000  # the workload's schedule: dt = 0.5 dt_crit, 2000 steps
 UQ_SCHEDULE_STEPS = 1000  # the ensemble's schedule: 1000 steps per sample
-# FP64 work per integration point of the FP64 element kernel's formulation:
-# 87.9 DFMA (2 flops each) + 44.5 DADD + 37.9 DMUL executed per point (counted
-# by ncu on the 64^3 case).  The FP64 pipe issues 2 of these instructions per
-# SM per cycle, whatever their kind.
+# Work per integration point of the FP64 form's element kernel.  It evaluates
+# the element in 64-bit fixed point on the integer pipes: 6 FP64 instructions
+# (the conversions of the forces) and 374 wide products, which an SM takes at
+# one per cycle (per warp).  The same formulation on the FP64 pipe executes
+# 170.2 instructions, 258.1 flops (87.9 DFMA, 44.5 DADD, 37.9 DMUL): what the
+# evaluation is worth in FP64.  (Counted by ncu on the 64^3 case.)
 FP64_FLOPS_PER_IP = 258.1
-FP64_INSTR_PER_IP = 170.2
-# DRAM bytes (read + write) of one element launch on the 128^3 cube, from one
-# ncu capture per form.
-ELEMENT_TRAFFIC_128 = {"fp64": 2.696480768e9 + 2.657063168e9, "fp32": 0.119112960e9 + 1.213583360e9}
+FP64_INSTR_PER_IP = 6.0
+WIDE_PRODUCTS_PER_IP = 374
+# DRAM bytes (read + write) of one element launch inside an advance (no point
+# records) on the 128^3 cube, from one ncu capture per form.
+ELEMENT_TRAFFIC_128 = {"fp64": 1.55e9 + 0.40124e9, "fp32": 0.13592e9 + 0.14358e9}
 
 
-def algorithmic_bytes(N, E, precision):
-    """Bytes each step moves once in the reference's field layout (the
-    ModelData contract after every step): nodes read X, u, v, a, m and write
-    u, v, a, f_int (200 B/node; this engine keeps a and f_int in registers
-    between the steps of one advance and writes them at its end);
-    elements read connectivity and write F and sigma per integration point
-    (992 B/element in FP64, 512 B in FP32).  The element kernel's share is
-    connectivity, F, sigma and the gathered X and u (48 B/node)."""
-    ip = 8 * (9 + 6) * (8 if precision == "fp64" else 4)
-    step = 200 * N + (32 + ip) * E
-    element = (32 + ip) * E + 48 * N
+def algorithmic_bytes(N, E):
+    """Bytes a step cannot do without: nodes read X, u, v and the mass and
+    write u and v (128 B/node), elements read their connectivity (32 B).  The
+    element kernel's share is connectivity and the gathered X and u (48
+    B/node).  Not counted: this engine's element forces, and F and sigma per
+    point, which are written on output steps and at the end of an advance."""
+    step = 128 * N + 32 * E
+    element = 32 * E + 48 * N
     return step, element
 
 
@@ -529,7 +529,7 @@ def run_ours(args):
                 "path": "nsm_host_loop_steps: the reference loop's host-side updates (one thread, pinned [N][3] "
                         "u, v, a, f_int) + nsm_compute_internal_force_host per step"}
 
-    step_bytes, elem_bytes = algorithmic_bytes(N, E_, args.precision)
+    step_bytes, elem_bytes = algorithmic_bytes(N, E_)
     peak, peak_kind = hbm_peak()
     elem_ms = head["prof"]["element_ms"] / max(head["prof"]["element_launches"], 1)
     node_ms = head["prof"]["node_ms"] / max(head["prof"]["node_launches"], 1)
@@ -549,7 +549,7 @@ def run_ours(args):
         "gpu_launches": head["launches"],
         "clocks": head["clocks"],
     }
-    hbm_roof = {"bound": "hbm", "kernel": "k_element<double>" if args.precision == "fp64" else "k_element_staged",
+    hbm_roof = {"bound": "hbm", "kernel": "k_element_fixed" if args.precision == "fp64" else "k_element_staged",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": peak_kind,
                 "traffic": ELEMENT_TRAFFIC_128.get(args.precision) if n == 128 else None,
@@ -558,26 +558,37 @@ def run_ours(args):
                 "algorithmic_bytes_per_launch": elem_bytes, "launch_ms": elem_ms, "node_launch_ms": node_ms,
                 "step_algorithmic_bytes": step_bytes}
     if args.precision == "fp64":
-        # The FP64 element kernel is bound by the FP64 pipe, not by HBM: its
-        # roofline is the pipe's rate, 2 FP64 instructions (a DFMA counting 2
-        # flops) per SM per cycle at the maximum SM clock.  MEASURED_PEAKS.json
-        # holds no FP64 figure, so the peak is that nominal rate.  The HBM
-        # fraction of the same launch is reported beside it (roofline_hbm).
+        # The FP64 pipe (2 FP64 instructions per SM per cycle, a DFMA counting 2
+        # flops) is the roof of an evaluation in FP64; the kernel evaluates in
+        # fixed point on the integer pipes, so its FP64-equivalent rate lies
+        # above that roof.  What bounds it is the integer multiplier
+        # (roofline_int).  MEASURED_PEAKS.json holds neither figure: both peaks
+        # are nominal, at the maximum SM clock.
         sms = E.device_sm_count(local)
         max_mhz = (head["clocks"] or {}).get("sm_max_mhz") or 2070.0
-        nominal = 2 * 2 * sms * max_mhz * 1e6 / 1e12
-        ach64 = FP64_FLOPS_PER_IP * 8 * E_ / (elem_ms * 1e-3) / 1e12
-        instr_rate = FP64_INSTR_PER_IP * 8 * E_ / (elem_ms * 1e-3)
+        ips = 8 * E_ / (elem_ms * 1e-3)
         pipe_rate = 2 * sms * max_mhz * 1e6
-        line["roofline"] = {"bound": "fp64", "kernel": "k_element<double>", "achieved": ach64, "peak": nominal,
+        nominal = 2 * pipe_rate / 1e12
+        ach64 = FP64_FLOPS_PER_IP * ips / 1e12
+        line["roofline"] = {"bound": "fp64", "kernel": "k_element_fixed", "achieved": ach64, "peak": nominal,
                             "unit": "TFLOP/s", "frac": ach64 / nominal,
                             "peak_source": f"nominal FP64 pipe: 2 DFMA per SM per cycle x {sms} SMs x {max_mhz:.0f} MHz",
+                            "note": "achieved is FP64-equivalent: the flops of the same formulation in FP64; the kernel "
+                                    "computes it in 64-bit fixed point on the integer pipes (roofline_int), so frac "
+                                    "may exceed 1",
                             "traffic": hbm_roof["traffic"], "traffic_source": hbm_roof["traffic_source"],
                             "launch_ms": elem_ms, "flops_per_ip": FP64_FLOPS_PER_IP,
                             "fp64_instructions_per_ip": FP64_INSTR_PER_IP,
-                            "pipe_instruction_frac": instr_rate / pipe_rate,
-                            "flops_source": "executed DFMA/DADD/DMUL per point, ncu (FMA = 2 flops)",
+                            "pipe_instruction_frac": FP64_INSTR_PER_IP * ips / pipe_rate,
+                            "flops_source": "DFMA/DADD/DMUL per point of the FP64 evaluation, ncu (FMA = 2 flops)",
                             "hbm_frac": hbm_roof["frac"]}
+        products = WIDE_PRODUCTS_PER_IP * ips
+        mult_rate = 32 * sms * max_mhz * 1e6
+        line["roofline_int"] = {"bound": "int_multiplier", "kernel": "k_element_fixed", "achieved": products / 1e12,
+                                "peak": mult_rate / 1e12, "unit": "T wide products/s", "frac": products / mult_rate,
+                                "peak_source": f"32 x 32 -> 64 bit products: one warp instruction per SM per cycle "
+                                               f"(measured) x {sms} SMs x {max_mhz:.0f} MHz",
+                                "launch_ms": elem_ms, "wide_products_per_ip": WIDE_PRODUCTS_PER_IP}
         line["roofline_hbm"] = hbm_roof
     else:
         line["roofline"] = hbm_roof

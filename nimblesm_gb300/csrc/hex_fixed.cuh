@@ -5,9 +5,9 @@
 // integer pipes take one wide product (32 x 32 bits to 64) and up to four
 // additions per clock (measured: DFMA 0.0625, mul.wide 1.0, IADD3 2.0 on one
 // of its two pipes).  A 64 x 64 bit product kept to 64 bits is three wide
-// products, so a dot product of three terms costs 9 of them and a dozen
-// additions (10 clocks) where three FP64 instructions cost 48, and an addition
-// 2 instructions instead of 16 clocks.  Elements are well suited to fixed
+// products, so a dot product of three terms costs 9 of them and two more
+// instructions (10 clocks) where three FP64 instructions cost 48, and an
+// addition 2 instructions instead of 16 clocks.  Elements are well suited to fixed
 // point: H = F - I, the cofactors and J are numbers near 0 or 1, and what has
 // a dimension (displacement, geometry, moduli) is scaled per element or per
 // material by a power of two.  Numbers carry 56 to 61 bits below the largest
@@ -57,12 +57,12 @@ NSM_HD Limbs split(i64 x)
 
 // a b (spelled out: the compiler takes the C++ form apart into 64-bit products
 // of the limbs' parts, five times the work).  The product alone, not mad.wide:
-// the hardware adds a 64-bit number to a wide product by two more instructions,
-// where sums in C++ take two products with one addition of three numbers (and
-// its carry): 1,513 instructions per point became 1,194 and the element kernel
-// 1,105 us instead of 1,240 at 2,097,152 elements; the funnel shifts below give
-// 14 us more.  (A third addend of zero in the additions of two, to keep them
-// off the multiplier: 1,103 to 1,193 us.)
+// sums in C++ let the compiler put the additions into the products (a sum of
+// three 64 x 64 bit products is 9 + 2 instructions), which it does not do for
+// a chain of mad.wide: 1,513 instructions per point became 1,194 and the
+// element kernel 1,105 us instead of 1,240 at 2,097,152 elements; the funnel
+// shifts below give 14 us more.  (A third addend of zero in additions of two,
+// to keep them off the multiplier's pipe: 1,103 to 1,193 us.)
 NSM_HD u64 mul_wide(int a, int b)
 {
 #ifdef __CUDA_ARCH__
