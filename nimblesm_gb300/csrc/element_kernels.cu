@@ -6,6 +6,7 @@
 // hex_math.cuh.
 #include <algorithm>
 
+#include "element_packed.cuh"
 #include "element_work.cuh"
 
 namespace nsm {
@@ -56,6 +57,8 @@ __device__ __forceinline__ void stage_nodes(const ElementArgs& a, const int* con
   }
 }
 
+// kPacked: two points per operation (element_packed.cuh).
+template <bool kPacked>
 __global__ void __launch_bounds__(128, 3) k_element_staged(ElementArgs a)
 {
   extern __shared__ __align__(16) uint8_t stage_mem[];  // [2][16][blockDim.x] float4, then [2][8][blockDim.x] int
@@ -81,7 +84,8 @@ __global__ void __launch_bounds__(128, 3) k_element_staged(ElementArgs a)
     if (e + stride < a.E) stage_nodes(a, cnxt, nxt, B);
     if (e + 2 * stride < a.E) stage_conn(a, e + 2 * stride, ccur, B);
     cp_async_commit();
-    element_work<float, false>(a, (int)e, StagedNodes{cur, B});
+    if constexpr (kPacked) element_work_packed(a, (int)e, StagedNodes{cur, B});
+    else element_work<float, false>(a, (int)e, StagedNodes{cur, B});
     // a whole warp's tile has been read before a lane's next copies arrive in it
     if (a.store_ip != kStoreNever && e - (threadIdx.x & 31) + 32 <= a.E) __syncwarp();
     float4* t = cur;
@@ -149,6 +153,24 @@ cudaError_t launch_element_pass(const ElementArgs& a, int is_float, int pass, cu
   return cudaGetLastError();
 }
 
+template <bool kPacked>
+static cudaError_t launch_staged(const ElementArgs& a, const ElementLaunch& l, int block, cudaStream_t stream)
+{
+  static std::atomic<unsigned long long> configured{0};
+  cudaError_t err = once_per_device(configured, [] {  // 72 KB at 128 threads: above the default 48 KB of dynamic shared memory
+    cudaError_t e = cudaFuncSetAttribute(k_element_staged<kPacked>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         2 * kStageBytes * 128);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_element_staged<kPacked>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return e;
+  });
+  if (err != cudaSuccess) return err;
+  ElementArgs b    = a;
+  b.persistent     = 1;
+  const int   grid = std::min(grid_for(a.E - a.e_begin, block), (l.blocks_per_sm > 0 ? l.blocks_per_sm : 1) * num_sms());
+  return launch_overlapped(k_element_staged<kPacked>, grid, block, 2 * kStageBytes * block, stream, a.overlap != 0, b);
+}
+
 cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
   if (a.E <= a.e_begin) return cudaSuccess;
@@ -164,23 +186,8 @@ cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cu
     }
     return cudaGetLastError();
   }
-  const size_t smem  = 2 * kStageBytes * block;
-  static bool  configured = false;
-  if (!configured) {  // 72 KB at 128 threads: above the default 48 KB of dynamic shared memory
-    const int   most = 2 * kStageBytes * 128;
-    cudaError_t err  = cudaSuccess;
-    err = cudaFuncSetAttribute(k_element_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_element_staged, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (err != cudaSuccess) return err;
-    configured = true;
-  }
-  ElementArgs  b     = a;
-  b.persistent       = 1;
-  int grid           = grid_for(a.E - a.e_begin, block);
-  const int g        = (l.blocks_per_sm > 0 ? l.blocks_per_sm : 1) * num_sms();
-  if (g < grid) grid = g;
-  return launch_overlapped(k_element_staged, grid, block, smem, stream, a.overlap != 0, b);
+  return a.store_ip == kStoreNever && !a.has_elastic ? launch_staged<true>(a, l, block, stream)
+                                                     : launch_staged<false>(a, l, block, stream);
 }
 
 // Energies of the current state, FP64 whatever the element precision:

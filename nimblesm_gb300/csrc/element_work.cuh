@@ -138,6 +138,38 @@ struct StagedNodes {
   __device__ __forceinline__ Tile tile(uint4*) const { return Tile{reinterpret_cast<uint4*>(s - (threadIdx.x & 31)), B}; }
 };
 
+// An element's nodal forces, and what they report.
+template <typename T>
+__device__ __forceinline__ void store_forces(const ElementArgs& a, const int e, const T f[8][3], bool bad)
+{
+  const long ld_e = a.ld_e;
+  T    fv[24];
+  bool finite = true;
+#pragma unroll
+  for (int n = 0; n < 8; n++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      fv[n * 3 + i] = f[n][i];
+      finite        = finite & finite_bits(f[n][i]);
+    }
+  bool planes = true;
+  if constexpr (sizeof(T) == 4) {
+    planes = a.fe_slot == nullptr;
+    if (!planes) {
+#pragma unroll
+      for (int n = 0; n < 8; n++)
+        reinterpret_cast<float4*>(a.fe)[__ldg(&a.fe_slot[n * ld_e + e])] =
+            make_float4(fv[3 * n], fv[3 * n + 1], fv[3 * n + 2], 0.0f);
+    }
+  }
+  if (planes) {
+    T* fe = reinterpret_cast<T*>(a.fe) + e;
+#pragma unroll
+    for (int q = 0; q < 24; q++) fe[(size_t)q * ld_e] = fv[q];
+  }
+  if (bad || !finite) atomicOr(a.status, (bad ? NSM_STATUS_BAD_JACOBIAN : 0) | (finite ? 0 : NSM_STATUS_NONFINITE));
+}
+
 // FP64 form: reference geometry precomputed (geo planes).  FP32 form: the
 // reference Jacobian is rebuilt from X each step with the same transform.
 // kPass: 0 the fused step (F, sigma, records, forces); with a block-material
@@ -283,31 +315,7 @@ __device__ __forceinline__ void element_work(const ElementArgs& a, const int e, 
   // the factor 8^2 of the modal gradient, dN/dxi another 8: scale -1/512.
   T f[8][3];
   nodal_adjoint<T>(S, T(-1.0 / 512.0), f);
-  T    fv[24];
-  bool finite = true;
-#pragma unroll
-  for (int n = 0; n < 8; n++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      fv[n * 3 + i] = f[n][i];
-      finite        = finite & finite_bits(f[n][i]);
-    }
-  bool planes = true;
-  if constexpr (sizeof(T) == 4) {
-    planes = a.fe_slot == nullptr;
-    if (!planes) {
-#pragma unroll
-      for (int n = 0; n < 8; n++)
-        reinterpret_cast<float4*>(a.fe)[__ldg(&a.fe_slot[n * ld_e + e])] =
-            make_float4(fv[3 * n], fv[3 * n + 1], fv[3 * n + 2], 0.0f);
-    }
-  }
-  if (planes) {
-    T* fe = reinterpret_cast<T*>(a.fe) + e;
-#pragma unroll
-    for (int q = 0; q < 24; q++) fe[(size_t)q * ld_e] = fv[q];
-  }
-  if (bad || !finite) atomicOr(a.status, (bad ? NSM_STATUS_BAD_JACOBIAN : 0) | (finite ? 0 : NSM_STATUS_NONFINITE));
+  store_forces<T>(a, e, f, bad);
 }
 
 }  // namespace nsm
