@@ -114,6 +114,16 @@ NSM_HD i64 mul(Limbs a, Limbs b)
   return s.value();
 }
 
+// The same to the nearest.
+template <int k>
+NSM_HD i64 mul_rounded(Limbs a, Limbs b)
+{
+  Acc<k> s;
+  s.mid = 1ull << (31 - k);
+  s.add(a, b);
+  return s.value();
+}
+
 constexpr i64 kOne = 1ll << 60;  // 1.0 of H, F, the cofactors, J
 
 // Powers and constants.
@@ -299,8 +309,12 @@ NSM_HD void powers(i64 t, i64& r5, i64& rj)
 // largest has 60 bits, e places beyond the scale of H at 2^60, and H, the
 // stress and the forces are at 2^(60 + e), ...  (`bits` the length of the
 // largest mode of the element, at 2^sc.)  e out of [-3, 40] after this: strains
-// above the domain.  The forces keep kElasticForce further places.
-constexpr int kElasticForce = 3;
+// above the domain.  The forces keep kElasticForce further places: with three,
+// sums in one of 1,000 elements left 63 bits, and one element left to the FP64
+// code makes a launch wait 45 us for it (21,952 elements, half of them elastic:
+// 42 to 74 us a step, 25.5 with two).  Products of the stress are rounded instead of
+// cut, which gives the forces 1.8e-16 of themselves (2.1e-16 before; FP64 2.0e-16).
+constexpr int kElasticForce = 2;
 NSM_HD void elastic_scale(int bits, int sc, int su, int& sh, int& e)
 {
   sh = 60 - bits;
@@ -368,10 +382,10 @@ NSM_HD unsigned elastic_force(const Moduli& m, i64 det, const i64 He[3][3], Poin
 #pragma unroll
   for (int q = 0; q < 6; q++) {
     const int i = q < 3 ? q : (q == 3 ? 0 : (q == 4 ? 1 : 2)), j = q < 3 ? q : (q == 3 ? 1 : (q == 4 ? 2 : 0));
-    const i64 v = mul<4>(split(He[i][j] + He[j][i]), g) + (q < 3 ? l : 0);
+    const i64 v = mul_rounded<4>(split(He[i][j] + He[j][i]), g) + (q < 3 ? l : 0);
     bad |= outside<29>(v);
     if (kStress) p.sig[q] = v;
-    s[q] = split(mul<2>(split(v), d));
+    s[q] = split(mul_rounded<2>(split(v), d));
   }
 #pragma unroll
   for (int J = 0; J < 3; J++) {
@@ -379,6 +393,7 @@ NSM_HD unsigned elastic_force(const Moduli& m, i64 det, const i64 He[3][3], Poin
 #pragma unroll
     for (int i = 0; i < 3; i++) {
       Acc<4 + kElasticForce> a;
+      a.mid = 1ull << (31 - (4 + kElasticForce));
       a.add(c0, s[sym_slot(0, i)]);
       a.add(c1, s[sym_slot(1, i)]);
       a.add(c2, s[sym_slot(2, i)]);
