@@ -206,13 +206,19 @@ void free_all(nsm_model* m)
 // (a new array), the device's write would wait for the page by itself: 0.4 to
 // 1.7 ms for 0.8 MB on a heap that grows and shrinks, 38 us into pages that are
 // there.  So each page is written to first (65 us in all; reading what it holds
-// and writing that back would fault twice: 10 times as long).
+// and writing that back would fault twice: 10 times as long).  Only pageable
+// memory: pinned pages are there, and what is not the host's is the copy's to
+// refuse.
 cudaError_t read_result(void* dst, const void* src, size_t bytes, cudaStream_t stream)
 {
-  static const size_t  page = (size_t)sysconf(_SC_PAGESIZE);
-  volatile char* const p    = static_cast<volatile char*>(dst);
-  for (size_t o = 0; o < bytes; o += page) p[o] = 0;
-  if (bytes > 0) p[bytes - 1] = 0;
+  static const size_t   page = (size_t)sysconf(_SC_PAGESIZE);
+  volatile char* const  p    = static_cast<volatile char*>(dst);
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
+  else if (at.type == cudaMemoryTypeUnregistered) {
+    for (size_t o = 0; o < bytes; o += page) p[o] = 0;
+    if (bytes > 0) p[bytes - 1] = 0;
+  }
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
 }
 
