@@ -481,6 +481,30 @@ cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream)
   return launch_nodes<double, true, false>(a, stream);
 }
 
+// The place of each element corner's force record: the node's j-th incidence at
+// j ld_n + n, the ones past its eighth in any order after all of those.
+__global__ void k_force_slots(int N, long ld_n, long ld_e, const int* __restrict__ node_ptr,
+                              const int* __restrict__ node_inc, int* __restrict__ counter, int* __restrict__ fe_slot)
+{
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const int k0 = node_ptr[n], count = node_ptr[n + 1] - k0;
+  int       past = count > kFirst ? 8 * (int)ld_n + atomicAdd(counter, count - kFirst) : 0;
+  for (int j = 0; j < count; j++) {
+    const int ec                         = node_inc[k0 + j];
+    fe_slot[(ec & 7) * ld_e + (ec >> 3)] = j < kFirst ? j * (int)ld_n + n : past++;
+  }
+}
+
+cudaError_t launch_force_slots(int N, long ld_n, long ld_e, const int* node_ptr, const int* node_inc, int* counter,
+                               int* fe_slot, cudaStream_t stream)
+{
+  if (N == 0) return cudaSuccess;
+  k_force_slots<<<grid_for(N, 256), 256, 0, stream>>>(N, ld_n, ld_e, node_ptr, node_inc, counter, fe_slot);
+  const cudaError_t err = cudaGetLastError();
+  return err != cudaSuccess ? err : cudaMemsetAsync(counter, 0, sizeof(int), stream);
+}
+
 // One thread per (slot, component) and step (grid row): a program's latency on
 // the FP64 pipe (a sine takes about 15 us) is that of one evaluation however
 // many steps are evaluated at once.

@@ -212,6 +212,10 @@ struct NodeArgs {
 // of L1: the FP32 step of a mesh without locality went from 89 to 109 us).
 constexpr int kSmallNodes = 4 * 256 * 152 / 3;
 cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream);
+// fe_slot from the incidences.  `counter`: a zero on the device, zero again
+// afterwards.
+cudaError_t launch_force_slots(int N, long ld_n, long ld_e, const int* node_ptr, const int* node_inc, int* counter,
+                               int* fe_slot, cudaStream_t stream);
 // The kinematic slots' expressions at their nodes (slot_node) and at the
 // schedule's times of `steps` steps from offset k: out [steps][num_slots][3].
 struct BcExprSteps {

@@ -796,21 +796,14 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
       for (int j = 0; j < 8 && ptr[n] + j < ptr[n + 1]; j++) slots[(size_t)j * m->ld_n + n] = inc[ptr[n] + j];
       if (ptr[n + 1] - ptr[n] > 8) more[n >> 5] |= 1u << (n & 31);
     }
-    size_t           fe_values = (size_t)24 * m->ld_e;
-    std::vector<int> at;
-    long             past = 8 * m->ld_n;  // records so far
-    for (int n = 0; n < N; n++) past += std::max(0, ptr[n + 1] - ptr[n] - 8);
-    if (m->precision == NSM_PRECISION_FP32_MIXED && past <= kMaxForceRecords &&
-        force_records_pay(N, E, m->ld_n, slots, gconn.data())) {
-      fe_values = (size_t)past * 4;
-      past      = 8 * m->ld_n;
-      at.assign((size_t)8 * m->ld_e, 0);
-      for (int n = 0; n < N; n++)
-        for (int k = ptr[n]; k < ptr[n + 1]; k++)
-          at[(size_t)(inc[k] & 7) * m->ld_e + (inc[k] >> 3)] =
-              (int)(k - ptr[n] < 8 ? (k - ptr[n]) * m->ld_n + n : past++);
-      NSM_CUDA_B(cudaMalloc(&m->d_fe_slot, sizeof(int) * at.size()));
-      NSM_CUDA_B(cudaMemcpyAsync(m->d_fe_slot, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, m->stream));
+    size_t fe_values = (size_t)24 * m->ld_e;
+    long   num_records = 8 * m->ld_n;
+    for (int n = 0; n < N; n++) num_records += std::max(0, ptr[n + 1] - ptr[n] - 8);
+    const bool records = m->precision == NSM_PRECISION_FP32_MIXED && num_records <= kMaxForceRecords &&
+                         force_records_pay(N, E, m->ld_n, slots, gconn.data());
+    if (records) {
+      fe_values = (size_t)num_records * 4;
+      NSM_CUDA_B(cudaMalloc(&m->d_fe_slot, sizeof(int) * 8 * m->ld_e));
     }
     NSM_CUDA_B(cudaMalloc(&m->d_fe, eb * fe_values));
     NSM_CUDA_B(cudaMemsetAsync(m->d_fe, 0, eb * fe_values, m->stream));
@@ -829,6 +822,9 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     if (E > 0)
       NSM_CUDA_B(cudaMemcpyAsync(m->d_node_inc, inc.data(), sizeof(int) * inc.size(), cudaMemcpyHostToDevice,
                                  m->stream));
+    if (records)
+      NSM_CUDA_B(nsm::launch_force_slots(N, m->ld_n, m->ld_e, m->d_node_ptr, m->d_node_inc, m->d_step_base, m->d_fe_slot,
+                                         m->stream));
     if (num_mats > 1) {
       NSM_CUDA_B(cudaMalloc(&m->d_elem_group, sizeof(int) * (E > 0 ? E : 1)));
       if (E > 0)
@@ -1683,15 +1679,23 @@ int nsm_launch_candidate_times(nsm_model* m, int repeats, double* ms, int capaci
   if (count) *count = kNumLaunchCandidates;
   NSM_CUDA(cudaSetDevice(m->device));
   const nsm::ElementLaunch keep = m->elaunch;
-  cudaEvent_t              a, b;
+  // as steps inside an advance launch it: without records
+  auto run = [&]() -> cudaError_t {
+    if (has_callbacks(m) || m->closure) return launch_element(m, -1, true);
+    nsm::ElementArgs args = element_args(m, -1, true);
+    args.store_ip         = nsm::kStoreNever;
+    return m->precision == NSM_PRECISION_FP64 ? nsm::launch_element_fp64(args, m->elaunch, m->stream)
+                                              : nsm::launch_element_fp32(args, m->elaunch, m->stream);
+  };
+  cudaEvent_t a, b;
   NSM_CUDA(cudaEventCreate(&a));
   NSM_CUDA(cudaEventCreate(&b));
   cudaError_t err = cudaSuccess;
   for (int c = 0; c < kNumLaunchCandidates && c < capacity && err == cudaSuccess; c++) {
     m->elaunch = kLaunchCandidates[c];
-    err        = launch_element(m, -1, true);  // warm
+    err        = run();  // warm
     if (err == cudaSuccess) err = cudaEventRecord(a, m->stream);
-    for (int r = 0; r < repeats && err == cudaSuccess; r++) err = launch_element(m, -1, true);
+    for (int r = 0; r < repeats && err == cudaSuccess; r++) err = run();
     if (err == cudaSuccess) err = cudaEventRecord(b, m->stream);
     if (err == cudaSuccess) err = cudaEventSynchronize(b);
     float t = 0;
@@ -1699,6 +1703,7 @@ int nsm_launch_candidate_times(nsm_model* m, int repeats, double* ms, int capaci
     ms[c] = t / repeats;
   }
   m->elaunch = keep;
+  if (err == cudaSuccess) err = launch_element(m, -1, true);  // the records are left those of the current state
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   NSM_CUDA(err);
