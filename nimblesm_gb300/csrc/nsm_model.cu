@@ -361,11 +361,14 @@ nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
   a.sched     = k < 0 ? nullptr : m->d_sched;
   a.step_base = m->d_step_base;
   a.k         = k;
-  // Started ahead of the node kernel's end where its blocks are few (more would
-  // share SMs that are free at that moment with each other: 4,096 elements 10.7
-  // us a step against 9.7, 100 elements 7.8 against 8.6), and for the learned
-  // closure, whose kernel has weights and tensor memory to set up.
-  a.overlap   = k >= 0 && (m->E <= 1024 || m->closure);
+  // Started ahead of the node kernel's end where its blocks are few (more share
+  // the SMs that are free at that moment with each other; us a step started
+  // after and ahead: 1,728 elements 7.5 and 6.3, 4,096 9.0 and 8.4, 10,648 13.8
+  // and 12.9, 13,824 14.6 and 15.5; FP32 4,096 6.3 and 5.8, 8,000 7.2 and 6.5,
+  // 13,824 8.0 and 8.2; 8,192 elements with the 49,130 nodes of ten samples 16.1
+  // and 18.8), and for the learned closure, whose kernel has weights and tensor
+  // memory to set up.
+  a.overlap   = k >= 0 && ((m->E <= 12000 && m->N <= 14000) || m->closure);
   a.status    = m->d_status;
   return a;
 }
