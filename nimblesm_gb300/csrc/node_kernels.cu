@@ -307,8 +307,13 @@ __device__ __forceinline__ void begin_step(const NodeArgs& a, int n, int c0, int
 // step waits for latency: a third of the serial FP64 operations (64 clocks
 // each for a warp by itself), and the loads of state and schedule overlap the
 // element kernel's end.  (Three components that far ahead would spill.)
-template <typename TF, bool kExact, int kComps, bool kRecords>
-__global__ void __launch_bounds__(256, kComps == 3 && sizeof(TF) == 4 && !kRecords ? 5 : 4) k_node_update(NodeArgs a)
+// kBlocks per SM: FP32 meshes beyond L2 wait for memory, 128^3 96.3 us with 5
+// (48 registers), 92.1 with 6 (40, 52 bytes spilled), 105 with 7 (32); within it
+// the spills cost more, 64^3 37.6 us a step with 5, 38.2 with 6 (90^3 101.5 and
+// 100).  FP64 122 us with 4, 133 with 5, 138 with 3; FP32 records 15.2 with 4,
+// 16.3 with 5.
+template <typename TF, bool kExact, int kComps, bool kRecords, int kBlocks>
+__global__ void __launch_bounds__(256, kBlocks) k_node_update(NodeArgs a)
 {
   constexpr bool kAhead = kComps == 1;
   const int      n      = a.n_begin + blockIdx.x * blockDim.x + threadIdx.x;
@@ -451,12 +456,15 @@ static cudaError_t launch_small(const NodeArgs& a, int count, cudaStream_t strea
   // element step with overlapped launches: 16.5 us with differing splits).
   static std::atomic<unsigned long long> configured{0};
   cudaError_t err = once_per_device(configured, [] {
-    return cudaFuncSetAttribute(k_node_update<TF, kExact, 1, kRecords>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return cudaFuncSetAttribute(k_node_update<TF, kExact, 1, kRecords, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   });
   if (err != cudaSuccess) return err;
   const int block = count <= 64 * 152 ? 64 : 256;  // the smallest meshes over more SMs
-  return launch_overlapped(k_node_update<TF, kExact, 1, kRecords>, dim3(grid_for(count, block), 3), block, 0, stream, a.overlap != 0, a);
+  return launch_overlapped(k_node_update<TF, kExact, 1, kRecords, 4>, dim3(grid_for(count, block), 3), block, 0, stream, a.overlap != 0, a);
 }
+
+// Nodes whose step (250 bytes each in the FP32 form) does not stay in L2.
+constexpr int kBeyondL2 = 500000;
 
 template <typename TF, bool kExact, bool kRecords>
 static cudaError_t launch_nodes(const NodeArgs& a, cudaStream_t stream)
@@ -470,8 +478,10 @@ static cudaError_t launch_nodes(const NodeArgs& a, cudaStream_t stream)
                              a.overlap != 0, a);
   }
   if (count <= kSmallNodes) return launch_small<TF, kExact, kRecords>(a, count, stream);
-  return launch_overlapped(k_node_update<TF, kExact, 3, kRecords>, dim3(grid_for(count, 256)), 256, 0, stream,
-                           a.overlap != 0, a);
+  constexpr int kFew = sizeof(TF) == 4 && !kRecords ? 5 : 4, kMore = sizeof(TF) == 4 && !kRecords ? 6 : 4;
+  return launch_overlapped(count > kBeyondL2 ? k_node_update<TF, kExact, 3, kRecords, kMore>
+                                             : k_node_update<TF, kExact, 3, kRecords, kFew>,
+                           dim3(grid_for(count, 256)), 256, 0, stream, a.overlap != 0, a);
 }
 
 cudaError_t launch_node_update(const NodeArgs& a, cudaStream_t stream)
