@@ -343,8 +343,10 @@ int nsm_time_kernels(nsm_model* model, int repeats, double* element_ms, double* 
 int nsm_autotune(nsm_model* model, int repeats, int* chosen, double* best_ms);
 /* The autotuner's measurements: mean milliseconds of `repeats` element-kernel
  * launches for each candidate launch shape, in candidate order, into
- * ms[0 .. capacity); *count receives the number of candidates.  The model's
- * own launch shape is left as it was. */
+ * ms[0 .. capacity); *count receives the number of candidates.  The launches
+ * are those of steps inside an advance, which store no point records; the
+ * records are left those of the current state, and the model's own launch
+ * shape as it was. */
 int nsm_launch_candidate_times(nsm_model* model, int repeats, double* ms, int capacity, int* count);
 /* Sets the element kernel's launch shape to candidate `candidate` of the
  * autotuner's list (what nsm_autotune does with its choice). */
