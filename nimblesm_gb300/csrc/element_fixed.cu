@@ -257,6 +257,10 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     if (!elastic) sc = min(sc, su);
     int      sh = su - sc, ee = 0;
     unsigned bad = (unsigned)(mat.exponent + 400) > 800u;
+    // An infinity or a NaN, or numbers whose sums may become one (2^1017 and
+    // more): an elastic element's modes do not show it, as the same value at all
+    // corners leaves nothing in any difference.
+    if (kHasElastic) bad |= exm > 0x7f7;
 
     // ---- modes and gradients ----
     fx::Gradient G[3];
