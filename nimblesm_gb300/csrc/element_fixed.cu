@@ -40,30 +40,42 @@ using fx::u64;
 // Geometry of 8 elements in fixed point, one block of kGeoRows rows of 32
 // lanes (row (side along xi, value), lane [side along (zeta, eta)][element]):
 // per point G0 (9 values, row-major, as limbs) and the reference volume; the
-// last row holds each element's exponents.  A warp's working set is this one
-// block, which a bulk copy brings to shared memory while the previous one is
-// computed on.
+// last row holds each element's exponents and, of elastic elements, fx::Rows
+// (bits 16-27).  A warp's working set is this one block, which a bulk copy
+// brings to shared memory while the previous one is computed on.
 constexpr int kGeoPoint = 10, kGeoRows = 2 * kGeoPoint + 1, kGeoBlock = kGeoRows * 32;  // words
 constexpr int kGeoBytes = kGeoBlock * 8;
 
 // From the FP64 planes: G0 scaled by 2^sG so that its largest entry over the
-// points is in [2^60, 2^61), the volume det J_X over 2^Ed (the largest in
-// [1/2, 1)) at 2^62, and the exponents su = 124 - sG and Ed - sG + 2.
-__global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ geo, i64* __restrict__ out)
+// points is in [2^60, 2^61) (of elastic elements each row's), the volume det J_X
+// over 2^Ed (the largest in [1/2, 1)) at 2^62, and the exponents su = 124 - sG
+// and Ed - sG + 2.
+__global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ geo, const int* __restrict__ elem_group,
+                                 const FixedMaterial* __restrict__ mats, i64* __restrict__ out)
 {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
-  double gmax = 0.0, dmax = 0.0;
+  const bool elastic = mats[elem_group ? elem_group[e] : 0].model == kElastic;
+  double     row[3] = {0.0, 0.0, 0.0}, dmax = 0.0;
   for (int p = 0; p < 8; p++) {
-    for (int q = 0; q < 9; q++) gmax = fmax(gmax, fabs(geo[(p * kGeoPerPoint + q) * ld_e + e]));
+    for (int q = 0; q < 9; q++) row[q / 3] = fmax(row[q / 3], fabs(geo[(p * kGeoPerPoint + q) * ld_e + e]));
     dmax = fmax(dmax, geo[(p * kGeoPerPoint + 9) * ld_e + e]);
   }
-  int eg = 0, ed = 0;
+  const double gmax = fmax(row[0], fmax(row[1], row[2])), gmin = fmin(row[0], fmin(row[1], row[2]));
+  int          eg = 0, ed = 0, places[3] = {0, 0, 0};
   frexp(gmax, &eg);
   frexp(dmax, &ed);
   // (values far from 1 leave the element to the FP64 code)
-  const bool fits = gmax > 1e-90 && gmax < 1e90 && dmax > 1e-60 && dmax < 1e60;
-  const int  sG   = 61 - eg, su = fits ? 124 - sG : 1 << 20, ef = fits ? ed - sG + 2 : 0;
+  bool fits = gmax > 1e-90 && gmax < 1e90 && gmin > 0.0 && dmax > 1e-60 && dmax < 1e60;
+  if (elastic && fits)
+    for (int d = 0; d < 3; d++) {
+      int er;
+      frexp(row[d], &er);
+      places[d] = eg - er;
+      if (places[d] > fx::kMaxRow) fits = false;
+    }
+  const int  sG = 61 - eg, su = fits ? 124 - sG : 1 << 20, ef = fits ? ed - sG + 2 : 0;
+  const int  low = elastic && fits ? (places[0] | places[1] << 4 | places[2] << 8) << 16 | (ef & 0xffff) : ef;
   i64* const base = out + (size_t)(e >> 3) * kGeoBlock + (e & 7);
   for (int p = 0; p < 8; p++) {
     const int  y = sy_of(p), z = sz_of(p), lane = (2 * z + y) * 8;
@@ -71,20 +83,21 @@ __global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ ge
     for (int q = 0; q < 9; q++) {
       const double g    = geo[(p * kGeoPerPoint + q) * ld_e + e];
       const bool   flip = (q / 3 == 1 && y == 0) || (q / 3 == 2 && z == 0);  // mirrored rows
-      const Limbs  l    = fx::split(fits ? __double2ll_rn(scalbn(flip ? -g : g, sG)) : 0);
+      const Limbs  l    = fx::split(fits ? __double2ll_rn(scalbn(flip ? -g : g, sG + places[q / 3])) : 0);
       dst[q * 32]       = (i64)(((u64)(unsigned)l.hi << 32) | (unsigned)l.lo);
     }
     dst[9 * 32] = fits ? __double2ll_rn(scalbn(geo[(p * kGeoPerPoint + 9) * ld_e + e], 62 - ed)) : 0;
-    if (sx_of(p) == 0) base[2 * kGeoPoint * 32 + lane] = (i64)(((u64)(unsigned)su << 32) | (unsigned)ef);
+    if (sx_of(p) == 0) base[2 * kGeoPoint * 32 + lane] = (i64)(((u64)(unsigned)su << 32) | (unsigned)low);
   }
 }
 
 size_t fixed_geometry_words(long ld_e) { return (size_t)((ld_e + 7) / 8) * kGeoBlock; }
 
-cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, long long* out, cudaStream_t stream)
+cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, const int* elem_group, const FixedMaterial* mats,
+                                  long long* out, cudaStream_t stream)
 {
   if (E == 0) return cudaSuccess;
-  k_fixed_geometry<<<grid_for(E, 128), 128, 0, stream>>>(E, ld_e, geo, out);
+  k_fixed_geometry<<<grid_for(E, 128), 128, 0, stream>>>(E, ld_e, geo, elem_group, mats, out);
   return cudaGetLastError();
 }
 
@@ -93,12 +106,19 @@ FixedMaterial fixed_material(const GroupMaterial& m)
   FixedMaterial f{0, 0, 0, 1 << 20, m.model};
   const double  most = std::fmax(m.bulk, m.shear);
   if (!std::isfinite(most) || !(most > 1e-90) || !(most < 1e90)) return f;  // left to the FP64 code
+  // as are ratios of the moduli at which that is the more exact one (hex_fixed.cuh)
+  if (m.model == kElastic ? m.bulk > 8.0 * m.shear : 2.0 * m.bulk < m.shear) return f;
   f.exponent = std::ilogb(most) + 4;
   f.half_k   = std::llrint(std::ldexp(m.bulk, 61 - f.exponent));
   f.shear    = std::llrint(std::ldexp(m.shear, 62 - f.exponent));
   f.lambda   = std::llrint(std::ldexp(m.bulk - 2.0 * m.shear / 3.0, 62 - f.exponent));
   return f;
 }
+
+// Largest scale of an elastic element's displacements: down to 2^-844 they have
+// 57 bits, and zeros convert to zero (fx::to_fixed; at 1079 they would not).
+// Smaller ones are left to the FP64 code.
+constexpr int kMaxScale = 900;
 
 template <int kXor>
 __device__ __forceinline__ i64 other(i64 x)
@@ -238,29 +258,41 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     i64* const       gs    = reinterpret_cast<i64*>(stage + buf * kGeoBytes) + (kPoints == 2 ? lane : (lane & 24) + (eb & 4) + j);
 
     // ---- displacements of the lane's two corners, at 2^sc ----
-    u64 u[3][2];
-    int exm = 0;
+    u64      u[3][2];
+    int      exm = 0;
+    unsigned low = 0;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
       for (int bx = 0; bx < 2; bx++) {
         u[i][bx] = (u64)__double_as_longlong(us[(buf * 6 + i * 2 + bx) * 32]);
         exm      = max(exm, (int)((unsigned)(u[i][bx] >> 32) & 0x7fffffffu));
+        low |= (unsigned)u[i][bx];
       }
+    if (kHasElastic) exm = max(exm, low != 0);
     exm = max(exm, __shfl_xor_sync(0xffffffffu, exm, kAcrossEta));
-    exm = max(exm, __shfl_xor_sync(0xffffffffu, exm, kAcrossZeta)) >> 20;
+    exm = max(exm, __shfl_xor_sync(0xffffffffu, exm, kAcrossZeta));
+    // (of all 24 numbers: none but zeros, or the largest one's exponent)
+    const bool at_rest = exm == 0;
+    exm >>= 20;
     const i64           ge      = gs[2 * kGeoPoint * 32];
     const FixedMaterial mat     = a.fixed_mats[a.elem_group ? __ldg(&a.elem_group[e]) : 0];
     const bool          elastic = kHasElastic && mat.model == kElastic;
     const int           su      = (int)(ge >> 32);
-    int                 sc      = 1079 - exm;
-    if (!elastic) sc = min(sc, su);
-    int      sh = su - sc, ee = 0;
+    int                 sc      = min(1079 - exm, elastic ? kMaxScale : su);
+    int                 ef      = (int)ge;
+    fx::Rows            rows    = {0, 0, 0};
+    int                 sh = su - sc, ee = 0;
     unsigned bad = (unsigned)(mat.exponent + 400) > 800u;
     // An infinity or a NaN, or numbers whose sums may become one (2^1017 and
     // more): an elastic element's modes do not show it, as the same value at all
     // corners leaves nothing in any difference.
     if (kHasElastic) bad |= exm > 0x7f7;
+    if (kHasElastic && elastic) {
+      bad |= exm < 1079 - kMaxScale && !at_rest;  // (shorter than 57 bits at the largest scale)
+      rows = fx::Rows{ef >> 16 & 15, ef >> 20 & 15, ef >> 24 & 15};
+      ef   = (int)(short)ef;
+    }
 
     // ---- modes and gradients ----
     fx::Gradient G[3];
@@ -280,20 +312,16 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       if (kHasElastic && __any_sync(0xffffffffu, elastic)) {
         u64 m = 0;
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int k = 0; k < 7; k++) m |= (u64)(v[i][k] ^ (v[i][k] >> 63));
+        for (int i = 0; i < 3; i++) m |= fx::mode_bits(v[i], rows);
         m |= (u64)other<kAcrossEta>((i64)m);
         m |= (u64)other<kAcrossZeta>((i64)m);
         if (elastic) {
           if (m == 0) sh = 0;
-          else fx::elastic_scale(64 - __clzll((i64)m), sc, su, sh, ee);
-          if (ee < -3) bad = 1, sh = 0, ee = 0;
-          const int up = max(sh, 0), down = min(max(-sh, 0), 63);
+          else fx::elastic_scale(64 - fx::kMaxRow - __clzll((i64)m), sc, su, sh, ee);
+          // strains above the domain; forces or stresses that are not normal numbers
+          if (ee < -3 || min(ef, 0) + mat.exponent - ee < -900) bad = 1, sh = 0, ee = 0;
 #pragma unroll
-          for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int k = 0; k < 7; k++) v[i][k] = (i64)((u64)v[i][k] << up) >> down;
+          for (int i = 0; i < 3; i++) fx::elastic_shift(v[i], rows, sh);
         }
       }
       if (!elastic && sh != 0) {
@@ -303,7 +331,8 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       }
 #pragma unroll
       for (int i = 0; i < 3; i++) {
-        fx::lane_gradient(v[i], G[i]);
+        if (kHasElastic) fx::elastic_gradient(v[i], rows, G[i]);
+        else fx::lane_gradient(v[i], G[i]);
         if (kPoints == 2) {  // the second point's increments wait where the displacements were
           us_i[(buf * 6 + i) * 32]     = G[i].y1;
           us_i[(buf * 6 + 3 + i) * 32] = G[i].z1;
@@ -336,8 +365,8 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
         fx::Point pt;
         if (kHasElastic && elastic) {
           i64       He[3][3];
-          const int up = max(-ee, 0), down = max(ee, 0);
-          fx::displacement_gradient(Du, g0, He);
+          const int up = max(-ee, 0), down = min(max(ee, 0), 63);
+          fx::displacement_gradient<true>(Du, g0, He);
 #pragma unroll
           for (int q = 0; q < 9; q++) {
             pt.H[q / 3][q % 3] = (i64)((u64)He[q / 3][q % 3] << up) >> down;
@@ -382,7 +411,7 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     }
 
     // ---- nodal forces of the lane's corners ----
-    const int    ef    = (int)ge + mat.exponent - ee - (elastic ? fx::kElasticForce : 0);
+    ef += mat.exponent - ee - (elastic ? fx::kElasticForce - fx::kElasticSum : 0);
     const double scale = __longlong_as_double((i64)(1023 + ef) << 52);
     double       f[2][3];
     if (kPoints == 1) {  // both lanes' forces
@@ -393,9 +422,12 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
 #pragma unroll
     for (int i = 0; i < 3; i++) {
       const i64      qx = gs[i * 32], qy = gs[(3 + i) * 32], qz = gs[(6 + i) * 32];
-      const fx::Sums S{Q[0][i] + qx, Q[1][i] + qy, Q[1][i] - qy, Q[2][i] + qz, Q[2][i] - qz};
+      fx::Sums       S{Q[0][i] + qx, Q[1][i] + qy, Q[1][i] - qy, Q[2][i] + qz, Q[2][i] - qz};
       fx::Parts      keep, send;
-      if (elastic) bad |= fx::too_large(S);
+      if (elastic) {
+        fx::common_scale(S, rows);
+        bad |= fx::too_large(S);
+      }
       fx::lane_adjoint(S, keep, send);
       const i64 e0 = keep.e0 + other<kAcrossZeta>(send.e0), e1 = keep.e1 + other<kAcrossZeta>(send.e1);
       const i64 o0 = keep.o0 + other<kAcrossZeta>(send.o0), o1 = keep.o1 + other<kAcrossZeta>(send.o1);

@@ -22,10 +22,15 @@
 // factors at strains from 1e-9 to 3e-2; beside a rigid displacement of the
 // element's size both are 10 to 100 times closer than in FP64.
 //
-// Domain.  |H| < 1/8 (Frobenius) at every point, displacements within 2^26 of
-// the element's scale, finite inputs.  The functions report what leaves it;
-// the caller then evaluates the element in FP64 as a whole, so each element's
-// result depends on its own inputs alone.
+// That is against an FP64 evaluation's J, an error of K 2^-53: neo-Hookean
+// elements of K < G / 2 (where it would be the smaller one) are not evaluated
+// here.  An FP64 evaluation of an elastic element has no such absolute error;
+// how its bits are kept here is said at elastic_scale.
+//
+// Domain.  |H| < 1/8 (Frobenius) at every point, neo-Hookean displacements
+// within 2^26 of the element's scale, finite inputs.  The functions report what
+// leaves it; the caller then evaluates the element in FP64 as a whole, so each
+// element's result depends on its own inputs alone.
 //
 // One element is shared by four lanes, each with one edge along xi: the two
 // points and two corners on its side along eta and zeta.  A lane works in
@@ -225,7 +230,9 @@ struct Point {
   i64      sig[6];   // stress over 2^exponent, 2^62 (elastic 2^(62 + e); when asked for)
 };
 
-// H = Du G0 (Du at 2^su, G0 at 2^sG, su + sG = 124 + e: H at 2^(60 + e)).
+// H = Du G0 (Du at 2^su, G0 at 2^sG, su + sG = 124 + e: H at 2^(60 + e)), cut
+// or rounded.
+template <bool kRound = false>
 NSM_HD void displacement_gradient(const i64 Du[3][3], const Limbs G0[3][3], i64 H[3][3])
 {
 #pragma unroll
@@ -234,6 +241,7 @@ NSM_HD void displacement_gradient(const i64 Du[3][3], const Limbs G0[3][3], i64 
 #pragma unroll
     for (int J = 0; J < 3; J++) {
       Acc<0> s;
+      if (kRound) s.mid = 1ull << 31;
       s.add(d0, G0[0][J]);
       s.add(d1, G0[1][J]);
       s.add(d2, G0[2][J]);
@@ -308,21 +316,81 @@ NSM_HD void powers(i64 t, i64& r5, i64& rj)
 // strains of 1e-3.  Its displacement modes are therefore shifted up until the
 // largest has 60 bits, e places beyond the scale of H at 2^60, and H, the
 // stress and the forces are at 2^(60 + e), ...  (`bits` the length of the
-// largest mode of the element, at 2^sc.)  e out of [-3, 40] after this: strains
-// above the domain.  The forces keep kElasticForce further places: with three,
-// sums in one of 1,000 elements left 63 bits, and one element left to the FP64
-// code makes a launch wait 45 us for it (21,952 elements, half of them elastic:
-// 42 to 74 us a step, 25.5 with two).  Products of the stress are rounded instead of
-// cut, which gives the forces 1.8e-16 of themselves (2.1e-16 before; FP64 2.0e-16).
-constexpr int kElasticForce = 2;
+// largest mode of the element, at 2^sc.)  e below -3: strains above the domain.
+//
+// The rows of its G0 are each scaled to their own largest entry (Rows), and the
+// modes to match, so that a flat element loses few places: forces to 1.0e-16 of
+// themselves for cubes (FP64 1.9e-16) and 1.3e-16 at an aspect ratio of 4 (FP64
+// 3.9e-16; tests/fixed_domain_check.cc).  Flatter elements than kMaxRow says,
+// and materials of K > 8 G (their shear modulus has fewer bits), are left to
+// FP64: in states that FP64 gives without a rounding (plane stress and shear
+// along the axes of an unjittered mesh) they would lose more than a place to it.
+//
+// The forces at the points keep kElasticForce further places: with more, their
+// sums could leave 63 bits, and one element left to the FP64 code makes a launch
+// wait 45 us for it.  Products are rounded, not cut.
+constexpr int kElasticForce = 3;
 NSM_HD void elastic_scale(int bits, int sc, int su, int& sh, int& e)
 {
   sh = 60 - bits;
   e  = sc + sh - su;
-  if (e > 40) {
-    sh -= e - 40;
-    e = 40;
-  }
+}
+
+// Binary places by which the rows xi, eta, zeta of an elastic element's G0 lie
+// below the largest (0) and are stored scaled up.
+constexpr int kMaxRow = 2;
+struct Rows {
+  int x, y, z;
+};
+NSM_HD int lower(int a, int b) { return a < b ? a : b; }
+
+// A mode belongs to the rows of its axes and is kept at the scale of the
+// largest of them (Du of a row at 2^(su - its places)).
+NSM_HD void mode_places(const Rows& r, int places[7])
+{
+  places[kX]   = r.x;
+  places[kY]   = r.y;
+  places[kZ]   = r.z;
+  places[kXY]  = lower(r.x, r.y);
+  places[kXZ]  = lower(r.x, r.z);
+  places[kYZ]  = lower(r.y, r.z);
+  places[kXYZ] = 0;
+}
+
+// The bits of one component's modes, each at its scale and kMaxRow places more:
+// the longest of an element gives `bits` of elastic_scale, kMaxRow less.  (Zero
+// for zeros alone.)
+NSM_HD u64 mode_bits(const i64 v[7], const Rows& r)
+{
+  int places[7];
+  mode_places(r, places);
+  u64 m = 0;
+#pragma unroll
+  for (int k = 0; k < 7; k++) m |= ((u64)(v[k] ^ (v[k] >> 63)) | (u64)(v[k] & 1)) << (kMaxRow - places[k]);
+  return m;
+}
+
+// Shift of the modes to the element's scale (0 <= sh < 60; below 2^62 on the way).
+NSM_HD void elastic_shift(i64 v[7], const Rows& r, int sh)
+{
+  int places[7];
+  mode_places(r, places);
+#pragma unroll
+  for (int k = 0; k < 7; k++) v[k] = (i64)((u64)v[k] << sh) >> places[k];
+}
+
+// lane_gradient with each row's values at the row's scale.
+NSM_HD void elastic_gradient(const i64 v[7], const Rows& r, Gradient& G)
+{
+  int places[7];
+  mode_places(r, places);
+  const i64 xy = times_g(v[kXY]), xz = times_g(v[kXZ]), yz = times_g(v[kYZ]), xyz = mul<0>(split(v[kXYZ]), split(kGG64));
+  const i64 hy = (xy >> (r.y - places[kXY])) + (xyz >> r.y), hz = (xz >> (r.z - places[kXZ])) + (xyz >> r.z);
+  G.x  = v[kX] + (xy >> (r.x - places[kXY])) + (xz >> (r.x - places[kXZ])) + (xyz >> r.x);
+  G.y  = v[kY] + (yz >> (r.y - places[kYZ])) - hy;
+  G.y1 = hy + hy;
+  G.z  = v[kZ] + (yz >> (r.z - places[kYZ])) - hz;
+  G.z1 = hz + hz;
 }
 
 // P[J][i] = det' adj(F) sigma at 2^62 over 2^exponent of the moduli, det' the
@@ -371,33 +439,36 @@ NSM_HD void neohookean_force(const Moduli& m, i64 det, Point& p, i64 P[3][3])
 }
 
 // The same for the elastic material, sigma = G (H + H^T) + lambda tr(H) I, with
-// H at 2^(60 + e) as He: P at 2^(62 + e + kElasticForce).
+// H at 2^(60 + e) as He: P at 2^(62 + e + kElasticForce).  adj(F) sigma is
+// formed as sigma + (adj(F) - I) sigma: the first term loses nothing, and the
+// products of the second have two places more.
 template <bool kStress>
 NSM_HD unsigned elastic_force(const Moduli& m, i64 det, const i64 He[3][3], Point& p, i64 P[3][3])
 {
   unsigned    bad = 0;
   const Limbs d = split(det), g = split(m.g);
-  const i64   l = mul<4>(split(He[0][0] + He[1][1] + He[2][2]), split(m.lambda));
-  Limbs       s[6];
+  const i64   l = mul_rounded<4>(split(He[0][0] + He[1][1] + He[2][2]), split(m.lambda));
+  i64         s[6];
 #pragma unroll
   for (int q = 0; q < 6; q++) {
     const int i = q < 3 ? q : (q == 3 ? 0 : (q == 4 ? 1 : 2)), j = q < 3 ? q : (q == 3 ? 1 : (q == 4 ? 2 : 0));
     const i64 v = mul_rounded<4>(split(He[i][j] + He[j][i]), g) + (q < 3 ? l : 0);
-    bad |= outside<29>(v);
     if (kStress) p.sig[q] = v;
-    s[q] = split(mul_rounded<2>(split(v), d));
+    s[q] = mul_rounded<2>(split(v), d);
+    bad |= outside<26>(s[q]);  // (P below 2^62.2)
   }
 #pragma unroll
   for (int J = 0; J < 3; J++) {
-    const Limbs c0 = split(p.C[0][J]), c1 = split(p.C[1][J]), c2 = split(p.C[2][J]);
+    Limbs c[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) c[k] = split((i64)((u64)(p.C[k][J] - (k == J ? kOne : 0)) << 2));
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      Acc<4 + kElasticForce> a;
-      a.mid = 1ull << (31 - (4 + kElasticForce));
-      a.add(c0, s[sym_slot(0, i)]);
-      a.add(c1, s[sym_slot(1, i)]);
-      a.add(c2, s[sym_slot(2, i)]);
-      P[J][i] = a.value();
+      Acc<2 + kElasticForce> a;
+      a.mid = 1ull << (31 - (2 + kElasticForce));
+#pragma unroll
+      for (int k = 0; k < 3; k++) a.add(c[k], split(s[sym_slot(k, i)]));
+      P[J][i] = a.value() + (i64)((u64)s[sym_slot(J, i)] << kElasticForce);
     }
   }
   return bad;
@@ -429,10 +500,26 @@ struct Sums {
   i64 x, y, y1, z, z1;
 };
 
-// Whether the forces of sums this large may leave 63 bits.
+// An elastic element's sums from the scales of their rows to a common one,
+// kElasticSum places below that of the forces at the points (one place: 7 to 14
+// of 20,000 unjittered cubes would be too large without it, none with it).
+constexpr int kElasticSum = 1;
+NSM_HD i64 rounded_down(i64 x, int places) { return (x + (1ll << (places - 1))) >> places; }
+NSM_HD void common_scale(Sums& S, const Rows& r)
+{
+  S.x  = rounded_down(S.x, r.x + kElasticSum);
+  S.y  = rounded_down(S.y, r.y + kElasticSum);
+  S.y1 = rounded_down(S.y1, r.y + kElasticSum);
+  S.z  = rounded_down(S.z, r.z + kElasticSum);
+  S.z1 = rounded_down(S.z1, r.z + kElasticSum);
+}
+
+// Whether the forces of sums this large may leave 63 bits: a force is at most
+// 29.8 of the largest sum (lane_adjoint: 3.15 even and 4.31 odd in xi, four
+// lanes), and those of 2^58 and less stay below 2^62.9.
 NSM_HD unsigned too_large(const Sums& S)
 {
-  return outside<25>(S.x) | outside<25>(S.y) | outside<25>(S.y1) | outside<25>(S.z) | outside<25>(S.z1);
+  return outside<26>(S.x) | outside<26>(S.y) | outside<26>(S.y1) | outside<26>(S.z) | outside<26>(S.z1);
 }
 
 // A lane's part of the forces in one component, even and odd in xi, with and

@@ -140,7 +140,9 @@ cudaError_t launch_element_pass(const ElementArgs& a, int is_float, int pass, cu
 int         num_sms();
 // The FP64 form's fixed-point geometry (words: 64-bit), from the geo planes.
 size_t      fixed_geometry_words(long ld_e);
-cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, long long* out, cudaStream_t stream);
+// (elem_group: material of each element, or null)
+cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, const int* elem_group, const FixedMaterial* mats,
+                                  long long* out, cudaStream_t stream);
 // F = I (sigma = 0) in every point record: the element data before the first step.
 cudaError_t launch_ip_identity(int E, long ld_e, void* ip, int ip_is_float, cudaStream_t stream);
 

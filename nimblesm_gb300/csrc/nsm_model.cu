@@ -875,7 +875,7 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
         e = cudaMemcpyAsync(m->d_fixed_mats, fixed_mats.data(), sizeof(nsm::FixedMaterial) * num_mats,
                             cudaMemcpyHostToDevice, m->stream);
       if (e == cudaSuccess)
-        e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_geo_fixed, m->stream);
+        e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_elem_group, m->d_fixed_mats, m->d_geo_fixed, m->stream);
     }
     m->dt_group.assign(S, 1.7976931348623157e308);
     if (e == cudaSuccess)
