@@ -449,6 +449,12 @@ int nsm_tc_selftest(int N, int K, const float* A, const float* B, float* D);
  * library is bounded the same way, at one second.) */
 int nsm_tc_wait_timeout_selftest(long limit_us, int* timed_out);
 
+/* Diagnostic of the FP64 element kernel's bounded wait, which a warp ends as a
+ * whole: half the lanes of a warp give up after `limit_us` (1..10000)
+ * microseconds, the phase completes at five times that.  *lanes_on: the lanes
+ * that would go on (0; any other number but 32 would leave a warp divided). */
+int nsm_warp_wait_selftest(long limit_us, int* lanes_on);
+
 /* Number of SMs of the device. */
 int nsm_device_sm_count(int device, int* count);
 

@@ -240,8 +240,11 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
   uint32_t phase = 0;  // bit b: parity of block b's next copy
   for (int buf = 0; g < g_end; g += g_step, buf ^= 1) {
     cp_async_wait_all();
-    if (!tc::mbar_wait(&bar[buf], (phase >> buf) & 1u)) {  // (bounded; nothing else of this warp is in flight)
-      atomicOr(a.status, NSM_STATUS_TIMEOUT);
+    if (!tc::mbar_wait_warp(&bar[buf], (phase >> buf) & 1u)) {
+      // Given up, as a warp.  Once more for the late copy, so that it does not
+      // land in another block's memory; nothing else of this warp is in flight.
+      tc::mbar_wait_warp(&bar[buf], (phase >> buf) & 1u);
+      if (lane == 0) atomicOr(a.status, NSM_STATUS_COPY_TIMEOUT);
       return;
     }
     phase ^= 1u << buf;

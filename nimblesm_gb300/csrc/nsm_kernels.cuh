@@ -12,6 +12,7 @@
 #define NSM_STATUS_BAD_JACOBIAN 1   // a non-positive Jacobian determinant (inverted element)
 #define NSM_STATUS_NONFINITE 2      // a NaN or Inf in a stress or force
 #define NSM_STATUS_TIMEOUT 8        // a bounded wait on the tensor cores ran out
+#define NSM_STATUS_COPY_TIMEOUT 16  // a bounded wait on a copy to shared memory ran out
 
 struct nsm_model;  // the handle of include/nimble_gb300.h
 

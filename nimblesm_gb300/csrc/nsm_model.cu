@@ -231,6 +231,7 @@ int read_status(nsm_model* m)
   if (status & NSM_STATUS_BAD_JACOBIAN) return fail(NSM_ERR_BAD_JACOBIAN, "non-positive Jacobian (inverted element)");
   if (status & NSM_STATUS_NONFINITE) return fail(NSM_ERR_NONFINITE, "non-finite element force");
   if (status & NSM_STATUS_TIMEOUT) return fail(NSM_ERR_STATE, "a bounded tensor-core wait ran out (learned closure)");
+  if (status & NSM_STATUS_COPY_TIMEOUT) return fail(NSM_ERR_STATE, "a bounded wait for the element geometry ran out");
   return NSM_OK;
 }
 

@@ -175,6 +175,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t phase, uint64
     if (global_ns() - t0 > limit_ns) return false;
   }
 }
+// The same by a whole warp (all lanes call it): true when every lane saw the
+// phase complete.  Near the limit the lanes can see different things, and a warp
+// must not go on with part of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* mbar, uint32_t phase, uint64_t limit_ns = 1000000000ull)
+{
+  const bool ok = mbar_wait(mbar, phase, limit_ns);
+  return __all_sync(0xffffffffu, ok);
+}
 
 }  // namespace tc
 }  // namespace nsm

@@ -93,7 +93,44 @@ __global__ void __launch_bounds__(128) k_tc_wait_timeout(long limit_us, int* __r
   if (warp == 0) tmem_dealloc(tmem_slot, 32);
 }
 
+// A warp's wait whose lanes see different things: half of them give up after
+// `limit_us`, the others see the phase complete at five times that.
+__global__ void __launch_bounds__(64) k_warp_wait(long limit_us, int* __restrict__ lanes_on)
+{
+  __shared__ uint64_t mbar;
+  const int           lane = threadIdx.x & 31;
+  const uint64_t      ns = 1000ull * (uint64_t)limit_us, t0 = global_ns();
+  if (threadIdx.x == 0) {
+    mbar_init(&mbar, 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    if (mbar_wait_warp(&mbar, 0, lane < 16 ? ns : 20 * ns)) atomicAdd(lanes_on, 1);
+  } else if (lane == 0) {
+    while (global_ns() - t0 < 5 * ns) __nanosleep(1000);
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&mbar)) : "memory");
+  }
+}
+
 }  // namespace
+
+extern "C" int nsm_warp_wait_selftest(long limit_us, int* lanes_on)
+{
+  if (!lanes_on || limit_us < 1 || limit_us > 10000) return NSM_ERR_INVALID_ARGUMENT;
+  int* dS = nullptr;
+  int  rc = NSM_OK, lanes = -1;
+  if (cudaMalloc(&dS, sizeof(int)) != cudaSuccess || cudaMemset(dS, 0, sizeof(int)) != cudaSuccess) rc = NSM_ERR_CUDA;
+  if (rc == NSM_OK) {
+    k_warp_wait<<<1, 64>>>(limit_us, dS);
+    if (cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemcpy(&lanes, dS, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = NSM_ERR_CUDA;
+  }
+  cudaFree(dS);
+  *lanes_on = lanes;
+  return rc;
+}
 
 extern "C" int nsm_tc_wait_timeout_selftest(long limit_us, int* timed_out)
 {

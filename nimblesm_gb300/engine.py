@@ -128,6 +128,7 @@ SIGNATURES = {
     "nsm_closure_fallbacks": (C.c_int, [_vp, C.POINTER(C.c_ulonglong)]),
     "nsm_tc_selftest": (C.c_int, [C.c_int, C.c_int, _dp_f, _dp_f, _dp_f]),
     "nsm_tc_wait_timeout_selftest": (C.c_int, [C.c_long, C.POINTER(C.c_int)]),
+    "nsm_warp_wait_selftest": (C.c_int, [C.c_long, C.POINTER(C.c_int)]),
     "nsm_device_sm_count": (C.c_int, [C.c_int, C.POINTER(C.c_int)]),
     "nsm_host_loop_steps": (C.c_int, [_vp, C.c_int, _dp, C.c_double, C.c_int, C.c_int, C.c_int, _dp,
                                       C.POINTER(_HostBcs), _dp, _dp, _dp, _dp, _dp]),
