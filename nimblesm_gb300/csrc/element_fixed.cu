@@ -179,13 +179,73 @@ __device__ __forceinline__ void load_g0(const i64* gp, Limbs g0[3][3])
   }
 }
 
+// Whether each of a warp's elements has a lane that reports it.
+template <int kElems>
+__device__ __forceinline__ bool none_inside(unsigned bad)
+{
+  unsigned b = __ballot_sync(0xffffffffu, bad != 0);
+  if (kElems == 4) b |= b >> 4;
+  b |= b >> 8;
+  b |= b >> 16;
+  return (~b & ((1u << kElems) - 1)) == 0;
+}
+
+// The block's elements that are left to the FP64 code, collected in the staging
+// (`room` ints per warp) and evaluated 32 to a warp: the FP64 pipe takes a warp
+// instruction as long for 8 lanes as for 32.  A block's warps have neighbouring
+// groups, so a round of its loop is `span` consecutive elements.  The first
+// batch falls to another warp, another scheduler, in every quarter of the grid,
+// since a small mesh has one batch per block and four blocks on an SM.  A mesh
+// turned by 0.6 takes 57 to 63 us a step up to 8,000 elements, 85 at 21,952, 756
+// at 262,144 and 5,690 at 2,097,152 (by one lane per element, 8 to a warp, 58 to
+// 154, 255, 2,770 and 21,730 us; without the fixed-point code, every element in
+// FP64, 58 to 64, 104, 697 and 5,260): the pipe 85% busy, after 0.35 ms in which
+// the fixed-point code finds them outside.  A quarter of 2,097,152 elements beyond
+// the domain: 2.4 ms.  (Evaluated between rounds, beside other blocks' fixed-point
+// work: 5.6 ms, but 9% more for meshes inside the domain, whose loop loses the
+// registers of the call.)
+template <int kElems>
+__device__ __noinline__ void left_to_fp64(const ElementArgs& a, int* queue, int room)
+{
+  const int  lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, span = warps * kElems;
+  const int  rounds = (warps * room - 1) / span;  // that the queue holds; queue[0]: its length
+  const long step   = (long)gridDim.x * span;
+  for (long e0 = (long)(a.e_begin / kElems) * kElems + (long)blockIdx.x * span; e0 < a.E; e0 += rounds * step) {
+    __syncthreads();
+    if (threadIdx.x == 0) queue[0] = 0;
+    __syncthreads();
+    for (int r = warp; r < rounds && e0 + r * step < a.E; r += warps) {
+      const long     e    = e0 + r * step + lane;
+      const bool     left = lane < span && e >= a.e_begin && e < a.E && a.elem_left[e];
+      const unsigned m    = __ballot_sync(0xffffffffu, left);
+      if (m == 0) continue;
+      int at = lane == 0 ? atomicAdd(queue, __popc(m)) : 0;
+      at     = __shfl_sync(0xffffffffu, at, 0);
+      if (left) queue[1 + at + __popc(m & ((1u << lane) - 1))] = (int)e;
+    }
+    __syncthreads();
+    const int n = queue[0], turn = (int)(4u * blockIdx.x / gridDim.x);
+    __syncthreads();
+    if (threadIdx.x == 0) queue[0] = warps;  // the next batch that no warp has
+    __syncthreads();
+    for (int b = (warp + turn) % warps; b * 32 < n;) {
+      if (b * 32 + lane < n) fallback_fp64(a, queue[1 + b * 32 + lane]);
+      __syncwarp();
+      if (lane == 0) b = atomicAdd(queue, 1);
+      b = __shfl_sync(0xffffffffu, b, 0);
+    }
+  }
+}
+
 // kStore: F and sigma are formed and stored when the launch asks for it.
 // kHasElastic: some material of the model is elastic.
 // kPoints: points per lane.  1 (small meshes; without records): two lanes share
 // what a lane does otherwise, each with one of the two points; the transforms
 // before and after are done by both.
+template <bool kStore, bool kHasElastic>
+constexpr int kBlocks = kStore || kHasElastic ? 3 : 4;  // per SM
 template <bool kStore, bool kHasElastic, int kPoints>
-__global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementArgs a)
+__global__ void __launch_bounds__(128, kBlocks<kStore, kHasElastic>) k_element_fixed(ElementArgs a)
 {
   static_assert(kPoints == 2 || (kPoints == 1 && !kStore), "points per lane");
   constexpr int  kElems = 4 * kPoints;  // of a warp, half a geometry block or a whole one
@@ -205,8 +265,6 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
   // groups of kElems elements; those at the ends of [e_begin, E) may be partial
   const long g_end = (a.E + kElems - 1) / kElems, g_step = (long)gridDim.x * (blockDim.x >> 5);
   long       g     = a.e_begin / kElems + (long)blockIdx.x * (blockDim.x >> 5) + warp;
-  const long first = g;
-  if (g >= g_end) return;
   auto load_ids = [&](long gr, int id[2]) {
     const long e = min(gr * kElems + j, (long)a.E - 1);  // (spare lanes repeat the last element)
     id[0]        = __ldg(&conn[e]);
@@ -228,15 +286,18 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
   }
   __syncwarp();
   int id[2];
-  load_ids(g, id);
-  stage_geo(0, g);
+  if (g < g_end) {
+    load_ids(g, id);
+    stage_geo(0, g);
+  }
   wait_prerequisites();  // the node kernel that writes u
   launch_dependents();
-  stage_u(0, id);
+  if (g < g_end) stage_u(0, id);
   cp_async_commit();
   if (g + g_step < g_end) load_ids(g + g_step, id);
 
   unsigned any_bad = 0;
+  bool     gave_up = false;
   uint32_t phase = 0;  // bit b: parity of block b's next copy
   for (int buf = 0; g < g_end; g += g_step, buf ^= 1) {
     cp_async_wait_all();
@@ -245,7 +306,8 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       // land in another block's memory; nothing else of this warp is in flight.
       tc::mbar_wait_warp(&bar[buf], (phase >> buf) & 1u);
       if (lane == 0) atomicOr(a.status, NSM_STATUS_COPY_TIMEOUT);
-      return;
+      gave_up = true;
+      break;
     }
     phase ^= 1u << buf;
     if (g + g_step < g_end) {
@@ -351,12 +413,15 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     i64              Q[3][3];
     const fx::Moduli mod{mat.half_k, mat.shear, mat.lambda, mat.exponent, mat.model};
     i64*             gp = gs + side * kGeoPoint * 32;
+    // All of the warp's elements outside by their modes already: only that is left
+    // to say.  (From the second round on: small meshes wait for the vote.)
+    const bool none = kPoints == 2 && g >= a.e_begin / kElems + g_step && none_inside<kElems>(bad);
     if (side) {
 #pragma unroll
       for (int i = 0; i < 3; i++) G[i].y += G[i].y1, G[i].z += G[i].z1;
     }
 #pragma unroll 1
-    for (int sx = 0; sx < kPoints; sx++, gp += kGeoPoint * 32) {
+    for (int sx = 0; sx < (none ? 0 : kPoints); sx++, gp += kGeoPoint * 32) {
       i64 P[3][3];
       {
         Limbs g0[3][3];
@@ -366,8 +431,8 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
         for (int i = 0; i < 3; i++) Du[i][0] = G[i].x, Du[i][1] = G[i].y, Du[i][2] = G[i].z;
         const i64 det = gp[9 * 32];
         fx::Point pt;
+        i64       He[3][3];
         if (kHasElastic && elastic) {
-          i64       He[3][3];
           const int up = max(-ee, 0), down = min(max(ee, 0), 63);
           fx::displacement_gradient<true>(Du, g0, He);
 #pragma unroll
@@ -375,13 +440,12 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
             pt.H[q / 3][q % 3] = (i64)((u64)He[q / 3][q % 3] << up) >> down;
             bad |= fx::outside<27>(pt.H[q / 3][q % 3]);  // (|H|^2 below would not show it)
           }
-          bad |= fx::kinematics(pt);
-          bad |= fx::elastic_force<kStore>(mod, det, He, pt, P);
         } else {
           fx::displacement_gradient(Du, g0, pt.H);
-          bad |= fx::kinematics(pt);
-          fx::neohookean_force<kStore>(mod, det, pt, P);
         }
+        bad |= fx::kinematics(pt);
+        if (kHasElastic && elastic) bad |= fx::elastic_force<kStore>(mod, det, He, pt, P);
+        else bad |= fx::neohookean_force<kStore>(mod, det, pt, P);
         if (store) {
           double       r[kIpRecord];
 #pragma unroll
@@ -413,42 +477,46 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
       }
     }
 
-    // ---- nodal forces of the lane's corners ----
-    ef += mat.exponent - ee - (elastic ? fx::kElasticForce - fx::kElasticSum : 0);
-    const double scale = __longlong_as_double((i64)(1023 + ef) << 52);
-    double       f[2][3];
-    if (kPoints == 1) {  // both lanes' forces
-      __syncwarp();
+    if (none) {
+      bad = 1;
+    } else {
+      // ---- nodal forces of the lane's corners ----
+      ef += mat.exponent - ee - (elastic ? fx::kElasticForce - fx::kElasticSum : 0);
+      const double scale = __longlong_as_double((i64)(1023 + ef) << 52);
+      double       f[2][3];
+      if (kPoints == 1) {  // both lanes' forces
+        __syncwarp();
 #pragma unroll
-      for (int q = 0; q < 9; q++) Q[q / 3][q % 3] = gs[(kGeoPoint + q) * 32];
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      const i64      qx = gs[i * 32], qy = gs[(3 + i) * 32], qz = gs[(6 + i) * 32];
-      fx::Sums       S{Q[0][i] + qx, Q[1][i] + qy, Q[1][i] - qy, Q[2][i] + qz, Q[2][i] - qz};
-      fx::Parts      keep, send;
-      if (elastic) {
-        fx::common_scale(S, rows);
-        bad |= fx::too_large(S);
+        for (int q = 0; q < 9; q++) Q[q / 3][q % 3] = gs[(kGeoPoint + q) * 32];
       }
-      fx::lane_adjoint(S, keep, send);
-      const i64 e0 = keep.e0 + other<kAcrossZeta>(send.e0), e1 = keep.e1 + other<kAcrossZeta>(send.e1);
-      const i64 o0 = keep.o0 + other<kAcrossZeta>(send.o0), o1 = keep.o1 + other<kAcrossZeta>(send.o1);
-      const i64 ev = (e0 + e1) + other<kAcrossEta>(e0 - e1), od = (o0 + o1) + other<kAcrossEta>(o0 - o1);
-      f[0][i] = (double)(od - ev) * scale;
-      f[1][i] = (double)(-od - ev) * scale;
-    }
-    if (kPoints == 1) bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossXi);
-    bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossEta);
-    bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossZeta);
-    if (bad == 0 && valid) {
-      double* const fe = reinterpret_cast<double*>(a.fe) + e;
 #pragma unroll
-      for (int bx = 0; bx < 2; bx++)
-        if (kPoints == 2 || bx == side) {
-#pragma unroll
-          for (int i = 0; i < 3; i++) fe[(size_t)(3 * (corner_of(bx, y, 0) + 4 * z) + i) * ld_e] = f[bx][i];
+      for (int i = 0; i < 3; i++) {
+        const i64      qx = gs[i * 32], qy = gs[(3 + i) * 32], qz = gs[(6 + i) * 32];
+        fx::Sums       S{Q[0][i] + qx, Q[1][i] + qy, Q[1][i] - qy, Q[2][i] + qz, Q[2][i] - qz};
+        fx::Parts      keep, send;
+        if (elastic) {
+          fx::common_scale(S, rows);
+          bad |= fx::too_large(S);
         }
+        fx::lane_adjoint(S, keep, send);
+        const i64 e0 = keep.e0 + other<kAcrossZeta>(send.e0), e1 = keep.e1 + other<kAcrossZeta>(send.e1);
+        const i64 o0 = keep.o0 + other<kAcrossZeta>(send.o0), o1 = keep.o1 + other<kAcrossZeta>(send.o1);
+        const i64 ev = (e0 + e1) + other<kAcrossEta>(e0 - e1), od = (o0 + o1) + other<kAcrossEta>(o0 - o1);
+        f[0][i] = (double)(od - ev) * scale;
+        f[1][i] = (double)(-od - ev) * scale;
+      }
+      if (kPoints == 1) bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossXi);
+      bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossEta);
+      bad |= __shfl_xor_sync(0xffffffffu, bad, kAcrossZeta);
+      if (bad == 0 && valid) {
+        double* const fe = reinterpret_cast<double*>(a.fe) + e;
+#pragma unroll
+        for (int bx = 0; bx < 2; bx++)
+          if (kPoints == 2 || bx == side) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) fe[(size_t)(3 * (corner_of(bx, y, 0) + 4 * z) + i) * ld_e] = f[bx][i];
+          }
+      }
     }
     // which elements are left to the FP64 code
     any_bad |= bad;
@@ -457,15 +525,14 @@ __global__ void __launch_bounds__(128, kStore ? 3 : 4) k_element_fixed(ElementAr
     __syncwarp();             // this group's staged data are read, its records written
   }
   // (after the loop: a call inside it would spill the loop's state)
-  if (__any_sync(0xffffffffu, any_bad != 0) && y == 0 && z == 0 && side == 0)
-    for (g = first; g < g_end; g += g_step) {
-      const long e = g * kElems + j;
-      if (e >= a.e_begin && e < a.E && a.elem_left[e]) fallback_fp64(a, (int)e);
-    }
+  if (!__syncthreads_or(any_bad != 0)) return;
+  if (__syncthreads_or(gave_up)) return;  // a late copy may still change the staging
+  left_to_fp64<kElems>(a, reinterpret_cast<int*>(stage_all), (kStore ? kStageBytesStore : kStageBytes) / 4);
 }
 
-// Blocks of 128 threads, four warps, four blocks per SM (three where records
-// are stored): 16 warps of 128 registers and 14 KB of staging.
+// Blocks of 128 threads, four warps, four blocks per SM: 16 warps of 128
+// registers and 14 KB of staging.  Three where records are stored or elastic
+// elements would spill: 64,000 of them 53.9 us a step, 58.6 with four.
 template <bool kStore, bool kHasElastic, int kPoints>
 static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
@@ -482,8 +549,12 @@ static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cu
   const int  warps  = l.block == 64 ? 2 : 4;
   constexpr int kElems = 4 * kPoints;
   const long groups = (a.E + kElems - 1L) / kElems - a.e_begin / kElems;
-  const int  per_sm = l.persistent ? l.blocks_per_sm : (kStore ? 3 : 4) * (4 / warps);
-  const long grid   = std::min<long>((groups + warps - 1) / warps, (long)per_sm * num_sms());
+  const int  per_sm = l.persistent ? l.blocks_per_sm : kBlocks<kStore, kHasElastic> * (4 / warps);
+  const long blocks = (groups + warps - 1) / warps, fit = (long)per_sm * num_sms();
+  // One block fewer past eight rounds: its 32 elements a round are then a stretch
+  // of the mesh elsewhere in each (608 blocks of 32 come back to the same quarter
+  // of a row of 128), and elements outside the domain are spread over all blocks.
+  const long grid   = blocks <= 8 * fit ? std::min(blocks, fit) : std::max(1L, fit - 1);
   return launch_overlapped(k_element_fixed<kStore, kHasElastic, kPoints>, (int)grid, 32 * warps, warps * bytes, stream, a.overlap != 0, a);
 }
 

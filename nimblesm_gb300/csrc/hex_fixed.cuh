@@ -27,10 +27,12 @@
 // here.  An FP64 evaluation of an elastic element has no such absolute error;
 // how its bits are kept here is said at elastic_scale.
 //
-// Domain.  |H| < 1/8 (Frobenius) at every point, neo-Hookean displacements
-// within 2^26 of the element's scale, finite inputs.  The functions report what
-// leaves it; the caller then evaluates the element in FP64 as a whole, so each
-// element's result depends on its own inputs alone.
+// Domain.  |H| < 1/2 (Frobenius; a rotation by 20 degrees) at every point; for
+// neo-Hookean elements also displacement modes below 1.375 2^60, which end at
+// |H| between 0.1 and 0.3, stresses below the larger modulus past |H| = 1/8, and
+// displacements within 2^26 of the element's scale; finite inputs.  The functions
+// report what leaves it; the caller then evaluates the element in FP64 as a
+// whole, so each element's result depends on its own inputs alone.
 //
 // One element is shared by four lanes, each with one edge along xi: the two
 // points and two corners on its side along eta and zeta.  A lane works in
@@ -181,11 +183,12 @@ NSM_HD void lane_modes(const i64 q[2][2], const i64 o[2][2], i64 v[7])
 }
 
 // Shift from the displacements' scale to the element's (0 <= sh <= 26): the
-// modes stay below 2^60.
+// modes stay below 1.375 2^60, the gradients below 2^61.8, and |H|^2, of at most
+// nine squares of 1.29, in 64 bits.
 NSM_HD unsigned lane_shift(i64 v[7], int sh)
 {
   unsigned  bad = 0;
-  const int lim = 1 << (28 - sh);
+  const int lim = (11 << 25) >> sh;
 #pragma unroll
   for (int k = 0; k < 7; k++) {
     bad |= (unsigned)((int)(v[k] >> 32) + lim) >= 2u * (unsigned)lim;
@@ -250,7 +253,10 @@ NSM_HD void displacement_gradient(const i64 Du[3][3], const Limbs G0[3][3], i64 
   }
 }
 
-// From H: |H|^2, the cofactors of F = I + H and t = J - 1.  Reports |H| >= 1/8.
+// From H: |H|^2, the cofactors of F = I + H and t = J - 1.  Reports |H| >= 1/2:
+// up to there the high limbs of H at 2^62, of the cofactors and of F at 2^60 are
+// below 2^29.3, and the sums of mixed products keep within 63 bits.  (|H|^2 is
+// right to 2^33 for any H that Du G0 can give, entries below 1.29.)
 NSM_HD unsigned kinematics(Point& p)
 {
   u64 sq = 0, mid = 0;
@@ -279,7 +285,7 @@ NSM_HD unsigned kinematics(Point& p)
   s.add(p.h[0][1], split(p.C[0][1]));
   s.add(p.h[0][2], split(p.C[0][2]));
   p.t = (p.C[0][0] - kOne) + s.value();
-  return (unsigned)((u64)p.n2 >> 54 != 0);
+  return (unsigned)((u64)p.n2 >> 58 != 0);
 }
 
 // J^(-5/3) and 1/J at 2^60 from t = J - 1.  y, J^(-1/3) to about 20 bits, is
@@ -400,9 +406,10 @@ NSM_HD void elastic_gradient(const i64 v[7], const Rows& r, Gradient& G)
 // q0 = K/2 (J - 1/J) - g tr(b - I) / 3, and adj(F) b = J F^T, so
 // adj(F) sigma = g J F^T + (q0 - g) adj(F): the stress itself is formed only
 // where it is stored.  With |H| < 1/8 and moduli of at most 1/8, |P| < 2^58.4
-// and the forces stay below 2^62.2.
+// and the forces stay below 2^62.2.  Up to |H| = 1/2 (J in [0.35, 2.2], J^(-5/3)
+// below 5.8, |P| < 2^62.5) that is checked, and larger P reported.
 template <bool kStress>
-NSM_HD void neohookean_force(const Moduli& m, i64 det, Point& p, i64 P[3][3])
+NSM_HD unsigned neohookean_force(const Moduli& m, i64 det, Point& p, i64 P[3][3])
 {
   const Limbs d  = split(det);
   const i64   tr = p.H[0][0] + p.H[1][1] + p.H[2][2];
@@ -436,6 +443,12 @@ NSM_HD void neohookean_force(const Moduli& m, i64 det, Point& p, i64 P[3][3])
       s.add(bd, split(p.C[i][J]));
       P[J][i] = s.value();
     }
+  unsigned bad = 0;
+  if ((p.n2 >> 54) != 0) {
+#pragma unroll
+    for (int q = 0; q < 9; q++) bad |= outside<26>(P[q / 3][q % 3]);
+  }
+  return bad;
 }
 
 // The same for the elastic material, sigma = G (H + H^T) + lambda tr(H) I, with

@@ -233,7 +233,7 @@ bool fixed_point(const Element& el, int model, double K, double G, double f[8][3
       }
       bad |= kinematics(pt);
       if (elastic) bad |= elastic_force<true>(m, det, He, pt, P);
-      else neohookean_force<true>(m, det, pt, P);
+      else bad |= neohookean_force<true>(m, det, pt, P);
       for (int k = 0; k < 6; k++) sig[p][k] = std::ldexp((double)pt.sig[k], EM - 62 - e);
       point_force(g0, P, Q);
       for (int i = 0; i < 3; i++) {
@@ -309,12 +309,17 @@ int main(int argc, char** argv)
   for (double s : {1e-12, 1e-9, 1e-6, 1e-4, 1e-2, 3e-2, 5e-2}) add("strain").strain = s;
   for (double s : {1e-240, 1e-100, 1e-30, 1e-20, 1e-15}) add("tiny_strain").strain = s;
   for (double s : {1e-270, 5e-322}) add("below_the_scales").strain = s;
-  for (double a : {0.01, 0.03, 0.05}) add("turned").rotation = a;
+  for (double s : {0.08, 0.12, 0.2, 0.3}) add("large_strain").strain = s;
+  for (double a : {0.01, 0.03, 0.05, 0.1, 0.2, 0.34}) add("turned").rotation = a;
+  for (double a : {0.1, 0.3}) {
+    Kind& k    = add("turned_and_strained");
+    k.rotation = a, k.strain = 0.03;
+  }
   for (double a : {1.0, 3.0}) {
     Kind& k    = add("swelling");
     k.swelling = true, k.jitter = 0, k.thin[2] = a;
   }
-  add("turned_far").rotation = 0.3;
+  add("turned_far").rotation = 0.6;
   for (double t : {1e-2, 1.0, 1e3}) add("moved").rigid = t;
   for (double x : {inf, -inf, nan, 1e307})
     for (bool c : {false, true}) {
