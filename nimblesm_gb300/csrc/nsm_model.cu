@@ -148,7 +148,7 @@ struct nsm_model {
   double                 t0 = 0;
   StepSched*             d_sched = nullptr;
 
-  std::map<int, cudaGraphExec_t> graphs;
+  std::map<std::pair<int, bool>, cudaGraphExec_t> graphs;  // by steps, and whether one may be an output step
 
   // Host-buffer pipeline (nsm_compute_internal_force_host): K element chunks,
   // the copy of u in by node ranges ahead of them and the copy of f_int out
@@ -329,8 +329,9 @@ double* field_ptr(nsm_model* m, int field)
 }
 
 // k: schedule offset of the step, or -1 outside the loop; `last`: nothing is
-// launched after this step that overwrites its records.
-nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
+// launched after this step that overwrites its records; `outputs`: some step of
+// the sequence is an output step.
+nsm::ElementArgs element_args(nsm_model* m, int k, bool last, bool outputs = true)
 {
   nsm::ElementArgs a{};
   a.E         = m->E;
@@ -357,8 +358,9 @@ nsm::ElementArgs element_args(nsm_model* m, int k, bool last)
   a.mats       = m->d_mats;
   a.num_groups = m->S;
   a.persistent = 0;
-  a.store_ip  = k < 0 ? nsm::kStoreAlways
-                      : (!m->store_ip ? nsm::kStoreOutput : (last ? nsm::kStoreAlways : nsm::kStoreNever));
+  if (k < 0) a.store_ip = nsm::kStoreAlways;
+  else if (m->store_ip) a.store_ip = last ? nsm::kStoreAlways : nsm::kStoreNever;
+  else a.store_ip = outputs ? nsm::kStoreOutput : nsm::kStoreNever;
   a.sched     = k < 0 ? nullptr : m->d_sched;
   a.step_base = m->d_step_base;
   a.k         = k;
@@ -487,10 +489,10 @@ cudaError_t element_split(nsm_model* m, int k)
   return e;
 }
 
-cudaError_t launch_element(nsm_model* m, int k, bool last)
+cudaError_t launch_element(nsm_model* m, int k, bool last, bool outputs = true)
 {
   if (has_callbacks(m)) return element_split(m, k);
-  nsm::ElementArgs a = element_args(m, k, last);
+  nsm::ElementArgs a = element_args(m, k, last, outputs);
   if (m->closure) {
     nsm::mlp::MlpElementArgs ma;
     nsm::mlp::element_args(m->closure, &ma, nullptr, nullptr);
@@ -530,7 +532,7 @@ cudaError_t node_step(nsm_model* m, int k_post, int k_pre, int K)
 
 // Launch sequence of a chunk of K schedule steps starting at the device base:
 // node(pre 0); {element(k); node(post k, pre k+1)}; node(post K-1); base += K.
-cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
+cudaError_t enqueue_chunk(nsm_model* m, int K, bool outputs, bool timed)
 {
   cudaError_t e;
   if ((e = node_step(m, -1, 0, K)) != cudaSuccess) return e;
@@ -538,30 +540,41 @@ cudaError_t enqueue_chunk(nsm_model* m, int K, bool timed)
     if (timed) {
       auto ev = next_events(m->ev_elem, m->ev_elem_used);
       cudaEventRecord(ev.first, m->stream);
-      if ((e = launch_element(m, k, k + 1 == K)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, k + 1 == K, outputs)) != cudaSuccess) return e;
       cudaEventRecord(ev.second, m->stream);
       auto en = next_events(m->ev_node, m->ev_node_used);
       cudaEventRecord(en.first, m->stream);
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1, K)) != cudaSuccess) return e;
       cudaEventRecord(en.second, m->stream);
     } else {
-      if ((e = launch_element(m, k, k + 1 == K)) != cudaSuccess) return e;
+      if ((e = launch_element(m, k, k + 1 == K, outputs)) != cudaSuccess) return e;
       if ((e = node_step(m, k, k + 1 < K ? k + 1 : -1, K)) != cudaSuccess) return e;
     }
   }
   return nsm::launch_advance_base(m->d_step_base, K, m->stream);
 }
 
-int get_graph(nsm_model* m, int K, cudaGraphExec_t* out)
+// Whether one of the next K steps is an output step: a model that stores the
+// point records of those alone (store_ip_data = 0) launches the kernels that
+// store none where there is none (64^3 elements, FP64: 190 -> 168 us a step).
+bool outputs_ahead(const nsm_model* m, int K)
 {
-  auto it = m->graphs.find(K);
+  for (int s = m->steps_done; s < m->steps_done + K; s++)
+    if (m->h_sched[(size_t)s * m->S].is_output) return true;
+  return false;
+}
+
+int get_graph(nsm_model* m, int K, bool outputs, cudaGraphExec_t* out)
+{
+  const auto key = std::make_pair(K, outputs || m->store_ip);  // (records by the sequence's end: one graph for both)
+  auto       it  = m->graphs.find(key);
   if (it != m->graphs.end()) {
     *out = it->second;
     return NSM_OK;
   }
   cudaGraph_t graph;
   NSM_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e  = enqueue_chunk(m, K, false);
+  cudaError_t e  = enqueue_chunk(m, K, outputs, false);
   cudaError_t e2 = cudaStreamEndCapture(m->stream, &graph);
   if (e != cudaSuccess) return cuda_fail(e, "capture");
   if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture");
@@ -569,8 +582,8 @@ int get_graph(nsm_model* m, int K, cudaGraphExec_t* out)
   e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-  m->graphs[K] = exec;
-  *out         = exec;
+  m->graphs[key] = exec;
+  *out           = exec;
   return NSM_OK;
 }
 
@@ -1573,7 +1586,7 @@ int nsm_advance(nsm_model* m, int num_steps)
   if (has_callbacks(m)) {  // one step at a time without graphs: each callback sees its step's times
     for (; num_steps > 0; num_steps--) {
       m->cb_failed  = false;
-      cudaError_t e = enqueue_chunk(m, 1, m->profiling);
+      cudaError_t e = enqueue_chunk(m, 1, true, m->profiling);
       if (m->cb_failed) return fail(NSM_ERR_STATE, "a block-material callback failed");
       NSM_CUDA(e);
       m->steps_done += 1;
@@ -1583,10 +1596,10 @@ int nsm_advance(nsm_model* m, int num_steps)
   while (num_steps > 0) {
     int K = num_steps < m->graph_steps ? num_steps : m->graph_steps;
     if (m->profiling) {
-      NSM_CUDA(enqueue_chunk(m, K, true));
+      NSM_CUDA(enqueue_chunk(m, K, outputs_ahead(m, K), true));
     } else {
       cudaGraphExec_t exec;
-      int             r = get_graph(m, K, &exec);
+      int             r = get_graph(m, K, outputs_ahead(m, K), &exec);
       if (r) return r;
       NSM_CUDA(cudaGraphLaunch(exec, m->stream));
     }
