@@ -41,8 +41,10 @@ int cuda_fail(cudaError_t e, const char* where)
     if (_e != cudaSuccess) return cuda_fail(_e, #call);   \
   } while (0)
 
-// Largest half of a model's table of expression values.
-constexpr size_t kBcExprBytes = 8 << 20;
+// Largest half of a model's table of expression values, in bytes and in rows (a
+// row of the grid each, of which there are at most 65,535; the latency of a
+// launch is spread over enough steps long before).
+constexpr size_t kBcExprBytes = 8 << 20, kBcExprRows = 4096;
 
 long pad(long n, long q) { return (n + q - 1) / q * q; }
 
@@ -288,7 +290,7 @@ int upload_bcs(nsm_model* m)
         NSM_CUDA(cudaMemcpyAsync(m->d_bc_slot_node, slot_node.data(), sizeof(int) * slot_node.size(),
                                  cudaMemcpyHostToDevice, m->stream));
         const size_t row = sizeof(double) * 3 * slot_node.size();
-        m->bc_expr_rows  = (int)std::min<size_t>(m->graph_steps, std::max<size_t>(1, kBcExprBytes / row));
+        m->bc_expr_rows  = (int)std::min<size_t>({(size_t)m->graph_steps, std::max<size_t>(1, kBcExprBytes / row), kBcExprRows});
         NSM_CUDA(cudaMalloc(&m->d_bc_expr_val, row * 2 * m->bc_expr_rows));
         NSM_CUDA(cudaMemsetAsync(m->d_bc_expr_val, 0, row * 2 * m->bc_expr_rows, m->stream));
       }
