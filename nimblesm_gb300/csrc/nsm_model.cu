@@ -204,6 +204,17 @@ void free_all(nsm_model* m)
   cudaFreeHost(m->h_status);
 }
 
+// Whether p is host memory that CUDA does not know (pageable).
+bool is_pageable(const void* p)
+{
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
 // A result to the caller's memory.  Where a page of it has not been touched yet
 // (a new array), the device's write would wait for the page by itself: 0.4 to
 // 1.7 ms for 0.8 MB on a heap that grows and shrinks, 38 us into pages that are
@@ -211,16 +222,16 @@ void free_all(nsm_model* m)
 // and writing that back would fault twice: 10 times as long).  Only pageable
 // memory: pinned pages are there, and what is not the host's is the copy's to
 // refuse.
+void touch_pages(void* dst, size_t bytes)
+{
+  static const size_t  page = (size_t)sysconf(_SC_PAGESIZE);
+  volatile char* const p    = static_cast<volatile char*>(dst);
+  for (size_t o = 0; o < bytes; o += page) p[o] = 0;
+  if (bytes > 0) p[bytes - 1] = 0;
+}
 cudaError_t read_result(void* dst, const void* src, size_t bytes, cudaStream_t stream)
 {
-  static const size_t   page = (size_t)sysconf(_SC_PAGESIZE);
-  volatile char* const  p    = static_cast<volatile char*>(dst);
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
-  else if (at.type == cudaMemoryTypeUnregistered) {
-    for (size_t o = 0; o < bytes; o += page) p[o] = 0;
-    if (bytes > 0) p[bytes - 1] = 0;
-  }
+  if (is_pageable(dst)) touch_pages(dst, bytes);
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
 }
 
@@ -1256,6 +1267,9 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
   cudaStream_t s_in = m->hp_stream[0], s_out = m->hp_stream[3], s_planes = m->hp_stream[4];
   cudaStream_t s_el[2] = {m->hp_stream[1], m->hp_stream[2]};
   cudaEvent_t* ev      = m->hp_ev.data();  // ev[0] start; ev[1 + 4j + {0, ..., 3}] in, in planes, elements, gathered
+  // A copy to pageable memory holds the host until it is done: those come after
+  // all launches, and the pages of a new array are touched meanwhile.
+  const bool   late    = is_pageable(f_host);
   cudaError_t  err     = cudaEventRecord(ev[0], m->stream);  // earlier work on the state is done first
   if (err == cudaSuccess) err = cudaStreamWaitEvent(s_in, ev[0], 0);
   auto copy_in = [&](int j) -> cudaError_t {
@@ -1284,7 +1298,15 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
                                            : nsm::launch_element_fp32(a, m->elaunch, s);
     return e != cudaSuccess ? e : cudaEventRecord(ev[3 + 4 * j], s);
   };
-  auto nodes_out = [&](int j) -> cudaError_t {
+  auto copy_out = [&](int j) -> cudaError_t {
+    const int r0 = m->hp_ready[j], r1 = m->hp_ready[j + 1];
+    if (r1 <= r0) return cudaSuccess;
+    const cudaError_t e = cudaStreamWaitEvent(s_out, ev[4 + 4 * j], 0);
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(f_host + 3L * r0, m->d_stage_out + 3L * r0,
+                                              sizeof(double) * 3 * (size_t)(r1 - r0), cudaMemcpyDeviceToHost, s_out);
+  };
+  auto nodes = [&](int j) -> cudaError_t {
     // chunks 0..j done: the last one on each element stream
     cudaError_t e = cudaStreamWaitEvent(m->stream, ev[3 + 4 * j], 0);
     if (e == cudaSuccess && j > 0) e = cudaStreamWaitEvent(m->stream, ev[3 + 4 * (j - 1)], 0);
@@ -1295,18 +1317,19 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
     a.N             = r1;
     a.f_rows        = m->d_stage_out;
     e               = nsm::launch_node_update(a, m->stream);
-    if (e == cudaSuccess) e = cudaEventRecord(ev[4 + 4 * j], m->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s_out, ev[4 + 4 * j], 0);
-    return e != cudaSuccess ? e
-                            : cudaMemcpyAsync(f_host + 3L * r0, m->d_stage_out + 3L * r0,
-                                              sizeof(double) * 3 * (size_t)(r1 - r0), cudaMemcpyDeviceToHost, s_out);
+    return e != cudaSuccess ? e : cudaEventRecord(ev[4 + 4 * j], m->stream);
   };
   // chunk by chunk, two copies in ahead of a chunk's kernels
   for (int j = 0; j < 2 && j < K && err == cudaSuccess; j++) err = copy_in(j);
   for (int j = 0; j < K && err == cudaSuccess; j++) {
     if (j + 2 < K) err = copy_in(j + 2);
     if (err == cudaSuccess) err = elements(j);
-    if (err == cudaSuccess) err = nodes_out(j);
+    if (err == cudaSuccess) err = nodes(j);
+    if (err == cudaSuccess && !late) err = copy_out(j);
+  }
+  if (err == cudaSuccess && late) {
+    touch_pages(f_host, sizeof(double) * 3 * (size_t)m->N);
+    for (int j = 0; j < K && err == cudaSuccess; j++) err = copy_out(j);
   }
   if (err == cudaSuccess) err = cudaStreamSynchronize(s_out);
   return err;
@@ -1370,7 +1393,7 @@ int nsm_compute_internal_force_host(nsm_model* m, const double* displacement, do
   NSM_CUDA(launch_element(m, -1, true));
   NSM_CUDA(nsm::launch_node_update(node_args(m, -1, -1, 1), m->stream));
   NSM_CUDA(nsm::launch_node_soa_to_aos(m->N, m->ld_n, m->d_f, f_out ? f_out : m->d_stage, m->stream));
-  if (!f_out) NSM_CUDA(cudaMemcpyAsync(internal_force, m->d_stage, bytes, cudaMemcpyDeviceToHost, m->stream));
+  if (!f_out) NSM_CUDA(read_result(internal_force, m->d_stage, bytes, m->stream));
   return read_status(m);  // synchronizes
 }
 
