@@ -2,6 +2,7 @@
 // ModelData for one block, the explicit loop as captured CUDA graphs, and the
 // host-buffer entry points.  C++ host code; all arithmetic on the path runs
 // in the kernels (setup_kernels.cu, element_kernels.cu, node_kernels.cu).
+#include <cuda.h>
 #include <unistd.h>
 
 #include <cmath>
@@ -1337,21 +1338,43 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
 
 }  // namespace
 
+// Whether `bytes` at p lie within the one allocation or registration that p is
+// in, as the driver has it.  (The addresses of the first and last byte do not
+// show it: host and device address are the same number, also on both sides of a
+// stretch that is not pinned.)
+static bool in_one_range(const void* p, size_t bytes)
+{
+  using Attribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const Attribute attribute = [] {
+    void*                           fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<Attribute>(fn);
+  }();
+  const CUdeviceptr at = (CUdeviceptr)reinterpret_cast<uintptr_t>(p);
+  CUdeviceptr       first = 0;
+  size_t            size  = 0;
+  return attribute && attribute(&first, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
+         attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) == CUDA_SUCCESS && at >= first && at - first <= size &&
+         bytes <= size - (size_t)(at - first);
+}
+
 // The device's address of `bytes` at p when all of them are pinned host memory
 // of one allocation (or registration) that the device can address, else null.
 static double* pinned_view(const double* p, size_t bytes)
 {
   if ((reinterpret_cast<uintptr_t>(p) & (alignof(double) - 1)) != 0) return nullptr;
-  cudaPointerAttributes first{}, last{};
-  const char* const     end = reinterpret_cast<const char*>(p) + bytes - 1;
-  if (cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
-      (const char*)last.devicePointer - (const char*)first.devicePointer != (ptrdiff_t)(bytes - 1))
-    return nullptr;
-  return reinterpret_cast<double*>(first.devicePointer);
+  if (at.type != cudaMemoryTypeHost || !at.devicePointer || !in_one_range(at.devicePointer, bytes)) return nullptr;
+  return reinterpret_cast<double*>(at.devicePointer);
 }
 
 int nsm_set_host_chunks(nsm_model* m, int chunks)
