@@ -566,6 +566,7 @@ static cudaError_t launch_fixed(const ElementArgs& a, const ElementLaunch& l, cu
 cudaError_t launch_element_fp64(const ElementArgs& a, const ElementLaunch& l, cudaStream_t stream)
 {
   if (a.E <= a.e_begin) return cudaSuccess;
+  if (!a.geo_fixed) return launch_element_plain(a, stream);
   if (a.store_ip != kStoreNever)
     return a.has_elastic ? launch_fixed<true, true, 2>(a, l, stream) : launch_fixed<true, false, 2>(a, l, stream);
   if (a.E - a.e_begin <= 4 * 4 * num_sms())

@@ -1,9 +1,9 @@
 // Fused hex8 element kernel of the FP32-mixed form: gather -> deformation
 // gradient -> neo-Hookean or elastic Cauchy stress -> B^T sigma, one thread per
 // element; the two passes of models with block-material callbacks (FP32 and
-// FP64); energies and the layout conversions.  The FP64 form's fused kernel is
-// element_fixed.cu; the element math and the reasons for its form are in
-// hex_math.cuh.
+// FP64); the FP64 form without its fixed-point geometry; energies and the layout
+// conversions.  The FP64 form's fused kernel is element_fixed.cu; the element
+// math and the reasons for its form are in hex_math.cuh.
 #include <algorithm>
 
 #include "element_packed.cuh"
@@ -150,6 +150,12 @@ cudaError_t launch_element_pass(const ElementArgs& a, int is_float, int pass, cu
     else
       k_element<double, true, false, 1, 2><<<grid, 128, 0, stream>>>(a);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_element_plain(const ElementArgs& a, cudaStream_t stream)
+{
+  k_element<double, true, false, 3><<<grid_for(a.E - a.e_begin, 128), 128, 0, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -104,7 +104,7 @@ struct ElementArgs {
   const float4* uf;        // [ld_n] FP32 copy of u, {x, y, z, 0} (FP32 form)
   const float4* Xf;        // [ld_n] FP32 copy of X (FP32 form)
   const double* geo;       // [8 * kGeoPerPoint][ld_e] (FP64 form only)
-  const long long* geo_fixed;      // fixed-point geometry (FP64 form only; element_fixed.cu)
+  const long long* geo_fixed;      // fixed-point geometry (FP64 form only; element_fixed.cu), or null: all in FP64
   const struct FixedMaterial* fixed_mats;  // materials in fixed point
   int              has_elastic;    // one of them is elastic
   unsigned char*   elem_left;      // [ld_e] scratch: elements outside the fixed-point domain
@@ -139,6 +139,8 @@ cudaError_t launch_element_fp32(const ElementArgs& a, const ElementLaunch& l, cu
 // recorded sigma (one thread per element).
 cudaError_t launch_element_pass(const ElementArgs& a, int is_float, int pass, cudaStream_t stream);
 int         num_sms();
+// The FP64 form by the FP64 code alone, one thread per element.
+cudaError_t launch_element_plain(const ElementArgs& a, cudaStream_t stream);
 // The FP64 form's fixed-point geometry (words: 64-bit), from the geo planes.
 size_t      fixed_geometry_words(long ld_e);
 // (elem_group: material of each element, or null)

@@ -94,7 +94,7 @@ struct nsm_model {
   int*    d_step_base = nullptr;
   double* d_scratch = nullptr;  // energy partials / setup temporaries
   double* d_stage = nullptr;    // [3N] AoS staging for host copies
-  double* d_derived = nullptr;  // [16 E] derived element data, from its first use on
+  double* d_derived = nullptr;  // [16 E] derived element data, from its first use on (small meshes)
   double* d_out = nullptr;      // small results
   double* d_group_out = nullptr;// [S] per-sample results
   int*    d_elem_group = nullptr;  // [E] material of each element (more than one material)
@@ -656,6 +656,30 @@ bool force_records_pay(int N, int E, long ld_n, const std::vector<int>& slots, c
   return records < planes;
 }
 
+// The fixed-point geometry's memory, a quarter of an FP64 model's, where the
+// device has it and as much again as the calls on the model take for a time
+// (point records to the host 576 bytes an element; a chunked force call's staging).
+// A mesh that fits without it runs all the same, its elements in FP64 (5.08 ms
+// for 2,097,152 instead of 1.09).
+cudaError_t allocate_fixed(nsm_model* m)
+{
+  const size_t geometry = sizeof(long long) * nsm::fixed_geometry_words(m->ld_e), mats = sizeof(nsm::FixedMaterial) * m->num_mats;
+  const size_t later = (size_t)576 * m->E + (size_t)24 * m->N + (64u << 20);
+  size_t       free = 0, total = 0;
+  cudaError_t  e = cudaMemGetInfo(&free, &total);
+  if (e != cudaSuccess || free < geometry + m->ld_e + mats + later) return e;
+  e = cudaMalloc(&m->d_geo_fixed, geometry);
+  if (e == cudaSuccess) e = cudaMalloc(&m->d_elem_left, m->ld_e);
+  if (e == cudaSuccess) e = cudaMalloc(&m->d_fixed_mats, mats);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  for (void* p : {(void*)m->d_geo_fixed, (void*)m->d_elem_left, (void*)m->d_fixed_mats}) cudaFree(p);
+  m->d_geo_fixed  = nullptr;
+  m->d_elem_left  = nullptr;
+  m->d_fixed_mats = nullptr;
+  return cudaSuccess;
+}
+
 // One handle over S samples: the samples' meshes are concatenated (node and
 // element ids offset per sample) and each node carries its sample's time
 // schedule.  Materials: `num_mats` entries, element e uses
@@ -896,13 +920,11 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     std::vector<nsm::FixedMaterial> fixed_mats;
     if (e == cudaSuccess && m->precision == NSM_PRECISION_FP64) {
       for (const auto& b : gm) fixed_mats.push_back(nsm::fixed_material(b));
-      e = cudaMalloc(&m->d_geo_fixed, sizeof(long long) * nsm::fixed_geometry_words(m->ld_e));
-      if (e == cudaSuccess) e = cudaMalloc(&m->d_elem_left, m->ld_e);
-      if (e == cudaSuccess) e = cudaMalloc(&m->d_fixed_mats, sizeof(nsm::FixedMaterial) * num_mats);
-      if (e == cudaSuccess)
+      e = allocate_fixed(m);
+      if (e == cudaSuccess && m->d_geo_fixed)
         e = cudaMemcpyAsync(m->d_fixed_mats, fixed_mats.data(), sizeof(nsm::FixedMaterial) * num_mats,
                             cudaMemcpyHostToDevice, m->stream);
-      if (e == cudaSuccess)
+      if (e == cudaSuccess && m->d_geo_fixed)
         e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_elem_group, m->d_fixed_mats, m->d_geo_fixed, m->stream);
     }
     m->dt_group.assign(S, 1.7976931348623157e308);
@@ -1517,9 +1539,11 @@ int nsm_compute_derived_element_data(nsm_model* m, double* volume, double* stres
   if (m->E == 0) return NSM_OK;
   const int    is_float = m->precision == NSM_PRECISION_FP64 ? 0 : 1;
   const size_t E        = (size_t)m->E;
-  // (kept: allocating and freeing it took 146 of 410 us at 29,667 elements)
-  if (!m->d_derived) NSM_CUDA(cudaMalloc(&m->d_derived, sizeof(double) * 16 * E));
-  double* const tmp = m->d_derived;
+  // (kept up to 32 MB: allocating and freeing it took 146 of 410 us at 29,667 elements)
+  const bool keep = sizeof(double) * 16 * E <= (32u << 20);
+  double*    tmp  = m->d_derived;
+  if (!tmp) NSM_CUDA(cudaMalloc(&tmp, sizeof(double) * 16 * E));
+  if (keep) m->d_derived = tmp;
   cudaError_t   e   = nsm::launch_derived_element(m->E, m->ld_e, m->d_conn, m->d_X, m->d_u, m->ld_n, m->d_ip, is_float, tmp,
                                                   tmp + E, tmp + 7 * E, m->d_status, m->stream);
   if (e == cudaSuccess && volume) e = read_result(volume, tmp, sizeof(double) * E, m->stream);
@@ -1527,6 +1551,7 @@ int nsm_compute_derived_element_data(nsm_model* m, double* volume, double* stres
   if (e == cudaSuccess && deformation_gradient)
     e = read_result(deformation_gradient, tmp + 7 * E, sizeof(double) * 9 * E, m->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+  if (!keep) cudaFree(tmp);
   if (e != cudaSuccess) return cuda_fail(e, "nsm_compute_derived_element_data");
   return read_status(m);
 }
