@@ -3,10 +3,14 @@
 // An FP64 addition takes a warp 64 clocks of a quarter of an SM, an integer
 // instruction one or two.  Aligned to the largest of them, with the leading
 // bit of that at bit 59, eight numbers add up without overflow, each cut below
-// 2^-59 of the largest's power of two, and the sum is rounded once: closer to
-// the exact sum than FP64 additions in any order, which round at 2^-53 of every
-// partial sum.  About 14 integer instructions per number and one conversion in
-// place of seven additions.
+// 2^-59 of the largest's power of two, and the sum is rounded once: the error is
+// below 8 2^-59 of that power of two plus half a unit of the sum.  FP64 additions
+// round every partial sum at 2^-53 of it and are up to 80 times further off,
+// also where the large terms nearly cancel, as they do at a node near
+// equilibrium (tests/fixed_sum_bound_check.cc).  They are the closer ones where
+// large terms cancel exactly and before smaller ones are added: of 1, -1 and
+// 1e-3 they leave 1e-3, the fixed point 1e-3 (1 - 8.5e-16).  About 14 integer
+// instructions per number and one conversion in place of seven additions.
 #pragma once
 
 #include <cmath>

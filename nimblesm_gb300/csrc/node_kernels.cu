@@ -1,13 +1,14 @@
 // Node kernels: assembly of the element forces and the central-difference
 // update.
 //
-// FP64 form: every product and sum is an explicit round-to-nearest intrinsic
-// (__dmul_rn / __dadd_rn are never fused), so given the same element forces
-// the nodal state equals the reference's bit for bit.  FP32-mixed form: the
-// FP32 element forces are assembled in FP32 and the FP64 update uses fused
-// multiply-adds -- on this chip FP64 operations, not bytes, bound a node
-// update, and the exact rounding of the reference buys nothing when the forces
-// themselves are FP32.
+// FP64 form: a node's first eight element forces are one sum in fixed point
+// (fixed_sum.cuh), and every product and sum after that an explicit
+// round-to-nearest intrinsic (__dmul_rn / __dadd_rn are never fused), so given
+// the same assembled force the nodal state equals the reference's bit for bit.
+// FP32-mixed form: the FP32 element forces are assembled in FP32 and the FP64
+// update uses fused multiply-adds -- on this chip FP64 operations, not bytes,
+// bound a node update, and the exact rounding of the reference buys nothing when
+// the forces themselves are FP32.
 #include "fixed_sum.cuh"
 #include "nsm_kernels.cuh"
 
@@ -159,11 +160,11 @@ __device__ __forceinline__ void load_record(const NodeArgs& a, int at, int c0, f
   }
 }
 
-// The assembled element force of node n, components c0 ...: element
-// contributions in increasing element order, the first eight of the FP64 form
-// as one sum in fixed point (sum8; on the FP64 pipe their additions were half
-// of the launch's: 128^3 elements 183 -> 130 us, 15,625 nodes of 11 samples
-// 24.5 -> 22).
+// The assembled element force of node n, components c0 ...: in the FP64 form the
+// first eight contributions as one sum in fixed point, which has no order (sum8;
+// on the FP64 pipe their additions were half of the launch's: 128^3 elements
+// 183 -> 130 us, 15,625 nodes of 11 samples 24.5 -> 22), then, and in the FP32
+// form from the first, additions in increasing element order.
 template <typename TF, bool kExact, int kComps, bool kRecords>
 __device__ __forceinline__ void gather_force(const NodeArgs& a, int n, const int ec[kFirst], bool more, int c0,
                                              double f[kComps])
@@ -353,9 +354,9 @@ __global__ void __launch_bounds__(256, kBlocks) k_node_update(NodeArgs a)
   launch_dependents();
 
   if (a.k_post >= 0 || a.gather_only) {
-    // ModelData::ComputeInternalForce: zero, then element contributions in
-    // increasing element order (src/nimble_model_data.cc:620-667,
-    // src/nimble_block.cc:373-383).
+    // ModelData::ComputeInternalForce: the sum of the element contributions
+    // (src/nimble_model_data.cc:620-667, src/nimble_block.cc:373-383), which the
+    // reference adds in increasing element order, as the FP32 form does.
     double f[kComps];
     if (closes) {
       f[0] = close_force<kExact>(a, group, [&](int k) {
