@@ -527,6 +527,10 @@ __global__ void __launch_bounds__(128, kBlocks<kStore, kHasElastic>) k_element_f
   // (after the loop: a call inside it would spill the loop's state)
   if (!__syncthreads_or(any_bad != 0)) return;
   if (__syncthreads_or(gave_up)) return;  // a late copy may still change the staging
+  if (lane == 0) {  // which is used otherwise from here on
+    tc::mbar_inval(&bar[0]);
+    tc::mbar_inval(&bar[1]);
+  }
   left_to_fp64<kElems>(a, reinterpret_cast<int*>(stage_all), (kStore ? kStageBytesStore : kStageBytes) / 4);
 }
 

@@ -127,6 +127,11 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mbar)), "r"(count) : "memory");
 }
+// The barrier's memory is free for other use.
+__device__ __forceinline__ void mbar_inval(uint64_t* mbar)
+{
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(mbar)) : "memory");
+}
 // Make initialised barriers visible to the asynchronous copies that arrive on them.
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from
