@@ -46,16 +46,21 @@ using fx::u64;
 constexpr int kGeoPoint = 10, kGeoRows = 2 * kGeoPoint + 1, kGeoBlock = kGeoRows * 32;  // words
 constexpr int kGeoBytes = kGeoBlock * 8;
 
+// A material that fixed_material leaves to the FP64 code.
+__device__ __forceinline__ bool unfit(const FixedMaterial& m) { return (unsigned)(m.exponent + 400) > 800u; }
+
 // From the FP64 planes: G0 scaled by 2^sG so that its largest entry over the
 // points is in [2^60, 2^61) (of elastic elements each row's), the volume det J_X
 // over 2^Ed (the largest in [1/2, 1)) at 2^62, and the exponents su = 124 - sG
-// and Ed - sG + 2.
+// and Ed - sG + 2.  `never`: counts the elements that their geometry or material
+// keeps out of the domain whatever their displacements.
 __global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ geo, const int* __restrict__ elem_group,
-                                 const FixedMaterial* __restrict__ mats, i64* __restrict__ out)
+                                 const FixedMaterial* __restrict__ mats, i64* __restrict__ out, int* __restrict__ never)
 {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
-  const bool elastic = mats[elem_group ? elem_group[e] : 0].model == kElastic;
+  const FixedMaterial mat     = mats[elem_group ? elem_group[e] : 0];
+  const bool          elastic = mat.model == kElastic;
   double     row[3] = {0.0, 0.0, 0.0}, dmax = 0.0;
   for (int p = 0; p < 8; p++) {
     for (int q = 0; q < 9; q++) row[q / 3] = fmax(row[q / 3], fabs(geo[(p * kGeoPerPoint + q) * ld_e + e]));
@@ -74,6 +79,7 @@ __global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ ge
       places[d] = eg - er;
       if (places[d] > fx::kMaxRow) fits = false;
     }
+  if (!fits || unfit(mat)) atomicAdd(never, 1);
   const int  sG = 61 - eg, su = fits ? 124 - sG : 1 << 20, ef = fits ? ed - sG + 2 : 0;
   const int  low = elastic && fits ? (places[0] | places[1] << 4 | places[2] << 8) << 16 | (ef & 0xffff) : ef;
   i64* const base = out + (size_t)(e >> 3) * kGeoBlock + (e & 7);
@@ -94,10 +100,10 @@ __global__ void k_fixed_geometry(int E, long ld_e, const double* __restrict__ ge
 size_t fixed_geometry_words(long ld_e) { return (size_t)((ld_e + 7) / 8) * kGeoBlock; }
 
 cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, const int* elem_group, const FixedMaterial* mats,
-                                  long long* out, cudaStream_t stream)
+                                  long long* out, int* never, cudaStream_t stream)
 {
   if (E == 0) return cudaSuccess;
-  k_fixed_geometry<<<grid_for(E, 128), 128, 0, stream>>>(E, ld_e, geo, elem_group, mats, out);
+  k_fixed_geometry<<<grid_for(E, 128), 128, 0, stream>>>(E, ld_e, geo, elem_group, mats, out, never);
   return cudaGetLastError();
 }
 
@@ -348,7 +354,7 @@ __global__ void __launch_bounds__(128, kBlocks<kStore, kHasElastic>) k_element_f
     int                 ef      = (int)ge;
     fx::Rows            rows    = {0, 0, 0};
     int                 sh = su - sc, ee = 0;
-    unsigned bad = (unsigned)(mat.exponent + 400) > 800u;
+    unsigned bad = unfit(mat);
     // An infinity or a NaN, or numbers whose sums may become one (2^1017 and
     // more): an elastic element's modes do not show it, as the same value at all
     // corners leaves nothing in any difference.

@@ -143,9 +143,10 @@ int         num_sms();
 cudaError_t launch_element_plain(const ElementArgs& a, cudaStream_t stream);
 // The FP64 form's fixed-point geometry (words: 64-bit), from the geo planes.
 size_t      fixed_geometry_words(long ld_e);
-// (elem_group: material of each element, or null)
+// (elem_group: material of each element, or null); adds the number of elements
+// that are never evaluated in fixed point to *never.
 cudaError_t launch_fixed_geometry(int E, long ld_e, const double* geo, const int* elem_group, const FixedMaterial* mats,
-                                  long long* out, cudaStream_t stream);
+                                  long long* out, int* never, cudaStream_t stream);
 // F = I (sigma = 0) in every point record: the element data before the first step.
 cudaError_t launch_ip_identity(int E, long ld_e, void* ip, int ip_is_float, cudaStream_t stream);
 

@@ -656,6 +656,14 @@ bool force_records_pay(int N, int E, long ld_n, const std::vector<int>& slots, c
   return records < planes;
 }
 
+void free_fixed(nsm_model* m)
+{
+  for (void* p : {(void*)m->d_geo_fixed, (void*)m->d_elem_left, (void*)m->d_fixed_mats}) cudaFree(p);
+  m->d_geo_fixed  = nullptr;
+  m->d_elem_left  = nullptr;
+  m->d_fixed_mats = nullptr;
+}
+
 // The fixed-point geometry's memory, a quarter of an FP64 model's, where the
 // device has it and as much again as the calls on the model take for a time
 // (point records to the host 576 bytes an element; a chunked force call's staging).
@@ -673,10 +681,7 @@ cudaError_t allocate_fixed(nsm_model* m)
   if (e == cudaSuccess) e = cudaMalloc(&m->d_fixed_mats, mats);
   if (e != cudaErrorMemoryAllocation) return e;
   cudaGetLastError();
-  for (void* p : {(void*)m->d_geo_fixed, (void*)m->d_elem_left, (void*)m->d_fixed_mats}) cudaFree(p);
-  m->d_geo_fixed  = nullptr;
-  m->d_elem_left  = nullptr;
-  m->d_fixed_mats = nullptr;
+  free_fixed(m);
   return cudaSuccess;
 }
 
@@ -918,6 +923,7 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     s.status     = m->d_status;
     cudaError_t e = nsm::launch_setup(s, m->stream);  // also for no elements: mass 0, the largest step
     std::vector<nsm::FixedMaterial> fixed_mats;
+    int                             never = 0;  // elements that stay out of the fixed-point domain
     if (e == cudaSuccess && m->precision == NSM_PRECISION_FP64) {
       for (const auto& b : gm) fixed_mats.push_back(nsm::fixed_material(b));
       e = allocate_fixed(m);
@@ -925,7 +931,12 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
         e = cudaMemcpyAsync(m->d_fixed_mats, fixed_mats.data(), sizeof(nsm::FixedMaterial) * num_mats,
                             cudaMemcpyHostToDevice, m->stream);
       if (e == cudaSuccess && m->d_geo_fixed)
-        e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_elem_group, m->d_fixed_mats, m->d_geo_fixed, m->stream);
+        e = cudaMemsetAsync(m->d_out, 0, sizeof(int), m->stream);
+      if (e == cudaSuccess && m->d_geo_fixed)
+        e = nsm::launch_fixed_geometry(E, m->ld_e, m->d_geo, m->d_elem_group, m->d_fixed_mats, m->d_geo_fixed,
+                                       reinterpret_cast<int*>(m->d_out), m->stream);
+      if (e == cudaSuccess && m->d_geo_fixed)
+        e = cudaMemcpyAsync(&never, m->d_out, sizeof(int), cudaMemcpyDeviceToHost, m->stream);
     }
     m->dt_group.assign(S, 1.7976931348623157e308);
     if (e == cudaSuccess)
@@ -933,6 +944,9 @@ int create_impl(int S, const nsm_mesh_desc* meshes, int num_mats, const nsm_mate
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);  // host vectors live until here
     cudaFree(me);
     if (e != cudaSuccess) return bail(cuda_fail(e, "setup"));
+    // Nearly all of them: without the pass that only says so (2,097,152 elements
+    // 5.08 ms a launch instead of 5.57).
+    if (m->d_geo_fixed && never > 0 && never >= 0.9 * E) free_fixed(m);
     m->dt_crit = 1.7976931348623157e308;
     for (double d : m->dt_group)
       if (d < m->dt_crit) m->dt_crit = d;

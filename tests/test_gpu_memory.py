@@ -1,5 +1,6 @@
-"""An FP64 model where the device has no room for its fixed-point geometry: the
-same mesh runs, its elements evaluated by the FP64 code."""
+"""FP64 models without fixed-point geometry: the device has no room for it, or
+(nearly) no element is inside the domain.  The same mesh runs, its elements
+evaluated by the FP64 code."""
 import numpy as np
 import pytest
 
@@ -54,3 +55,48 @@ def test_a_model_without_room_for_the_fixed_geometry(blocks):
     for key in want:
         a, b = np.asarray(got[key], float), np.asarray(want[key], float)
         assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(b), key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", [0.0, 0.5, 0.95, 1.0])
+def test_meshes_out_of_the_domain_keep_no_fixed_geometry(share):
+    """A share of the elements is elastic of a low shear modulus (K = 20 G), which
+    fixed point does not take: from nine tenths on, the model is as large as an
+    FP64 one without it, and the forces are the ones that the FP64 code gives
+    those elements beside others."""
+    torch = pytest.importorskip("torch")
+    from nimblesm_gb300 import build as B
+    B.build()
+    torch.zeros(1, device="cuda")
+    p = cube_problem(40, jitter=0.2, seed=4)
+    E.Model(p).close()
+
+    def size():
+        free0 = torch.cuda.mem_get_info()[0]
+        m = E.Model(p)
+        return m, free0 - torch.cuda.mem_get_info()[0]
+
+    m, whole = size()  # neo-Hookean, all of it inside
+    m.close()
+    p.blocks = [Material("elastic", p.density, 20 * p.shear_modulus, p.shear_modulus),
+                Material("neohookean", p.density, p.bulk_modulus, p.shear_modulus)]
+    p.elem_block = (np.arange(p.num_elem) >= share * p.num_elem).astype(np.int32)
+    if share == 0.0 or share == 1.0:
+        p.blocks, p.elem_block = [p.blocks[int(share == 0.0)]], np.zeros(p.num_elem, np.int32)
+    u = np.random.default_rng(1).normal(0, 1e-3 / 40, p.coords.shape)
+    m, used = size()
+    assert (used < whole - 673 * p.num_elem // 2) == (share >= 0.9), (used, whole)
+    f = m.ComputeInternalForceHost(u)
+    m.close()
+    if share == 1.0:  # the same elements beside enough others that there is fixed geometry
+        extra = cube_problem(40, jitter=0.2, seed=5)
+        extra.v_init = None
+        q = cube_problem(40, jitter=0.2, seed=4)
+        q.coords = np.concatenate([q.coords, extra.coords + 2.0])
+        q.conn = np.concatenate([q.conn, extra.conn + p.num_nodes])
+        q.blocks = [p.blocks[0], Material("neohookean", p.density, p.bulk_modulus, p.shear_modulus)]
+        q.elem_block = (np.arange(2 * p.num_elem) >= p.num_elem).astype(np.int32)
+        q.bcs, q.v_init = [], None
+        both = E.Model(q)
+        assert np.array_equal(both.ComputeInternalForceHost(np.concatenate([u, u]))[: p.num_nodes], f)
+        both.close()
