@@ -45,7 +45,8 @@ UQ_SCHEDULE_STEPS = 1000  # the ensemble's schedule: 1000 steps per sample
 # (the conversions of the forces) and 374 wide products, which an SM takes at
 # one per cycle (per warp).  The same formulation on the FP64 pipe executes
 # 170.2 instructions, 258.1 flops (87.9 DFMA, 44.5 DADD, 37.9 DMUL): what the
-# evaluation is worth in FP64.  (Counted by ncu on the 64^3 case.)
+# evaluation is worth in FP64.  (Instructions counted by ncu on the 64^3 case,
+# the products in the source.)
 FP64_FLOPS_PER_IP = 258.1
 FP64_INSTR_PER_IP = 6.0
 WIDE_PRODUCTS_PER_IP = 374

@@ -20,10 +20,12 @@
  *     one handle must not overlap (like the reference's ModelData, which is not
  *     thread-safe); different handles are independent.
  *   - Arithmetic: NSM_PRECISION_FP64 takes and gives FP64 numbers; nodal
- *     state, mass, time step and energies are computed in IEEE FP64, the
- *     element work (gradient, F, stress, B^T sigma) in 64-bit fixed point whose
- *     error is below an FP64 evaluation's, or in FP64 where an element leaves
- *     its domain (strains of about 0.1; csrc/hex_fixed.cuh).
+ *     state, mass, time step and energies are computed in IEEE FP64 (but a
+ *     node's sum of element forces, to 2^-56 of the largest), the element work
+ *     (gradient, F, stress, B^T sigma) in 64-bit fixed point inside its domain
+ *     and in FP64 outside it (csrc/hex_fixed.cuh: |F - I| of 0.1 to 0.5, and
+ *     shapes and moduli for which its error in general deformations is below an
+ *     FP64 evaluation's).
  *     NSM_PRECISION_FP32_MIXED computes the element work in FP32 and keeps the
  *     nodal state, mass, time step and energies in FP64.
  */

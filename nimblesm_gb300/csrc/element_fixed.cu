@@ -4,9 +4,9 @@
 //
 // Bound: the integer pipes and issue.  On the FP64 pipe the same work is 170
 // FP64 instructions per point at 16 clocks each per SM: 5.08 ms for 128^3
-// elements, pipe 89% busy.  Here it is about 1,190 integer instructions per
-// point, 360 of them wide products (one per clock and SM), the others at two
-// to four per clock: 1.09 ms (issue 46%, multiplier 73%), 1.52 ms with F and sigma
+// elements, pipe 89% busy.  Here it is 1,190 instructions per point, 374 of
+// them wide products (one per clock and SM; 530 on the multiplier's pipe), the
+// others at two to four per clock: 1.10 ms (issue 46%), 1.56 ms with F and sigma
 // stored; one launch on 4,096 elements 11 us against 60 us.
 //
 // Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
@@ -23,7 +23,8 @@
 // displacements (cp.async) and connectivity in flight.
 //
 // An element outside the fixed-point domain is evaluated by the FP64 code
-// (element_work), records included.
+// (element_work), records included, and where (nearly) all are, or the device has
+// no room for this geometry, every element is (launch_element_plain).
 #include <algorithm>
 #include <cmath>
 
@@ -113,7 +114,7 @@ FixedMaterial fixed_material(const GroupMaterial& m)
   const double  most = std::fmax(m.bulk, m.shear);
   if (!std::isfinite(most) || !(most > 1e-90) || !(most < 1e90)) return f;  // left to the FP64 code
   // as are ratios of the moduli at which that is the more exact one (hex_fixed.cuh)
-  if (m.model == kElastic ? m.bulk > 8.0 * m.shear : 2.0 * m.bulk < m.shear) return f;
+  if (m.model == kElastic ? m.bulk > 4.0 * m.shear : 2.0 * m.bulk < m.shear) return f;
   f.exponent = std::ilogb(most) + 4;
   f.half_k   = std::llrint(std::ldexp(m.bulk, 61 - f.exponent));
   f.shear    = std::llrint(std::ldexp(m.shear, 62 - f.exponent));

@@ -66,9 +66,9 @@ NSM_HD Limbs split(i64 x)
 // of the limbs' parts, five times the work).  The product alone, not mad.wide:
 // sums in C++ let the compiler put the additions into the products (a sum of
 // three 64 x 64 bit products is 9 + 2 instructions), which it does not do for
-// a chain of mad.wide: 1,513 instructions per point became 1,194 and the
+// a chain of mad.wide: 1,513 instructions per point became 1,190 and the
 // element kernel 1,105 us instead of 1,240 at 2,097,152 elements; the funnel
-// shifts below give 14 us more.  (A third addend of zero in additions of two,
+// shifts below gave 14 us more.  (A third addend of zero in additions of two,
 // to keep them off the multiplier's pipe: 1,103 to 1,193 us.)
 NSM_HD u64 mul_wide(int a, int b)
 {
@@ -328,9 +328,11 @@ NSM_HD void powers(i64 t, i64& r5, i64& rj)
 // modes to match, so that a flat element loses few places: forces to 1.0e-16 of
 // themselves for cubes (FP64 1.9e-16) and 1.3e-16 at an aspect ratio of 4 (FP64
 // 3.9e-16; tests/fixed_domain_check.cc).  Flatter elements than kMaxRow says,
-// and materials of K > 8 G (their shear modulus has fewer bits), are left to
-// FP64: in states that FP64 gives without a rounding (plane stress and shear
-// along the axes of an unjittered mesh) they would lose more than a place to it.
+// and materials of K > 4 G (their shear modulus has fewer bits), are left to
+// FP64: where it has nothing to round but the result (shear along the axes of an
+// unjittered mesh, 1.1e-16; plane stress, 1.6e-16) the forces of cubes with
+// K = 2 G are off by 1.6e-16 and 1.3e-16 here, at K = 4 G and an aspect ratio of
+// 4 by 6e-16 and 5e-16, and more beyond.
 //
 // The forces at the points keep kElasticForce further places: with more, their
 // sums could leave 63 bits, and one element left to the FP64 code makes a launch
