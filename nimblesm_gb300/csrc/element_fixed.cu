@@ -11,10 +11,10 @@
 //
 // Four lanes per element (lanes j, j + 8, j + 16, j + 24 of a warp hold the
 // j-th of 8 consecutive elements; in small meshes eight, with a point each), two
-// points each, in a loop that is not
-// unrolled: the code of one point stays in the instruction cache (four points
-// unrolled, two lanes per element, ran at 25% issue with instruction fetch the
-// largest stall), and a small mesh waits for two points in a row, not eight.
+// points each, in a loop that is not unrolled: the code of one point stays in
+// the instruction cache (four points unrolled, two lanes per element, ran at 25%
+// issue with instruction fetch the largest stall), and a small mesh waits for
+// two points in a row, not eight.
 // The lanes exchange 18 numbers before and 18 after.  Everything an element's
 // result depends on is its own, so any launch shape gives the same bits.
 //
