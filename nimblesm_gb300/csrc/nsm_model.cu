@@ -30,8 +30,11 @@ int fail(int code, const std::string& msg)
   return code;
 }
 
+// (The error is reported here and must not come up again as the result of the
+// next call's first launch.)
 int cuda_fail(cudaError_t e, const char* where)
 {
+  cudaGetLastError();
   g_error = std::string(where) + ": " + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? NSM_ERR_OUT_OF_MEMORY : NSM_ERR_CUDA;
 }
@@ -1368,7 +1371,9 @@ cudaError_t internal_force_pipelined(nsm_model* m, const double* u_host, double*
     touch_pages(f_host, sizeof(double) * 3 * (size_t)m->N);
     for (int j = 0; j < K && err == cudaSuccess; j++) err = copy_out(j);
   }
-  if (err == cudaSuccess) err = cudaStreamSynchronize(s_out);
+  if (err == cudaSuccess) return cudaStreamSynchronize(s_out);
+  // (refused on the way: nothing of the call touches the caller's arrays afterwards)
+  for (cudaStream_t s : {s_in, s_planes, s_el[0], s_el[1], m->stream, s_out}) cudaStreamSynchronize(s);
   return err;
 }
 

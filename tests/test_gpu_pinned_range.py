@@ -36,6 +36,11 @@ def test_arrays_pinned_at_both_ends_only():
             m.ComputeInternalForceHost(arrays[0], out=arrays[1])
         with pytest.raises(E.EngineError):
             m.ComputeInternalForceHost(u, out=arrays[1])
+        for chunks in (3, 1):  # refused part of the way; and the handle still works
+            m.set_host_chunks(chunks)
+            with pytest.raises(E.EngineError):
+                m.ComputeInternalForceHost(arrays[0], out=arrays[1])
+            assert np.array_equal(m.ComputeInternalForceHost(u), want)
         for at in registered:
             assert int(rt.cudaHostUnregister(at)) == 0
         registered = [raw.ctypes.data + first]  # both in one piece
